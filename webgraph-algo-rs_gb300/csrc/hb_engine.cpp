@@ -525,7 +525,7 @@ int device_partition(hb_handle* h, const uint64_t* off0, uint32_t win_nodes, uin
         HB_CUDA(h, cudaMemcpyAsync(h->d_heavy, heavy.data(), h->n_heavy * 4, cudaMemcpyHostToDevice,
                                    h->stream));
         // heavy-kernel items: a node of more than HEAVY_SPLIT arcs becomes
-        // segments of HEAVY_SEG arcs; items by decreasing arcs (ties in list
+        // segments of at most HEAVY_SEG arcs; items by decreasing arcs (ties in list
         // order), so the longest start first. The key holds 2^32 - 1 - degree.
         struct Item {
             uint64_t arcs;
@@ -538,8 +538,7 @@ int device_partition(hb_handle* h, const uint64_t* off0, uint32_t win_nodes, uin
             if (d > hbk::HEAVY_SPLIT) {
                 const uint32_t nseg = (uint32_t)((d + hbk::HEAVY_SEG - 1) / hbk::HEAVY_SEG);
                 for (uint32_t k = 0; k < nseg; k++)
-                    items.push_back({std::min<uint64_t>(hbk::HEAVY_SEG, d - (uint64_t)k * hbk::HEAVY_SEG),
-                                     (uint32_t)i, k, nseg, slots});
+                    items.push_back({hbk::heavy_seg_arcs(d, nseg), (uint32_t)i, k, nseg, slots});
                 slots += nseg;
             } else {
                 items.push_back({d, (uint32_t)i, 0, 1, 0});
@@ -758,6 +757,9 @@ hbk::UnionArgs union_args(hb_handle* h) {
         long long bits;
         std::memcpy(&bits, &small, sizeof bits);
         a.small_bits = bits;
+        // a little below a_scaled / (2.5 m): where the estimate may round across
+        // 2.5 m the kernels count the zero registers and compare exactly
+        a.hs_small = (uint64_t)(a.a_scaled / small * (1.0 - 1e-6));
     }
     a.ln_table = h->d_lnt;
     a.tiles = h->d_tiles;
@@ -1282,8 +1284,21 @@ struct MultiCtx {
 static bool job_kernel_log2m(int l) { return l == 4 || l == 6 || l == 8; }
 static constexpr uint32_t kMaxJobs = hbk::MAX_JOBS;
 static constexpr size_t kMaxMultiGraphs = 64;
-// default degree buckets: lane-group nodes up to 64 successors, 8-lane teams up to 4096
+// default degree buckets: lane-group nodes up to 64 successors; the pair the
+// bucket tuner falls back to has 8-lane teams up to 4096
 static constexpr uint32_t kDefaultSmallMax = 64, kDefaultMediumMax = 4096;
+// The default bound of the 8-lane teams. A team walks a node's arcs 8 at a
+// time, so a node of 4096 arcs is 512 dependent gathers, about 0.28 ms: the
+// whole iteration of a graph whose counters are small, and hidden only where
+// an iteration takes milliseconds. Above the bound a node is a block's.
+// Union time of a standard iteration with bounds 4096 / 1024 / 512 / 256:
+// web-like 2e5, log2m 5 (6 MB of counters) 94 / 49 / 41 / 45 us; web-like 1e6,
+// log2m 6 (64 MB) 278 / 170 / 161 / 174 us; R-MAT 2^20, log2m 8 (268 MB) 563 /
+// 546 / 575 / 573 us; web-like 3.3e7, log2m 6 (2.1 GB) 4.66 / 4.65 / 4.94 /
+// 5.64 ms.
+static uint32_t auto_medium_max(uint64_t n, uint64_t counter_bytes) {
+    return n * counter_bytes >= (128ull << 20) ? 1024 : 512;
+}
 
 static void multi_free(MultiCtx& mc) {
     cudaSetDevice(mc.device);
@@ -2253,7 +2268,7 @@ static int create_impl(const hb_graph_view* graph, const hb_graph_view* transpos
     // Work partition and renumbering (host), then the CSR (and the transpose
     // when given) uploaded, validated and renumbered on the device.
     h->small_max = o.small_max_degree != HB_AUTO ? o.small_max_degree : kDefaultSmallMax;
-    h->medium_max = o.medium_max_degree != HB_AUTO ? o.medium_max_degree : kDefaultMediumMax;
+    h->medium_max = o.medium_max_degree != HB_AUTO ? o.medium_max_degree : auto_medium_max(h->n, h->stride);
     if (h->medium_max < h->small_max) h->medium_max = h->small_max;
     const bool device_transpose = !transpose && (o.flags & HB_TRANSPOSE_ON_DEVICE);
     unsigned long long* trows = nullptr;

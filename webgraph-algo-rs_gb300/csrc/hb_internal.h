@@ -22,10 +22,12 @@ int load_bvgraph(const std::string& basename, Csr& g, std::string& err, uint64_t
 namespace hbk {
 
 constexpr int MAX_DISCOUNT = 8;
-// heavy nodes with more arcs than HEAVY_SPLIT run as segments of HEAVY_SEG
-// arcs, one CTA each (k_union_heavy)
-constexpr uint64_t HEAVY_SPLIT = 32768;
-constexpr uint64_t HEAVY_SEG = 16384;
+// heavy nodes with more arcs than HEAVY_SPLIT run as equal segments of at most
+// HEAVY_SEG arcs, one CTA each (k_union_heavy)
+constexpr uint64_t HEAVY_SPLIT = 6144;
+constexpr uint64_t HEAVY_SEG = 4096;
+// arcs of a segment of a node of `arcs` arcs in nseg segments
+__host__ __device__ constexpr uint64_t heavy_seg_arcs(uint64_t arcs, uint64_t nseg) { return (arcs + nseg - 1) / nseg; }
 
 // What one tile (or one block of the heavy-node kernel) contributes to an
 // iteration; summed in a fixed order after the union kernels.
@@ -68,7 +70,8 @@ struct UnionArgs {
     const IterConsts* ic;     // this iteration's d = t + 1, 1/d and discount factors (device)
     int systolic;             // 1: scan only must-be-checked nodes
     int quirk;                // Rust i32-shift count semantics
-    int any31;                // some register may hold 31 (only then count looks for it)
+    int any31;                // some register may hold 30 or 31 (counts then take their general form)
+    uint64_t hs_small;        // below this harmonic sum the estimate is above 2.5 m, so no zero register matters
     uint64_t n;
     double alpha_m_m;
     double a_scaled;          // alpha_m_m * 2^31
@@ -126,7 +129,7 @@ struct InitArgs {
     double alpha_m_m;
     const double* ln_table;
     int quirk;
-    int* any31;               // set to 1 when an initial register holds 31
+    int* any31;               // set to 1 when an initial register holds 30 or 31
 };
 
 static_assert(sizeof(IterConsts) % 8 == 0 && sizeof(TilePartial) % 8 == 0, "copied as 64-bit words");

@@ -81,30 +81,9 @@ __device__ __forceinline__ void publish(double nf, unsigned long long vis, unsig
 }
 
 // ---------------------------------------------------------------------------
-// end of a node's union, run by the G lanes (one per chunk) of a team: store
-// the merged counter into the next state; true when it differs from the
-// previous one (HB:1052).
-// ---------------------------------------------------------------------------
-template <int LOG2M>
-__device__ __forceinline__ bool commit_node(const UnionArgs& a, uint64_t v, int c,
-                                            unsigned team_mask,
-                                            const uint32_t (&prev)[Geo<LOG2M>::NW],
-                                            const uint32_t (&acc)[Geo<LOG2M>::NW]) {
-    using Gm = Geo<LOG2M>;
-    constexpr int G = Gm::CHUNKS, NW = Gm::NW;
-    uint32_t diff = 0;
-#pragma unroll
-    for (int i = 0; i < NW; i++) diff |= prev[i] ^ acc[i];
-    bool changed = diff != 0u;
-    if constexpr (G > 1) changed = __any_sync(team_mask, changed);
-    store_chunk<LOG2M>(a.next, v, c, acc);
-    return changed;
-}
-
-// ---------------------------------------------------------------------------
 // End of a node's union, for the nodes whose counter changed: the per-node
-// arithmetic of HB:1052-1093, run by the G lanes that hold the new counter
-// (lane c == 0 does the f64 part), while it is still in registers:
+// arithmetic of HB:1052-1093, by the lanes that hold the new counter (one of
+// them does the f64 part), while it is still in registers:
 //   post = count(new counter)   (exact integer harmonic sum, one division)
 //   pre  = cached count of the previous counter
 //   NF  += post (standard) or post - pre (systolic); unchanged nodes add
@@ -130,49 +109,144 @@ __device__ __forceinline__ NodeSums load_sums(const UnionArgs& a, uint32_t v) {
     return s;
 }
 
+// The scalars of node v, by one lane: its counter's harmonic sum hs * 2^-31,
+// zero registers (0 will do when hs < hs_small) and registers holding 31.
 template <int LOG2M>
-__device__ __forceinline__ void finish_node(const UnionArgs& a, uint32_t v, int c, unsigned gmask,
-                                            const uint32_t (&acc)[Geo<LOG2M>::NW], bool changed,
-                                            const NodeSums& ns, double& nf, uint32_t& vis) {
-    using Gm = Geo<LOG2M>;
-    constexpr int G = Gm::CHUNKS, REGS = Gm::CHUNK_REGS;
-    if (changed) {
-        uint64_t hs = 0;
-        uint32_t z = 0, c31 = 0;
-        count_chunk<REGS>(acc, hs, z, c31, a.any31 != 0);
-        if constexpr (G > 1) {
+__device__ __forceinline__ void finish_scalars(const UnionArgs& a, uint32_t v, uint64_t hs, uint32_t z, uint32_t c31,
+                                               bool changed, const NodeSums& ns, double& nf, uint32_t& vis) {
+    if (!changed) {
+        if (!a.systolic) nf = __dadd_rn(nf, ns.pre);
+        return;
+    }
+    const double pre = ns.pre;
+    const double post = estimate_fast(signed_hsum(hs, c31, a.quirk), z, a.alpha_m_m, a.a_scaled, a.small_bits,
+                                      (double)Geo<LOG2M>::M, a.ln_table);
+    a.est[v] = post;
+    if (a.systolic) nf = __dadd_rn(nf, -pre);
+    nf = __dadd_rn(nf, post);
+    const double delta = __dsub_rn(post, pre);
+    // delta > 0.0 as an integer test: positive, not NaN
+    const long long db = __double_as_longlong(delta);
+    if (db > 0 && db <= 0x7ff0000000000000ll) {
+        const double d1 = __ldg(&a.ic->d1);
+        if (a.sod) a.sod[v] = __dadd_rn(ns.sod, __dmul_rn(delta, d1));
+        if (a.harm) a.harm[v] = __dadd_rn(ns.harm, div_by_small_int(delta, d1, __ldg(&a.ic->rd1)));
+        for (int k = 0; k < a.ndisc; k++)
+            a.disc[k][v] = __dadd_rn(a.disc[k][v], __dmul_rn(delta, __ldg(&a.ic->disc_factor[k])));
+    }
+    vis += ns.indeg;
+}
+
+// Counts of the counter whose words are spread over the lanes of `mask`
+// (W words each; xor offsets OFF0, 2 OFF0, ... below END reach them all; a
+// lane with `own` false holds copies). Every lane gets the totals.
+template <int W, int OFF0, int END>
+__device__ __forceinline__ void count_lanes(const UnionArgs& a, const uint32_t (&w)[W], bool own, unsigned mask,
+                                            uint64_t& hs, uint32_t& z, uint32_t& c31) {
+    hs = sum_words<W>(w, a.any31 != 0, c31);
+    if (!own) {
+        hs = 0;
+        c31 = 0;
+    }
 #pragma unroll
-            for (int off = 1; off < G; off <<= 1) {
-                hs += __shfl_xor_sync(gmask, hs, off);
-                z += __shfl_xor_sync(gmask, z, off);
-                c31 += __shfl_xor_sync(gmask, c31, off);
+    for (int off = OFF0; off < END; off <<= 1) {
+        hs += __shfl_xor_sync(mask, hs, off);
+        if (a.any31) c31 += __shfl_xor_sync(mask, c31, off);
+    }
+    z = 0;
+    if (a.any31 || hs >= a.hs_small) {
+        z = own ? zero_words<W>(w) : 0u;
+#pragma unroll
+        for (int off = OFF0; off < END; off <<= 1) z += __shfl_xor_sync(mask, z, off);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Reduce-scatter of NW-word rows over the lanes at xor offsets OFF0 .. END / 2:
+// with every step a lane gives half of its words away, while it has several,
+// and merges the half it keeps with its partner's. The merged row then lies
+// spread over the lanes, FW words each from word `first`; `own` is cleared in
+// lanes whose words another lane holds too. A butterfly of whole rows moves NW
+// words in every step, and one lane then compares, stores and counts alone: a
+// medium node of 128 arcs at log2m 6 took 483 warp instructions that way and
+// takes 371 this way (1.11 -> 1.09 ms for 10^6 such nodes, which are bound by
+// the gathers; the tail of a small iteration is these chains).
+// ---------------------------------------------------------------------------
+template <int NW, int OFF0, int END>
+struct Scatter {
+    static constexpr int steps() {
+        int s = 0;
+        for (int o = OFF0; o < END; o <<= 1) s++;
+        return s;
+    }
+    static constexpr int FW = (NW >> steps()) > 1 ? (NW >> steps()) : 1;
+};
+
+template <int NW, int OFF0, int END>
+__device__ __forceinline__ void reduce_scatter(uint32_t (&acc)[NW], uint32_t (&out)[Scatter<NW, OFF0, END>::FW],
+                                               int& first, bool& own, unsigned mask) {
+    const int lane = threadIdx.x & 31;
+    first = 0;
+    own = true;
+    int have = NW;
+#pragma unroll
+    for (int o = OFF0; o < END; o <<= 1) {
+        const bool up = (lane & o) != 0;
+        if (have > 1) {
+            have /= 2;
+#pragma unroll
+            for (int i = 0; i < NW / 2; i++) {
+                if (i >= have) break;
+                const uint32_t give = up ? acc[i] : acc[i + have];
+                uint32_t keep[1] = {up ? acc[i + have] : acc[i]};
+                const uint32_t got[1] = {__shfl_xor_sync(mask, give, o)};
+                merge_chunk<4>(keep, got);
+                acc[i] = keep[0];
             }
+            if (up) first += have;
+        } else {
+            uint32_t keep[1] = {acc[0]};
+            const uint32_t got[1] = {__shfl_xor_sync(mask, acc[0], o)};
+            merge_chunk<4>(keep, got);
+            acc[0] = keep[0];
+            own = own && !up;
         }
-        if (c == 0) {
-            const double pre = ns.pre;
-            const double post = estimate_fast(signed_hsum(hs, c31, a.quirk), z, a.alpha_m_m,
-                                              a.a_scaled, a.small_bits, (double)Gm::M, a.ln_table);
-            a.est[v] = post;
-            if (a.systolic) {
-                nf = __dadd_rn(nf, -pre);
-                nf = __dadd_rn(nf, post);
-            } else {
-                nf = __dadd_rn(nf, post);
-            }
-            const double delta = __dsub_rn(post, pre);
-            // delta > 0.0 as an integer test: positive, not NaN
-            const long long db = __double_as_longlong(delta);
-            if (db > 0 && db <= 0x7ff0000000000000ll) {
-                const double d1 = __ldg(&a.ic->d1);
-                if (a.sod) a.sod[v] = __dadd_rn(ns.sod, __dmul_rn(delta, d1));
-                if (a.harm) a.harm[v] = __dadd_rn(ns.harm, div_by_small_int(delta, d1, __ldg(&a.ic->rd1)));
-                for (int k = 0; k < a.ndisc; k++)
-                    a.disc[k][v] = __dadd_rn(a.disc[k][v], __dmul_rn(delta, __ldg(&a.ic->disc_factor[k])));
-            }
-            vis += ns.indeg;
+    }
+#pragma unroll
+    for (int i = 0; i < Scatter<NW, OFF0, END>::FW; i++) out[i] = acc[i];
+}
+
+// W consecutive words (aligned to W words, at most four in one access)
+template <int W>
+__device__ __forceinline__ void load_words(const uint8_t* p, uint32_t (&w)[W]) {
+    if constexpr (W == 1) {
+        w[0] = __ldg(reinterpret_cast<const uint32_t*>(p));
+    } else if constexpr (W == 2) {
+        const uint2 t = __ldg(reinterpret_cast<const uint2*>(p));
+        w[0] = t.x;
+        w[1] = t.y;
+    } else {
+#pragma unroll
+        for (int i = 0; i < W; i += 4) {
+            const uint4 t = __ldg(reinterpret_cast<const uint4*>(p + 4 * i));
+            w[i] = t.x;
+            w[i + 1] = t.y;
+            w[i + 2] = t.z;
+            w[i + 3] = t.w;
         }
-    } else if (!a.systolic && c == 0) {
-        nf = __dadd_rn(nf, ns.pre);
+    }
+}
+
+template <int W>
+__device__ __forceinline__ void store_words(uint8_t* p, const uint32_t (&w)[W]) {
+    if constexpr (W == 1) {
+        *reinterpret_cast<uint32_t*>(p) = w[0];
+    } else if constexpr (W == 2) {
+        *reinterpret_cast<uint2*>(p) = make_uint2(w[0], w[1]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < W; i += 4)
+            *reinterpret_cast<uint4*>(p + 4 * i) = make_uint4(w[i], w[i + 1], w[i + 2], w[i + 3]);
     }
 }
 
@@ -589,36 +663,41 @@ __device__ __forceinline__ void run_nodes(const UnionArgs& a, const uint32_t* __
                 }
             }
             if constexpr (PB > 1) {
+                // the team's partial rows: merged and spread over its lanes,
+                // which end the node together
+                constexpr int FW = Scatter<NW, G, TB>::FW;
                 __syncwarp(tmask);
+                uint32_t w[FW], prev[FW], diff = 0;
+                int first;
+                bool own;
+                reduce_scatter<NW, G, TB>(acc, w, first, own, tmask);
+                const uint64_t at = v * (uint64_t)Gm::COUNTER_BYTES + (uint32_t)(c * Gm::CHUNK_BYTES + 4 * first);
+                load_words<FW>(a.curr + at, prev);
 #pragma unroll
-                for (int off = G; off < TB; off <<= 1) {
-                    // four words at a time keeps few registers live
-#pragma unroll
-                    for (int k = 0; k < NW; k += 4) {
-                        uint32_t x4[4], y4[4];
-#pragma unroll
-                        for (int j = 0; j < 4; j++) {
-                            x4[j] = acc[k + j];
-                            y4[j] = __shfl_xor_sync(tmask, acc[k + j], off);
-                        }
-                        merge_chunk<16>(x4, y4);
-#pragma unroll
-                        for (int j = 0; j < 4; j++) acc[k + j] = x4[j];
-                    }
+                for (int k = 0; k < FW; k++) diff |= w[k] ^ prev[k];
+                if (own) store_words<FW>(a.next + at, w);
+                changed = __any_sync(tmask, diff != 0u);
+                uint64_t hs = 0;
+                uint32_t z = 0, c31 = 0;
+                if (changed) count_lanes<FW, 1, TB>(a, w, own, tmask, hs, z, c31);
+                if (tl == 0) {
+                    scanned++;
+                    sarcs += (uint32_t)(s1 - s0);
+                    finish_scalars<LOG2M>(a, v, hs, z, c31, changed, load_sums(a, v), nf, vis);
                 }
-            }
-            if (p == 0) {
+            } else {
                 // the previous counter, read again (L1/L2) rather than kept in registers
                 changed = differs_from<LOG2M>(a.curr, v, c, acc);
                 if constexpr (G > 1) changed = __any_sync(lmask, changed);
                 store_chunk<LOG2M>(a.next, v, c, acc);
+                uint64_t hs = 0;
+                uint32_t z = 0, c31 = 0;
+                if (changed) count_lanes<NW, 1, G>(a, acc, true, lmask, hs, z, c31);
                 if (c == 0) {
                     scanned++;
                     sarcs += (uint32_t)(s1 - s0);
+                    finish_scalars<LOG2M>(a, v, hs, z, c31, changed, load_sums(a, v), nf, vis);
                 }
-                NodeSums ns{};
-                if (c == 0) ns = load_sums(a, v);
-                finish_node<LOG2M>(a, v, c, lmask, acc, changed, ns, nf, vis);
             }
         } else if (copy && p == 0) {
             uint32_t w[NW];
@@ -1122,39 +1201,39 @@ __device__ __forceinline__ void staged_nodes(const UnionArgs& a, uint32_t buf, i
             for (int k = 0; k < NW; k++) acc[k] = 0u;
         }
         staged_gather<LOG2M, PIPE>(a, ids, v, c, s0 + p, s1, PB, acc);
-        if constexpr (PB > 1) {
-            __syncwarp(tmask);
-#pragma unroll
-            for (int off = G; off < TB; off <<= 1) {
-#pragma unroll
-                for (int k = 0; k < NW; k += 4) {
-                    uint32_t x4[4], y4[4];
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        x4[j] = acc[k + j];
-                        y4[j] = __shfl_xor_sync(tmask, acc[k + j], off);
-                    }
-                    merge_chunk<16>(x4, y4);
-#pragma unroll
-                    for (int j = 0; j < 4; j++) acc[k + j] = x4[j];
-                }
-            }
+        NodeSums ns{};
+        if (tl == 0) {
+            scanned++;
+            sarcs += s1 - s0;
+            ns.pre = lds<double>(buf + SG::OFF_EST + 8 * slot);
+            ns.sod = a.sod ? lds<double>(buf + SG::OFF_SOD + 8 * slot) : 0.0;
+            ns.harm = a.harm ? lds<double>(buf + SG::OFF_HARM + 8 * slot) : 0.0;
+            ns.indeg = lds<uint32_t>(buf + SG::OFF_INDEG + 4 * slot);
         }
-        if (p == 0) {
+        uint64_t hs = 0;
+        uint32_t z = 0, c31 = 0;
+        if constexpr (PB > 1) {
+            // as run_nodes ends a medium node
+            constexpr int FW = Scatter<NW, G, TB>::FW;
+            __syncwarp(tmask);
+            uint32_t w[FW], prev[FW], diff = 0;
+            int wfirst;
+            bool own;
+            reduce_scatter<NW, G, TB>(acc, w, wfirst, own, tmask);
+            const uint64_t at = v * (uint64_t)Gm::COUNTER_BYTES + (uint32_t)(c * Gm::CHUNK_BYTES + 4 * wfirst);
+            load_words<FW>(a.curr + at, prev);
+#pragma unroll
+            for (int k = 0; k < FW; k++) diff |= w[k] ^ prev[k];
+            if (own) store_words<FW>(a.next + at, w);
+            changed = __any_sync(tmask, diff != 0u);
+            if (changed) count_lanes<FW, 1, TB>(a, w, own, tmask, hs, z, c31);
+        } else {
             changed = differs_from<LOG2M>(a.curr, v, c, acc);
             if constexpr (G > 1) changed = __any_sync(lmask, changed);
             store_chunk<LOG2M>(a.next, v, c, acc);
-            NodeSums ns{};
-            if (c == 0) {
-                scanned++;
-                sarcs += s1 - s0;
-                ns.pre = lds<double>(buf + SG::OFF_EST + 8 * slot);
-                ns.sod = a.sod ? lds<double>(buf + SG::OFF_SOD + 8 * slot) : 0.0;
-                ns.harm = a.harm ? lds<double>(buf + SG::OFF_HARM + 8 * slot) : 0.0;
-                ns.indeg = lds<uint32_t>(buf + SG::OFF_INDEG + 4 * slot);
-            }
-            finish_node<LOG2M>(a, v, c, lmask, acc, changed, ns, nf, vis);
+            if (changed) count_lanes<NW, 1, G>(a, acc, true, lmask, hs, z, c31);
         }
+        if (tl == 0) finish_scalars<LOG2M>(a, v, hs, z, c31, changed, ns, nf, vis);
     }
     // modified bits: the item's nodes are consecutive, one bit per node slot
     const unsigned ball = __ballot_sync(0xffffffffu, changed && p == 0 && c == 0);
@@ -1250,139 +1329,163 @@ __global__ void k_chunk_items(const uint2* __restrict__ chunks, uint64_t n_chunk
 
 // ---------------------------------------------------------------------------
 // heavy nodes: one CTA per work item. An item is a whole heavy node, or, for
-// a node of more than HEAVY_SPLIT arcs, one segment of HEAVY_SEG of its arcs
-// (a single CTA on the largest R-MAT node, 240 K arcs at 2^24, took the whole
-// heavy kernel's time). Lanes split the item's successors (G lanes per
-// counter); the per-lane partial counters are merged by a butterfly of
-// shuffles and then across warps through shared memory. A segment stores its
-// partial counter in the node's slot and counts itself in; the last segment
-// to arrive merges the node's partials (and the node's own counter) and ends
-// the node as a whole node does. The maximum is order independent, so the
-// result is the same whichever segment arrives last.
+// a node of more than HEAVY_SPLIT arcs, one of its equal segments of at most
+// HEAVY_SEG arcs. Lanes split the item's successors (G lanes per counter); the
+// lanes' partial counters are merged and spread over the warp by a
+// reduce-scatter and meet in shared memory, where the first warp merges them
+// and ends the node with a few words a lane. A segment stores its partial
+// counter in the node's slot and counts itself in; the last segment to arrive
+// merges the node's partials (and the node's own counter) and ends the node.
+// The maximum is order independent, so the result is the same whichever
+// segment arrives last.
+// What bounds it is the chain of an item: 256 / G arcs at a time, one gather
+// each, about 0.6 us. Segments of 16,384 arcs were 64 such steps, 40-78 us, the
+// whole of a small iteration; 4096 are 16. With the shorter ends, more nodes
+// are better off here than on an 8-lane team (see auto_medium_max), and with
+// idle items skipped 256 at a time, a systolic iteration that checks next to
+// nothing takes 18 instead of 64 us (web-like 3.3e7, 36,000 heavy nodes).
 // ---------------------------------------------------------------------------
-// chunk c of a partial counter written by another block of this launch (L2,
-// not the non-coherent path)
 template <int LOG2M>
-__device__ __forceinline__ void load_chunk_cg(const uint8_t* base, uint64_t slot, int c,
-                                              uint32_t (&w)[Geo<LOG2M>::NW]) {
+__global__ void __launch_bounds__(256) k_union_heavy(const __grid_constant__ UnionArgs a) {
     using Gm = Geo<LOG2M>;
-    const uint4* p = reinterpret_cast<const uint4*>(base + slot * (uint64_t)Gm::COUNTER_BYTES +
-                                                    (uint64_t)c * Gm::CHUNK_BYTES);
-#pragma unroll
-    for (int q = 0; q < Gm::NW / 4; q++) {
-        const uint4 t = __ldcg(p + q);
-        w[4 * q] = t.x;
-        w[4 * q + 1] = t.y;
-        w[4 * q + 2] = t.z;
-        w[4 * q + 3] = t.w;
-    }
-}
-
-template <int LOG2M>
-__global__ void __launch_bounds__(256) k_union_heavy(UnionArgs a) {
-    using Gm = Geo<LOG2M>;
-    constexpr int G = Gm::CHUNKS, NW = Gm::NW, REGS = Gm::CHUNK_REGS;
+    constexpr int G = Gm::CHUNKS, NW = Gm::NW, M4 = Gm::M / 4;
     constexpr int TEAM = 256, P = TEAM / G, WARPS = TEAM / 32;
-    __shared__ uint32_t red[WARPS][G][NW];
+    constexpr int FW = Scatter<NW, G, 32>::FW;
+    // words of a row per lane of the warp that ends the node
+    constexpr int EW = M4 > 32 ? M4 / 32 : 1;
+    __shared__ __align__(16) uint32_t red[WARPS][M4];
+    __shared__ uint32_t s_idx[TEAM], s_warp[WARPS];
     __shared__ uint32_t s_last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int tid = threadIdx.x;
     const int p = tid / G, c = tid % G;
-    const unsigned leader_mask = G == 32 ? 0xffffffffu : ((1u << G) - 1u);
+    const uint64_t eat = (uint64_t)(lane * EW < M4 ? lane * EW : 0) * 4;  // byte of the ending lane's words
+    const bool elane = lane * EW < M4;
     uint32_t modc = 0, scanned = 0, sarcs = 0, vis = 0;
-    for (uint64_t idx = blockIdx.x; idx < a.heavy_len; idx += gridDim.x) {
-        double nf = 0.0;
-        // {heavy index, segment, segments of the node, the node's first partial slot}
-        const uint4 it = __ldg(a.heavy_items + idx);
-        const uint32_t hi = it.x, seg = it.y, nseg = it.z, slot = it.w;
-        const uint64_t v = __ldg(a.list + hi);
-        const uint64_t s0 = __ldg(a.off + v), s1 = __ldg(a.off + v + 1);
-        const uint64_t e0 = s0 + (uint64_t)seg * HEAVY_SEG;
-        const uint64_t e1 = nseg == 1 ? s1 : min(s1, e0 + (uint64_t)HEAVY_SEG);
-        const bool scan = !a.systolic || test_bit(a.mbc, v);
-        if (scan) {
-            uint32_t prev[NW], acc[NW];
-            if (p == 0 && seg == 0) {
-                load_chunk<LOG2M>(a.curr, v, c, prev);
-#pragma unroll
-                for (int i = 0; i < NW; i++) acc[i] = prev[i];
-            } else {
-#pragma unroll
-                for (int i = 0; i < NW; i++) acc[i] = prev[i] = 0u;
+    // The block's items are blockIdx.x, blockIdx.x + gridDim.x, ...: its
+    // threads look at 256 of them at once and list, in order, the ones with
+    // something to do, so an iteration that checks few nodes costs little.
+    for (uint64_t b0 = blockIdx.x; b0 < a.heavy_len; b0 += (uint64_t)TEAM * gridDim.x) {
+        const uint64_t mine = b0 + (uint64_t)tid * gridDim.x;
+        uint32_t kind = 0;  // 1 merge, 2 copy
+        if (mine < a.heavy_len) {
+            const uint4 it = __ldg(a.heavy_items + mine);
+            const uint32_t v = __ldg(a.list + it.x);
+            if (!a.systolic || test_bit(a.mbc, v)) kind = 1;
+            else if (it.y == 0 && test_bit(a.curr_mod, v)) kind = 2;
+        }
+        const unsigned any = __ballot_sync(0xffffffffu, kind != 0);
+        if (lane == 0) s_warp[warp] = __popc(any);
+        __syncthreads();
+        uint32_t at = 0, total = 0;
+        for (int w = 0; w < WARPS; w++) {
+            if (w < warp) at += s_warp[w];
+            total += s_warp[w];
+        }
+        if (kind) s_idx[at + __popc(any & ((1u << lane) - 1u))] = (uint32_t)tid | (kind << 16);
+        __syncthreads();
+        for (uint32_t i = 0; i < total; i++) {
+            const uint32_t e = s_idx[i];
+            // {heavy index, segment, segments of the node, the node's first partial slot}
+            const uint4 it = __ldg(a.heavy_items + b0 + (uint64_t)(e & 0xffffu) * gridDim.x);
+            const uint32_t hi = it.x, seg = it.y, nseg = it.z, slot = it.w;
+            const uint32_t v = __ldg(a.list + hi);
+            if (e >> 16 == 2) {
+                if (tid < G) {
+                    uint32_t w[NW];
+                    load_chunk<LOG2M>(a.curr, v, c, w);
+                    store_chunk<LOG2M>(a.next, v, c, w);
+                }
+                continue;
             }
-            gather_rolling<LOG2M>(a, (uint32_t)v, c, e0 + p, e1, P, !a.gather_all, acc, 0);
+            const uint64_t s0 = __ldg(a.off + v), s1 = __ldg(a.off + v + 1);
+            const uint64_t len = heavy_seg_arcs(s1 - s0, nseg);
+            const uint64_t e0 = s0 + seg * len, e1 = min(s1, e0 + len);
+            uint32_t acc[NW];
+#pragma unroll
+            for (int k = 0; k < NW; k++) acc[k] = 0u;
+            gather_rolling<LOG2M>(a, v, c, e0 + p, e1, P, !a.gather_all, acc, 0);
             __syncwarp();
+            {
+                uint32_t w[FW];
+                int first;
+                bool own;
+                reduce_scatter<NW, G, 32>(acc, w, first, own, 0xffffffffu);
+                if (own) {
 #pragma unroll
-            for (int off = G; off < 32; off <<= 1) {
-                uint32_t y[NW];
-#pragma unroll
-                for (int i = 0; i < NW; i++) y[i] = __shfl_xor_sync(0xffffffffu, acc[i], off);
-                merge_chunk<REGS>(acc, y);
-            }
-            if (lane < G) {
-#pragma unroll
-                for (int i = 0; i < NW; i++) red[warp][c][i] = acc[i];
+                    for (int k = 0; k < FW; k++) red[warp][c * NW + first + k] = w[k];
+                }
             }
             __syncthreads();
-            if (warp == 0 && lane < G) {
-                for (int w = 1; w < WARPS; w++) {
-                    uint32_t y[NW];
+            // warp 0 merges the warps' rows, each lane EW words of it
+            uint32_t w[EW];
+            if (warp == 0) {
 #pragma unroll
-                    for (int i = 0; i < NW; i++) y[i] = red[w][c][i];
-                    merge_chunk<REGS>(acc, y);
+                for (int k = 0; k < EW; k++) w[k] = elane ? red[0][lane * EW + k] : 0u;
+#pragma unroll
+                for (int q = 1; q < WARPS; q++) {
+                    uint32_t y[EW];
+#pragma unroll
+                    for (int k = 0; k < EW; k++) y[k] = elane ? red[q][lane * EW + k] : 0u;
+                    merge_chunk<4 * EW>(w, y);
                 }
             }
             bool last = true;
             if (nseg > 1) {
                 // this segment's partial into its slot, then count it in
-                if (warp == 0 && lane < G) {
-                    store_chunk<LOG2M>(a.heavy_part, (uint64_t)slot + seg, c, acc);
+                if (warp == 0) {
+                    if (elane) store_words<EW>(a.heavy_part + ((uint64_t)slot + seg) * Gm::COUNTER_BYTES + eat, w);
                     __threadfence();
+                    __syncwarp();
+                    if (lane == 0) {
+                        const uint32_t before = atomicAdd(a.heavy_arrive + slot, 1u);
+                        s_last = before == nseg - 1;
+                        __threadfence();
+                    }
+                    __syncwarp();
                 }
-                __syncthreads();
-                if (tid == 0) {
-                    const uint32_t before = atomicAdd(a.heavy_arrive + slot, 1u);
-                    s_last = before == nseg - 1;
-                    __threadfence();
-                }
-                __syncthreads();
-                last = s_last != 0;
-                if (last && warp == 0 && lane < G) {
-                    // the node's own counter and every segment's partial
-                    load_chunk<LOG2M>(a.curr, v, c, prev);
-#pragma unroll
-                    for (int i = 0; i < NW; i++) acc[i] = prev[i];
+                last = warp == 0 && s_last != 0;
+                if (last) {
                     for (uint32_t k = 0; k < nseg; k++) {
-                        uint32_t y[NW];
-                        load_chunk_cg<LOG2M>(a.heavy_part, (uint64_t)slot + k, c, y);
-                        merge_chunk<REGS>(acc, y);
+                        // written by other blocks of this launch: from L2
+                        const uint32_t* q = reinterpret_cast<const uint32_t*>(
+                            a.heavy_part + ((uint64_t)slot + k) * Gm::COUNTER_BYTES + eat);
+                        uint32_t y[EW];
+#pragma unroll
+                        for (int j = 0; j < EW; j++) y[j] = elane ? __ldcg(q + j) : 0u;
+                        merge_chunk<4 * EW>(w, y);
                     }
                     if (lane == 0) a.heavy_arrive[slot] = 0u;  // ready for the next launch
                 }
             }
-            if (last && warp == 0 && lane < G) {
-                NodeSums ns{};
-                if (c == 0) ns = load_sums(a, (uint32_t)v);
-                const bool changed = commit_node<LOG2M>(a, v, c, leader_mask, prev, acc);
-                if (c == 0) {
+            if (last && warp == 0) {
+                const uint64_t row = (uint64_t)v * Gm::COUNTER_BYTES + eat;
+                uint32_t prev[EW], diff = 0;
+#pragma unroll
+                for (int k = 0; k < EW; k++) prev[k] = 0u;
+                if (elane) load_words<EW>(a.curr + row, prev);
+                merge_chunk<4 * EW>(w, prev);
+#pragma unroll
+                for (int k = 0; k < EW; k++) diff |= w[k] ^ prev[k];
+                if (elane) store_words<EW>(a.next + row, w);
+                const bool changed = __any_sync(0xffffffffu, diff != 0u);
+                uint64_t hs = 0;
+                uint32_t z = 0, c31 = 0;
+                if (changed) count_lanes<EW, 1, 32>(a, w, elane, 0xffffffffu, hs, z, c31);
+                if (lane == 0) {
                     scanned++;
                     sarcs += (uint32_t)(s1 - s0);
                     if (changed) {
                         atomicOr(a.next_mod + (v >> 5), 1u << (v & 31));
                         modc++;
                     }
+                    double nf = 0.0;
+                    finish_scalars<LOG2M>(a, v, hs, z, c31, changed, load_sums(a, v), nf, vis);
+                    a.nf_items[a.heavy_item_base + hi] = nf;
                 }
-                finish_node<LOG2M>(a, (uint32_t)v, c, leader_mask, acc, changed, ns, nf, vis);
-                if (c == 0) a.nf_items[a.heavy_item_base + hi] = nf;
             }
-        } else if (seg == 0 && test_bit(a.curr_mod, v)) {
-            if (tid < G) {
-                uint32_t prev[NW];
-                load_chunk<LOG2M>(a.curr, v, c, prev);
-                store_chunk<LOG2M>(a.next, v, c, prev);
-            }
+            __syncthreads();
         }
-        __syncthreads();
     }
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
@@ -1416,7 +1519,7 @@ __device__ __forceinline__ uint32_t add_hash(uint8_t* counter, uint64_t x) {
 template <int LOG2M>
 __global__ void __launch_bounds__(256) k_init(InitArgs a) {
     using Gm = Geo<LOG2M>;
-    bool saw31 = false;
+    bool saw_big = false;
     for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < a.n;
          v += (uint64_t)gridDim.x * blockDim.x) {
         uint8_t* counter = a.curr + v * (uint64_t)Gm::COUNTER_BYTES;
@@ -1425,7 +1528,7 @@ __global__ void __launch_bounds__(256) k_init(InitArgs a) {
             const uint64_t u = a.hash_id ? __ldg(a.hash_id + v) : __ldg(a.perm + v);
             const uint64_t x = a.hash_kind == 1 ? hash_jenkins(u, a.seed) : hash_sip13(u);
             const uint32_t val = add_hash<LOG2M>(counter, x);
-            saw31 |= val == 31u;
+            saw_big |= val >= 30u;
             // one register holds val, the other m-1 are zero
             const uint64_t hs = (uint64_t)(Gm::M - 1) * 0x80000000ull + (uint64_t)(0x80000000u >> val);
             const uint32_t c31 = val == 31u;
@@ -1444,7 +1547,7 @@ __global__ void __launch_bounds__(256) k_init(InitArgs a) {
                 z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
                 z ^= z >> 31;
                 const uint64_t x = a.hash_kind == 1 ? hash_jenkins(z, a.seed) : hash_sip13(z);
-                saw31 |= add_hash<LOG2M>(counter, x) == 31u;
+                saw_big |= add_hash<LOG2M>(counter, x) >= 30u;
             }
             uint64_t hs = 0;
             uint32_t z = 0, c31 = 0;
@@ -1459,8 +1562,8 @@ __global__ void __launch_bounds__(256) k_init(InitArgs a) {
         }
     }
     // Registers only ever take values some initial register had; remember
-    // whether 31 occurs so counts can skip looking for it.
-    if (__syncthreads_or(saw31) && threadIdx.x == 0) atomicOr(a.any31, 1);
+    // whether 30 or 31 occurs, which the fast form of the counts excludes.
+    if (__syncthreads_or(saw_big) && threadIdx.x == 0) atomicOr(a.any31, 1);
 }
 
 // ---------------------------------------------------------------------------

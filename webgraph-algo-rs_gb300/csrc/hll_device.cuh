@@ -89,25 +89,48 @@ __device__ __forceinline__ uint32_t zero_bytes(uint32_t w) {
     return 4u - __popc(((w | 0x80808080u) - 0x01010101u) & 0x80808080u);
 }
 
-// Partial count of one chunk: hsum += sum over registers of 2^(31-v),
-// zeroes += #(v == 0), and, only when `with31`, c31 += #(v == 31).
-// 2^(31-v): funnel-shifting 0x80000000 right uses the shift amount mod 32, so
-// the word shifted right by 8k gives register k's term without masking.
-template <int REGS>
-__device__ __forceinline__ void count_chunk(const uint32_t (&w)[REGS / 4], uint64_t& hsum,
-                                            uint32_t& zeroes, uint32_t& c31, bool with31) {
-    uint32_t lo = 0, hi = 0;
+// Sum over the registers of W words of 2^(31-v) (shares of a counter add), and
+// the registers holding 31. Funnel-shifting uses the shift amount mod 32, so the
+// word shifted right by 8k gives register k's term without masking. Without
+// registers above 29 (`big` false) a word's four terms, scaled by 2^-2, add
+// exactly in 32 bits: 9 instructions a word and a 64-bit add, where a 64-bit
+// sum of single terms took 16. With the zero registers counted only where the
+// small-range correction may apply, 32 nodes of one arc take 733 warp
+// instructions at log2m 6 instead of 881.
+template <int W>
+__device__ __forceinline__ uint64_t sum_words(const uint32_t (&w)[W], bool big, uint32_t& c31) {
+    uint64_t sum = 0;
+    c31 = 0;
+    if (big) {
+        uint32_t lo = 0, hi = 0;
 #pragma unroll
-    for (int i = 0; i < REGS / 4; i++) {
+        for (int i = 0; i < W; i++) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const uint32_t term = __funnelshift_r(0x80000000u, 0u, w[i] >> (8 * k));
-            asm("add.cc.u32 %0, %0, %2;\n\taddc.u32 %1, %1, 0;" : "+r"(lo), "+r"(hi) : "r"(term));
+            for (int k = 0; k < 4; k++) {
+                const uint32_t term = __funnelshift_r(0x80000000u, 0u, w[i] >> (8 * k));
+                asm("add.cc.u32 %0, %0, %2;\n\taddc.u32 %1, %1, 0;" : "+r"(lo), "+r"(hi) : "r"(term));
+            }
+            c31 += zero_bytes(w[i] ^ 0x1f1f1f1fu);
         }
-        zeroes += zero_bytes(w[i]);
-        if (with31) c31 += zero_bytes(w[i] ^ 0x1f1f1f1fu);
+        return ((uint64_t)hi << 32) | lo;
     }
-    hsum += ((uint64_t)hi << 32) | lo;
+#pragma unroll
+    for (int i = 0; i < W; i++) {
+        uint32_t t = __funnelshift_r(0x20000000u, 0u, w[i]);
+#pragma unroll
+        for (int k = 1; k < 4; k++) t += __funnelshift_r(0x20000000u, 0u, w[i] >> (8 * k));
+        sum += t;
+    }
+    return sum << 2;
+}
+
+// zero registers of W words
+template <int W>
+__device__ __forceinline__ uint32_t zero_words(const uint32_t (&w)[W]) {
+    uint32_t z = 0;
+#pragma unroll
+    for (int i = 0; i < W; i++) z += zero_bytes(w[i]);
+    return z;
 }
 
 // HLL:181-185 from the exact integer harmonic sum (reference arithmetic, f64

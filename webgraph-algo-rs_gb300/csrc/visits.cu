@@ -6,23 +6,15 @@
 // State: the graph in device CSR, a visited bitmap that persists across
 // visits until hb_visit_reset (par_fair.rs:101, 322-324), and a queue that
 // holds every node visited since the last reset in visit order, with its
-// predecessor. A visit is level-synchronous like the reference's frontier
-// loop (par_fair.rs:169-213):
-//   k_visit_roots   roots not yet visited are marked and form level 0;
-//   k_visit_expand  one warp per frontier node walks its successors 32 at a
-//                   time; a successor whose visited bit a lane sets first
-//                   (atomicOr, after a plain read that skips the common
-//                   already-visited case) is staged with its predecessor
-//                   in the warp's run in shared memory, and a run goes to
-//                   the next level with one atomicAdd on the tail per up to
-//                   RUN nodes; nodes with more than HEAVY_MIN successors
-//                   are deferred to
-//   k_visit_heavy   one block per node.
+// predecessor and distance. A visit is level-synchronous like the reference's
+// frontier loop (par_fair.rs:169-213): hbl::k_starts marks the roots not yet
+// visited, hbl::k_level (visit_level.cuh) claims a level's successors; levels are
+// launched as many at a time as the last visit took, and the host looks when
+// they are through.
 // The Unknown events of the reference (node, pred, distance) are the queue
-// slots of the visit with the level of each slot; Known events are counted.
-// Within a level the order is unspecified, as in the reference's parallel
-// visit; distances are exact, and the predecessor of a node is a node of
-// the previous level with an arc to it.
+// slots of the visit; Known events are counted. Within a level the order is
+// unspecified, as in the reference's parallel visit; distances are exact, and
+// the predecessor of a node is a node of the previous level with an arc to it.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -32,146 +24,9 @@
 #include <vector>
 
 #include "hb_internal.h"
+#include "visit_level.cuh"
 
 namespace hbv {
-
-constexpr uint32_t HEAVY_MIN = 4096;
-
-__device__ __forceinline__ bool claim(uint32_t* visited, uint32_t s) {
-    const uint32_t w = s >> 5, bit = 1u << (s & 31);
-    if (*(volatile uint32_t*)(visited + w) & bit) return false;
-    return !(atomicOr(visited + w, bit) & bit);
-}
-
-// appends the lanes' claimed nodes (warp-aggregated), with predecessor p
-__device__ __forceinline__ void append(bool c, uint32_t s, uint32_t p, uint32_t* queue, uint32_t* pred,
-                                       unsigned long long* tail) {
-    const unsigned mask = __ballot_sync(0xffffffffu, c);
-    if (!mask) return;
-    const int lane = threadIdx.x & 31;
-    unsigned long long base = 0;
-    if (lane == __ffs(mask) - 1) base = atomicAdd(tail, (unsigned long long)__popc(mask));
-    base = __shfl_sync(0xffffffffu, base, __ffs(mask) - 1);
-    if (c) {
-        const unsigned long long slot = base + __popc(mask & ((1u << lane) - 1u));
-        queue[slot] = s;
-        pred[slot] = p;
-    }
-}
-
-// A warp's claimed nodes and their predecessors wait in shared memory and
-// go to the queue in runs of up to RUN slots: a per-chunk append puts one
-// same-address atomic on the tail in the chain of almost every frontier
-// node of a level of many small-degree nodes.
-constexpr int RUN = 128;
-constexpr int EXPAND_THREADS = 256;
-
-// writes the warp's run [0, fill) to the queue (every lane of the warp)
-__device__ __forceinline__ void write_run(const uint32_t* rn, const uint32_t* rp, int fill, uint32_t* queue,
-                                          uint32_t* pred, unsigned long long* tail) {
-    __syncwarp();
-    const int lane = threadIdx.x & 31;
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(tail, (unsigned long long)fill);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    for (int k = lane; k < fill; k += 32) {
-        queue[base + k] = rn[k];
-        pred[base + k] = rp[k];
-    }
-    __syncwarp();
-}
-
-// adds the lanes' claimed nodes (predecessor p) to the warp's run, writing
-// the run out when another chunk might not fit (every lane of the warp)
-__device__ __forceinline__ void stage(bool c, uint32_t s, uint32_t p, uint32_t* rn, uint32_t* rp, int& fill,
-                                      uint32_t* queue, uint32_t* pred, unsigned long long* tail) {
-    const unsigned mask = __ballot_sync(0xffffffffu, c);
-    if (c) {
-        const int k = fill + __popc(mask & ((1u << (threadIdx.x & 31)) - 1u));
-        rn[k] = s;
-        rp[k] = p;
-    }
-    fill += __popc(mask);
-    if (fill > RUN - 32) {
-        write_run(rn, rp, fill, queue, pred, tail);
-        fill = 0;
-    }
-}
-
-__global__ void k_visit_roots(const uint32_t* __restrict__ roots, uint64_t nroots, uint32_t* visited,
-                              uint32_t* queue, uint32_t* pred, unsigned long long* tail) {
-    // whole warps iterate together (the limit is a multiple of 32) so that
-    // every lane of a warp takes part in the append
-    const uint64_t limit = (nroots + 31) & ~31ull;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < limit;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const bool in = i < nroots;
-        const uint32_t r = in ? roots[i] : 0u;
-        const bool c = in && claim(visited, r);
-        append(c, r, r, queue, pred, tail);
-    }
-}
-
-// level [b, e) of the queue -> the next level, appended at *tail
-__global__ void k_visit_expand(const uint64_t* __restrict__ off, const uint32_t* __restrict__ succ,
-                               uint32_t* visited, uint32_t* queue, uint32_t* pred, uint64_t b,
-                               uint64_t e, unsigned long long* tail, uint32_t* heavy,
-                               unsigned long long* heavy_n, unsigned long long* known) {
-    __shared__ uint32_t run_node[EXPAND_THREADS / 32][RUN], run_pred[EXPAND_THREADS / 32][RUN];
-    uint32_t* rn = run_node[threadIdx.x >> 5];
-    uint32_t* rp = run_pred[threadIdx.x >> 5];
-    int fill = 0;  // the same in every lane of the warp
-    const int lane = threadIdx.x & 31;
-    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    unsigned long long kn = 0;
-    for (uint64_t i = b + warp; i < e; i += warps) {
-        const uint32_t v = queue[i];
-        const uint64_t s0 = off[v], s1 = off[v + 1];
-        if (s1 - s0 > HEAVY_MIN) {
-            if (lane == 0) heavy[atomicAdd(heavy_n, 1ull)] = v;
-            continue;
-        }
-        for (uint64_t a = s0; a < s1; a += 32) {
-            const uint64_t x = a + lane;
-            uint32_t s = 0;
-            bool c = false;
-            if (x < s1) {
-                s = __ldg(succ + x);
-                c = claim(visited, s);
-                kn += !c;
-            }
-            stage(c, s, v, rn, rp, fill, queue, pred, tail);
-        }
-    }
-    if (fill) write_run(rn, rp, fill, queue, pred, tail);
-    if (kn) atomicAdd(known, kn);
-}
-
-// the deferred nodes of a level, one block each
-__global__ void k_visit_heavy(const uint64_t* __restrict__ off, const uint32_t* __restrict__ succ,
-                              uint32_t* visited, uint32_t* queue, uint32_t* pred,
-                              unsigned long long* tail, const uint32_t* heavy,
-                              const unsigned long long* heavy_n, unsigned long long* known) {
-    const uint64_t count = *heavy_n;
-    unsigned long long kn = 0;
-    for (uint64_t h = blockIdx.x; h < count; h += gridDim.x) {
-        const uint32_t v = heavy[h];
-        const uint64_t s0 = off[v], s1 = off[v + 1];
-        for (uint64_t a = s0; a < s1; a += blockDim.x) {
-            const uint64_t x = a + threadIdx.x;
-            uint32_t s = 0;
-            bool c = false;
-            if (x < s1) {
-                s = __ldg(succ + x);
-                c = claim(visited, s);
-                kn += !c;
-            }
-            append(c, s, v, queue, pred, tail);
-        }
-    }
-    if (kn) atomicAdd(known, kn);
-}
 
 __global__ void k_visit_validate(const uint64_t* __restrict__ off, const uint32_t* __restrict__ succ,
                                  uint64_t n, uint64_t m, int* bad) {
@@ -193,12 +48,19 @@ struct hb_visit {
     uint64_t* d_off = nullptr;
     uint32_t* d_succ = nullptr;
     uint32_t* d_visited = nullptr;
-    uint32_t* d_queue = nullptr;   // every node visited since the last reset, in visit order
+    uint32_t* d_queue = nullptr;   // every node visited since the last reset, in visit order,
+    hbl::Entry* d_info = nullptr;
+    hbl::Entry* d_entry = nullptr; // its entry in its level,
+    uint32_t* d_tile[2] = {nullptr, nullptr};
+    uint32_t* d_qpred = nullptr;   // its predecessor
+    uint32_t* d_qdist = nullptr;   // and distance
+    uint32_t* d_dist = nullptr;    // hb_visit_each: distance and predecessor by node (allocated there)
     uint32_t* d_pred = nullptr;
-    uint32_t* d_heavy = nullptr;
     uint32_t* d_roots = nullptr;   // roots of the current visit (capacity n)
-    unsigned long long* d_cnt = nullptr;   // [0] tail, [1] deferred nodes, [2] known arcs
-    unsigned long long* h_cnt = nullptr;   // page-locked copy
+    hbl::Control* d_ctl = nullptr;
+    hbl::Control* h_ctl = nullptr; // page-locked copy
+    int* d_bad = nullptr;
+    int ahead = 2;                 // level launches of the next visit
     uint64_t tail = 0;
     int sms = 1;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -229,6 +91,65 @@ static int visit_cuda(hb_visit* v, cudaError_t e, const char* what) {
         if (_r) return _r;                              \
     } while (0)
 
+// One visit from the given roots; dist and pred (by node, device) get its
+// nodes' entries, or are null. On return the stream is idle.
+static int visit_levels(hb_visit* v, const uint64_t* roots, size_t nroots, uint64_t max_distance, uint32_t* dist,
+                        uint32_t* pred, hb_visit_stats& st) {
+    if (nroots == 0) return HB_OK;
+    cudaStream_t s = v->stream;
+    const uint64_t q0 = v->tail;
+    hbl::Level a{};
+    a.info = v->d_info;
+    a.succ = v->d_succ;
+    a.visited = v->d_visited;
+    a.dist = dist;
+    a.pred = pred;
+    a.queue = v->d_queue;
+    a.entry = v->d_entry;
+    a.qpred = v->d_qpred;
+    a.qdist = v->d_qdist;
+    a.ctl = v->d_ctl;
+    a.max_d = (uint32_t)std::min<uint64_t>(max_distance, 0xffffffffull);
+    a.tile[0] = v->d_tile[0];
+    a.tile[1] = v->d_tile[1];
+    a.n = v->n;
+    a.small = hbl::small_units(v->n, v->m);
+    std::vector<uint32_t> r32(nroots);
+    for (size_t i = 0; i < nroots; i++) r32[i] = (uint32_t)roots[i];
+    *v->h_ctl = hbl::Control{};
+    v->h_ctl->tail = q0;
+    VC(v, cudaMemcpyAsync(v->d_ctl, v->h_ctl, sizeof(hbl::Control), cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
+    VC(v, cudaEventRecord(v->ev0, s), "cudaEventRecord");
+    // d_roots holds n roots: longer lists (repeated roots) go in pieces
+    const uint64_t nr = std::min<uint64_t>(nroots, std::max<uint64_t>(v->n, 1));
+    for (size_t at = 0; at < nroots; at += nr) {
+        const uint64_t k = std::min<uint64_t>(nr, nroots - at);
+        // the next piece's copy must not overwrite roots still being read
+        if (at) VC(v, cudaStreamSynchronize(s), "cudaStreamSynchronize");
+        VC(v, cudaMemcpyAsync(v->d_roots, r32.data() + at, k * 4, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
+        VC(v, hbl::launch_starts<true>(a, v->d_roots, k, (uint32_t)q0, at + nr >= nroots, v->sms, s), "k_starts");
+    }
+    // levels, as many launches as the last visit took; one past the last level does nothing
+    int in = 0;
+    for (int k = v->ahead;; k = 2) {
+        VC(v, (hbl::launch_levels<false, true>(a, k, in, v->sms, s)), "k_level");
+        VC(v, cudaEventRecord(v->ev1, s), "cudaEventRecord");
+        VC(v, cudaMemcpyAsync(v->h_ctl, v->d_ctl, sizeof(hbl::Control), cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
+        VC(v, cudaStreamSynchronize(s), "cudaStreamSynchronize");
+        if (hbl::done(v->h_ctl->st[0], a.max_d)) break;
+    }
+    const hbl::Control& c = *v->h_ctl;
+    v->ahead = (int)std::max<uint32_t>(1, std::min<uint32_t>(c.launches, 64));
+    v->tail = c.st[0].e;
+    st.visited = v->tail - q0;
+    st.levels = st.visited ? c.st[0].last + 1 : 0;
+    st.known_arcs = c.known;
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, v->ev0, v->ev1);
+    st.device_ms = ms;
+    return HB_OK;
+}
+
 static void visit_free(hb_visit* v) {
     if (!v) return;
     cudaSetDevice(v->device);
@@ -237,11 +158,18 @@ static void visit_free(hb_visit* v) {
     cudaFree(v->d_succ);
     cudaFree(v->d_visited);
     cudaFree(v->d_queue);
+    cudaFree(v->d_info);
+    cudaFree(v->d_entry);
+    cudaFree(v->d_tile[0]);
+    cudaFree(v->d_tile[1]);
+    cudaFree(v->d_qpred);
+    cudaFree(v->d_qdist);
+    cudaFree(v->d_dist);
     cudaFree(v->d_pred);
-    cudaFree(v->d_heavy);
     cudaFree(v->d_roots);
-    cudaFree(v->d_cnt);
-    if (v->h_cnt) cudaFreeHost(v->h_cnt);
+    cudaFree(v->d_ctl);
+    cudaFree(v->d_bad);
+    if (v->h_ctl) cudaFreeHost(v->h_ctl);
     if (v->ev0) cudaEventDestroy(v->ev0);
     if (v->ev1) cudaEventDestroy(v->ev1);
     if (v->own_stream && v->stream) cudaStreamDestroy(v->stream);
@@ -290,11 +218,16 @@ int hb_visit_create(const hb_graph_view* g, int device, void* stream, hb_visit**
         (r = visit_cuda(v, cudaMalloc((void**)&v->d_succ, std::max<uint64_t>(m, 1) * 4), "cudaMalloc")) ||
         (r = visit_cuda(v, cudaMalloc((void**)&v->d_visited, std::max<uint64_t>(words, 1) * 4), "cudaMalloc")) ||
         (r = visit_cuda(v, cudaMalloc((void**)&v->d_queue, nn * 4), "cudaMalloc")) ||
-        (r = visit_cuda(v, cudaMalloc((void**)&v->d_pred, nn * 4), "cudaMalloc")) ||
-        (r = visit_cuda(v, cudaMalloc((void**)&v->d_heavy, nn * 4), "cudaMalloc")) ||
+        (r = visit_cuda(v, cudaMalloc((void**)&v->d_info, nn * sizeof(hbl::Entry)), "cudaMalloc")) ||
+        (r = visit_cuda(v, cudaMalloc((void**)&v->d_entry, nn * sizeof(hbl::Entry)), "cudaMalloc")) ||
+        (r = visit_cuda(v, cudaMalloc((void**)&v->d_tile[0], hbl::tiles(n, m) * 4), "cudaMalloc")) ||
+        (r = visit_cuda(v, cudaMalloc((void**)&v->d_tile[1], hbl::tiles(n, m) * 4), "cudaMalloc")) ||
+        (r = visit_cuda(v, cudaMalloc((void**)&v->d_qpred, nn * 4), "cudaMalloc")) ||
+        (r = visit_cuda(v, cudaMalloc((void**)&v->d_qdist, nn * 4), "cudaMalloc")) ||
         (r = visit_cuda(v, cudaMalloc((void**)&v->d_roots, nn * 4), "cudaMalloc")) ||
-        (r = visit_cuda(v, cudaMalloc((void**)&v->d_cnt, 4 * 8), "cudaMalloc")) ||
-        (r = visit_cuda(v, cudaMallocHost((void**)&v->h_cnt, 4 * 8), "cudaMallocHost")))
+        (r = visit_cuda(v, cudaMalloc((void**)&v->d_ctl, sizeof(hbl::Control)), "cudaMalloc")) ||
+        (r = visit_cuda(v, cudaMalloc((void**)&v->d_bad, sizeof(int)), "cudaMalloc")) ||
+        (r = visit_cuda(v, cudaMallocHost((void**)&v->h_ctl, sizeof(hbl::Control)), "cudaMallocHost")))
         return fail(r);
     if ((r = visit_cuda(v, cudaMemcpyAsync(v->d_off, g->offsets, (n + 1) * 8, cudaMemcpyHostToDevice, v->stream),
                         "cudaMemcpyAsync")))
@@ -304,7 +237,7 @@ int hb_visit_create(const hb_graph_view* g, int device, void* stream, hb_visit**
                              "cudaMemcpyAsync")))
         return fail(r);
     // the CSR is checked before any kernel indexes with it
-    int* d_bad = (int*)(v->d_cnt + 3);
+    int* d_bad = v->d_bad;
     int bad = 0;
     if ((r = visit_cuda(v, cudaMemsetAsync(d_bad, 0, sizeof(int), v->stream), "cudaMemsetAsync"))) return fail(r);
     const int grid = (int)std::min<uint64_t>((std::max(n, m) + 255) / 256 + 1, 8192);
@@ -315,6 +248,8 @@ int hb_visit_create(const hb_graph_view* g, int device, void* stream, hb_visit**
         (r = visit_cuda(v, cudaStreamSynchronize(v->stream), "cudaStreamSynchronize")))
         return fail(r);
     if (bad) return fail(visit_err(v, HB_ERR_INVALID, "graph has decreasing offsets or successors >= num_nodes"));
+    hbl::k_info<<<(int)std::min<uint64_t>(n / 256 + 1, 8192), 256, 0, v->stream>>>(v->d_off, n, v->d_info);
+    if ((r = visit_cuda(v, cudaGetLastError(), "k_info"))) return fail(r);
     v->host_visited.assign(std::max<uint64_t>(words, 1), 0);
     if ((r = visit_cuda(v, cudaEventCreate(&v->ev0), "cudaEventCreate")) ||
         (r = visit_cuda(v, cudaEventCreate(&v->ev1), "cudaEventCreate")))
@@ -347,79 +282,20 @@ int hb_visit_run(hb_visit* v, const uint64_t* roots, size_t nroots, uint64_t max
     for (size_t i = 0; i < nroots; i++)
         if (roots[i] >= v->n) return visit_err(v, HB_ERR_INVALID, "root " + std::to_string(roots[i]) + " >= num_nodes");
     VC(v, cudaSetDevice(v->device), "cudaSetDevice");
-    cudaStream_t s = v->stream;
     hb_visit_stats st{};
     const uint64_t q0 = v->tail;
-    std::vector<uint64_t> level_end;
-    if (nroots) {
-        std::vector<uint32_t> r32(nroots);
-        for (size_t i = 0; i < nroots; i++) r32[i] = (uint32_t)roots[i];
-        // d_roots holds n roots: longer lists (repeated roots) go in pieces
-        const uint64_t nr = std::min<uint64_t>(nroots, std::max<uint64_t>(v->n, 1));
-        unsigned long long zero2[3] = {q0, 0, 0};
-        VC(v, cudaMemcpyAsync(v->d_cnt, zero2, 3 * 8, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
-        VC(v, cudaEventRecord(v->ev0, s), "cudaEventRecord");
-        for (size_t at = 0; at < nroots; at += nr) {
-            const uint64_t k = std::min<uint64_t>(nr, nroots - at);
-            VC(v, cudaMemcpyAsync(v->d_roots, r32.data() + at, k * 4, cudaMemcpyHostToDevice, s),
-               "cudaMemcpyAsync");
-            const int grid = (int)std::min<uint64_t>((k + 31 + 255) / 256, 4096);
-            hbv::k_visit_roots<<<grid, 256, 0, s>>>(v->d_roots, k, v->d_visited, v->d_queue, v->d_pred,
-                                                    v->d_cnt);
-            VC(v, cudaGetLastError(), "k_visit_roots");
-            // the next piece's copy must not overwrite roots still being read
-            VC(v, cudaStreamSynchronize(s), "cudaStreamSynchronize");
-        }
-        VC(v, cudaMemcpyAsync(v->h_cnt, v->d_cnt, 8, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
-        VC(v, cudaStreamSynchronize(s), "cudaStreamSynchronize");
-        uint64_t b = q0, e = v->h_cnt[0];
-        if (e > b) level_end.push_back(e);
-        const int egrid = v->sms * 8, hgrid = v->sms * 2;
-        uint64_t d = 0;
-        while (e > b && d < max_distance) {
-            VC(v, cudaMemsetAsync(v->d_cnt + 1, 0, 8, s), "cudaMemsetAsync");
-            const int g1 = (int)std::min<uint64_t>(((e - b) * 32 + hbv::EXPAND_THREADS - 1) / hbv::EXPAND_THREADS,
-                                                   (uint64_t)egrid);
-            hbv::k_visit_expand<<<g1, hbv::EXPAND_THREADS, 0, s>>>(v->d_off, v->d_succ, v->d_visited, v->d_queue, v->d_pred,
-                                                   b, e, v->d_cnt, v->d_heavy, v->d_cnt + 1, v->d_cnt + 2);
-            VC(v, cudaGetLastError(), "k_visit_expand");
-            hbv::k_visit_heavy<<<hgrid, 256, 0, s>>>(v->d_off, v->d_succ, v->d_visited, v->d_queue, v->d_pred,
-                                                     v->d_cnt, v->d_heavy, v->d_cnt + 1, v->d_cnt + 2);
-            VC(v, cudaGetLastError(), "k_visit_heavy");
-            VC(v, cudaMemcpyAsync(v->h_cnt, v->d_cnt, 8, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
-            VC(v, cudaStreamSynchronize(s), "cudaStreamSynchronize");
-            b = e;
-            e = v->h_cnt[0];
-            if (e > b) level_end.push_back(e);
-            d++;
-        }
-        VC(v, cudaEventRecord(v->ev1, s), "cudaEventRecord");
-        VC(v, cudaMemcpyAsync(v->h_cnt, v->d_cnt, 3 * 8, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
-        VC(v, cudaStreamSynchronize(s), "cudaStreamSynchronize");
-        v->tail = v->h_cnt[0];
-        st.known_arcs = v->h_cnt[2];
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, v->ev0, v->ev1);
-        st.device_ms = ms;
-    }
-    const uint64_t count = v->tail - q0;
-    st.visited = count;
-    st.levels = level_end.size();
+    if (int r = visit_levels(v, roots, nroots, max_distance, nullptr, nullptr, st)) return r;
+    const uint64_t count = st.visited;
     // the events into the caller's buffers
     if (count && (nodes || preds || dists)) {
         const size_t k = std::min<uint64_t>(capacity, count);
         if (nodes)
-            VC(v, cudaMemcpyAsync(nodes, v->d_queue + q0, k * 4, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
+            VC(v, cudaMemcpyAsync(nodes, v->d_queue + q0, k * 4, cudaMemcpyDeviceToHost, v->stream), "cudaMemcpyAsync");
         if (preds)
-            VC(v, cudaMemcpyAsync(preds, v->d_pred + q0, k * 4, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
-        VC(v, cudaStreamSynchronize(s), "cudaStreamSynchronize");
-        if (dists) {
-            uint64_t lvl = 0;
-            for (uint64_t i = 0; i < k; i++) {
-                while (lvl < level_end.size() && q0 + i >= level_end[lvl]) lvl++;
-                dists[i] = (uint32_t)lvl;
-            }
-        }
+            VC(v, cudaMemcpyAsync(preds, v->d_qpred + q0, k * 4, cudaMemcpyDeviceToHost, v->stream), "cudaMemcpyAsync");
+        if (dists)
+            VC(v, cudaMemcpyAsync(dists, v->d_qdist + q0, k * 4, cudaMemcpyDeviceToHost, v->stream), "cudaMemcpyAsync");
+        VC(v, cudaStreamSynchronize(v->stream), "cudaStreamSynchronize");
     }
     if (stats) *stats = st;
     if (capacity < count)
@@ -433,30 +309,62 @@ int hb_visit_each(hb_visit* v, const uint64_t* roots, size_t nroots, uint32_t* d
     if (!v) return visit_err(nullptr, HB_ERR_INVALID, "visit is NULL");
     if ((dist && len != v->n) || (pred && len != v->n))
         return visit_err(v, HB_ERR_INVALID, "dist and pred must hold num_nodes entries");
-    std::vector<uint32_t> nodes(v->n), preds(pred ? v->n : 0), ds(v->n);
     const uint64_t words = (v->n + 31) / 32;
-    if (words) {
-        VC(v, cudaSetDevice(v->device), "cudaSetDevice");
-        VC(v, cudaMemcpyAsync(v->host_visited.data(), v->d_visited, words * 4, cudaMemcpyDeviceToHost,
-                              v->stream),
-           "cudaMemcpyAsync");
-        VC(v, cudaStreamSynchronize(v->stream), "cudaStreamSynchronize");
+    if (nroots == 0 || words == 0)
+        return nroots ? visit_err(v, HB_ERR_INVALID, "root " + std::to_string(roots[0]) + " >= num_nodes") : HB_OK;
+    VC(v, cudaSetDevice(v->device), "cudaSetDevice");
+    cudaStream_t s = v->stream;
+    VC(v, cudaMemcpyAsync(v->host_visited.data(), v->d_visited, words * 4, cudaMemcpyDeviceToHost, s),
+       "cudaMemcpyAsync");
+    // the caller's entries, which the visits write over by node on the device
+    // (in place of a pass of scattered host writes over the events)
+    if (dist) {
+        if (!v->d_dist) VC(v, cudaMalloc((void**)&v->d_dist, v->n * 4), "cudaMalloc");
+        VC(v, cudaMemcpyAsync(v->d_dist, dist, v->n * 4, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
     }
-    for (size_t i = 0; i < nroots; i++) {
+    if (pred) {
+        if (!v->d_pred) VC(v, cudaMalloc((void**)&v->d_pred, v->n * 4), "cudaMalloc");
+        VC(v, cudaMemcpyAsync(v->d_pred, pred, v->n * 4, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
+    }
+    VC(v, cudaStreamSynchronize(s), "cudaStreamSynchronize");
+    int rc = HB_OK;
+    bool wrote = false;
+    std::vector<uint32_t> nodes;
+    for (size_t i = 0; i < nroots && rc == HB_OK; i++) {
         const uint64_t r = roots[i];
-        if (r >= v->n) return visit_err(v, HB_ERR_INVALID, "root " + std::to_string(r) + " >= num_nodes");
+        if (r >= v->n) {
+            rc = visit_err(v, HB_ERR_INVALID, "root " + std::to_string(r) + " >= num_nodes");
+            break;
+        }
         if ((v->host_visited[r >> 5] >> (r & 31)) & 1) continue;  // seq.rs:130: already visited
         hb_visit_stats st{};
-        int rc = hb_visit_run(v, &r, 1, UINT64_MAX, nodes.data(), pred ? preds.data() : nullptr, ds.data(),
-                              v->n, &st);
-        if (rc) return rc;
-        for (uint64_t k = 0; k < st.visited; k++) {
-            if (dist) dist[nodes[k]] = ds[k];
-            if (pred) pred[nodes[k]] = preds[k];
-            v->host_visited[nodes[k] >> 5] |= 1u << (nodes[k] & 31);
+        const uint64_t q0 = v->tail;
+        rc = visit_levels(v, &r, 1, UINT64_MAX, dist ? v->d_dist : nullptr, pred ? v->d_pred : nullptr, st);
+        wrote = true;
+        if (rc != HB_OK || i + 1 == nroots) break;
+        // what is visited by now, for the next roots: the bitmap, or the few nodes of a small visit
+        if (st.visited > words) {
+            rc = visit_cuda(v, cudaMemcpyAsync(v->host_visited.data(), v->d_visited, words * 4, cudaMemcpyDeviceToHost, s),
+                            "cudaMemcpyAsync");
+        } else {
+            nodes.resize(st.visited);
+            rc = visit_cuda(v, cudaMemcpyAsync(nodes.data(), v->d_queue + q0, st.visited * 4, cudaMemcpyDeviceToHost, s),
+                            "cudaMemcpyAsync");
         }
+        if (rc == HB_OK) rc = visit_cuda(v, cudaStreamSynchronize(s), "cudaStreamSynchronize");
+        if (rc == HB_OK && st.visited <= words)
+            for (uint32_t x : nodes) v->host_visited[x >> 5] |= 1u << (x & 31);
     }
-    return HB_OK;
+    if (wrote) {
+        int e = HB_OK;
+        if (dist)
+            e = visit_cuda(v, cudaMemcpyAsync(dist, v->d_dist, v->n * 4, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
+        if (pred && e == HB_OK)
+            e = visit_cuda(v, cudaMemcpyAsync(pred, v->d_pred, v->n * 4, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
+        if (e == HB_OK) e = visit_cuda(v, cudaStreamSynchronize(s), "cudaStreamSynchronize");
+        if (rc == HB_OK) rc = e;
+    }
+    return rc;
 }
 
 const char* hb_visit_last_error(const hb_visit* v) { return v ? v->err.c_str() : t_visit_err.c_str(); }

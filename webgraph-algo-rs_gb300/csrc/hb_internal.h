@@ -162,6 +162,12 @@ int launch_relabel_arcs(const uint64_t* off, uint64_t n, uint64_t m, const uint3
 // transpose scatter with per-row cursors (positions of the next arc of each row)
 int launch_scatter_arcs(const uint64_t* off, uint64_t n, uint64_t m, const uint32_t* tile_start,
                         const uint32_t* succ, unsigned long long* cursor, uint32_t* tsucc, void* stream);
+// arcs between components (comp by node), in arc order: with src null their
+// number per arc tile into count; else their ends into src and dst, at holding
+// the exclusive scan of the counts (arc_tiles(m) + 1 words)
+int launch_cross_arcs(const uint64_t* off, uint64_t n, uint64_t m, const uint32_t* tile_start, const uint32_t* succ,
+                      const uint32_t* comp, unsigned long long* count, const uint64_t* at, uint32_t* src, uint32_t* dst,
+                      void* stream);
 // dst[u] = src[inv[u]]: a per-node array back to caller order
 int launch_gather_f64(const double* src, const uint32_t* inv, double* dst, uint64_t n,
                       void* stream);

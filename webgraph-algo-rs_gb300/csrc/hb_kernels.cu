@@ -1825,6 +1825,60 @@ __global__ void __launch_bounds__(LBS_THREADS) k_scatter_arcs(
     }
 }
 
+// The arcs whose two ends lie in different components, in arc order. First
+// pass (src null): their number in every tile, into count. Second pass: their
+// ends, from slot at[tile] on.
+__global__ void __launch_bounds__(LBS_THREADS) k_cross_arcs(
+    const uint64_t* __restrict__ off, uint64_t n, uint64_t m, const uint32_t* __restrict__ tile_start,
+    uint64_t ntiles, const uint32_t* __restrict__ succ, const uint32_t* __restrict__ comp,
+    unsigned long long* __restrict__ count, const uint64_t* __restrict__ at, uint32_t* __restrict__ src_out,
+    uint32_t* __restrict__ dst_out) {
+    __shared__ uint32_t src[LBS_TILE];
+    __shared__ uint32_t warp_max[LBS_THREADS / 32], warp_n[LBS_ITEMS][LBS_THREADS / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (uint64_t k = blockIdx.x; k < ntiles; k += gridDim.x) {
+        if (src_out && at[k] == at[k + 1]) continue;  // uniform over the block
+        lbs_sources(off, n, m, tile_start, ntiles, k, src, warp_max);
+        uint32_t hit = 0, to[LBS_ITEMS];
+        unsigned mask[LBS_ITEMS];
+#pragma unroll
+        for (int j = 0; j < LBS_ITEMS; j++) {
+            const uint64_t e = k * LBS_TILE + j * LBS_THREADS + threadIdx.x;
+            to[j] = e < m ? __ldg(succ + e) : 0u;
+            if (e < m && __ldg(comp + to[j]) != __ldg(comp + src[j * LBS_THREADS + threadIdx.x])) hit |= 1u << j;
+        }
+#pragma unroll
+        for (int j = 0; j < LBS_ITEMS; j++) {
+            mask[j] = __ballot_sync(0xffffffffu, (hit >> j) & 1u);
+            if (lane == 0) warp_n[j][warp] = __popc(mask[j]);
+        }
+        __syncthreads();
+        if (!src_out) {
+            if (threadIdx.x == 0) {
+                uint32_t t = 0;
+                for (int j = 0; j < LBS_ITEMS; j++)
+                    for (int w = 0; w < LBS_THREADS / 32; w++) t += warp_n[j][w];
+                count[k] = t;
+            }
+        } else if (hit) {
+            uint64_t slot = at[k];
+            for (int j = 0; j < LBS_ITEMS; j++) {
+                uint64_t s = slot;
+                for (int w = 0; w < LBS_THREADS / 32; w++) {
+                    if (w < warp) s += warp_n[j][w];
+                    slot += warp_n[j][w];
+                }
+                if ((hit >> j) & 1u) {
+                    s += __popc(mask[j] & ((1u << lane) - 1u));
+                    src_out[s] = src[j * LBS_THREADS + threadIdx.x];
+                    dst_out[s] = to[j];
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
 __global__ void k_gather_f64(const double* __restrict__ src, const uint32_t* __restrict__ inv,
                              double* __restrict__ dst, uint64_t n) {
     for (uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n;
@@ -2454,6 +2508,17 @@ int launch_scatter_arcs(const uint64_t* off, uint64_t n, uint64_t m, const uint3
     ++t_launches;
     k_scatter_arcs<<<arc_grid(nt), LBS_THREADS, 0, (cudaStream_t)stream>>>(off, n, m, tile_start, nt,
                                                                          succ, cursor, tsucc);
+    return (int)cudaGetLastError();
+}
+
+int launch_cross_arcs(const uint64_t* off, uint64_t n, uint64_t m, const uint32_t* tile_start, const uint32_t* succ,
+                      const uint32_t* comp, unsigned long long* count, const uint64_t* at, uint32_t* src, uint32_t* dst,
+                      void* stream) {
+    const uint64_t nt = arc_tiles(m);
+    if (nt == 0) return 0;
+    ++t_launches;
+    k_cross_arcs<<<arc_grid(nt), LBS_THREADS, 0, (cudaStream_t)stream>>>(off, n, m, tile_start, nt, succ, comp, count, at,
+                                                                       src, dst);
     return (int)cudaGetLastError();
 }
 

@@ -6,34 +6,40 @@
 // The work of the algorithm is its breadth-first visits (forward on the
 // graph, backward on the transpose) and, after each, an update of per-node
 // bounds; between visits it picks the next start node with a filtered
-// argmax / argmin over all nodes. All of that runs on the device:
-//   k_sw_expand / k_sw_heavy  level-synchronous visit: one warp per frontier
-//                             node (a block for nodes above SW_HEAVY arcs);
-//                             a successor is claimed by an atomicCAS on its
-//                             distance word and appended to the next level
-//                             through a per-warp run in shared memory (one
-//                             atomicAdd per run of up to 128 nodes); an optional
-//                             component array keeps a visit inside each
-//                             start node's strongly connected component
+// argmax / argmin over all nodes. A step is one run of launches with one
+// synchronisation at its end:
+//   k_sw_select               filtered argmax / argmin, with the reference's tie
+//                             rules (larger / smaller value, then tie value, then
+//                             smaller node); the start stays on the device;
+//   k_sw_begin                distances and visited bits cleared, the start queued;
+//   hbl::k_level              the levels of the visit (visit_level.cuh), as many
+//                             launches as the visits before it took; an optional
+//                             component array keeps a visit inside each start
+//                             node's strongly connected component
 //                             (computer.rs:745-800: all pivots at once);
-//   k_sw_fwd_update, k_sw_bwd_update
+//   k_sw_forward / k_sw_backward, k_sw_missing
 //                             the per-node bound updates of a forward /
-//                             backward visit (computer.rs:572-693) over the
-//                             visited nodes; a new minimal radius is an
-//                             atomicMin of (eccentricity << 32 | node);
-//   k_sw_select               filtered argmax / argmin per block, with the
-//                             reference's tie rules (larger / smaller value,
-//                             then tie value, then smaller node), finished on
-//                             the host over the block results;
-//   k_sw_missing              the five counts of find_missing_nodes;
+//                             backward visit (computer.rs:572-693), a new minimal
+//                             radius as an atomicMin of (eccentricity << 32 |
+//                             node), and the five counts of find_missing_nodes;
+//                             the last block writes what the host needs into
+//                             page-locked memory. When the visit has not ended,
+//                             they do nothing and the host adds levels.
+// and for all_cc_upper_bound:
 //   k_sw_pivot_*              the best pivot of every component
 //                             (computer.rs:418-475) by three atomicMin passes;
-//   k_sw_refine               the node pass of all_cc_upper_bound.
+//   k_sw_refine               the node pass.
+// What bounds a step is the chain of its launches and, inside a level, of its
+// accesses. Web-like 2.6e5 (2.6 M arcs), 621 visits: 0.15 ms a visit, where three
+// launches a level, eight levels at a time, and four synchronisations took
+// 0.69; every eccentricity of a symmetric graph of 3000 nodes, whose visits one
+// block runs: 58 us a step where it took 130.
 // The strongly connected component of the largest out-degree node comes from
 // two device visits (one for a symmetric graph); the host runs Tarjan's
 // algorithm (sccs/tarjan.rs) or the symmetric labelling (sccs/symm_seq.rs) on
-// the nodes outside it (see directed_components, symmetric_components), and
-// finds the arcs between components (scc_graph.rs) and the two passes over
+// the nodes outside it (see directed_components, symmetric_components). The
+// arcs between components are listed on the device (cross_arcs); the host picks
+// one per pair of components (scc_graph.rs) and runs the two passes over
 // the component DAG of all_cc_upper_bound (computer.rs:829-873), which touch
 // one value per component and per DAG arc.
 //
@@ -54,194 +60,217 @@
 #include <vector>
 
 #include "hb_internal.h"
+#include "visit_level.cuh"
 
 namespace hbs {
 
 constexpr uint32_t INF = 0xffffffffu;
-constexpr uint32_t SW_HEAVY = 4096;
 constexpr int SW_THREADS = 256;
-
-__device__ __forceinline__ bool sw_claim(uint32_t* dist, uint32_t s, uint32_t d) {
-    if (*(volatile uint32_t*)(dist + s) != INF) return false;
-    return atomicCAS(dist + s, INF, d) == INF;
-}
-
-__device__ __forceinline__ void sw_append(bool c, uint32_t s, uint32_t* queue, unsigned long long* tail) {
-    const unsigned mask = __ballot_sync(0xffffffffu, c);
-    if (!mask) return;
-    const int lane = threadIdx.x & 31;
-    unsigned long long base = 0;
-    if (lane == __ffs(mask) - 1) base = atomicAdd(tail, (unsigned long long)__popc(mask));
-    base = __shfl_sync(0xffffffffu, base, __ffs(mask) - 1);
-    if (c) queue[base + __popc(mask & ((1u << lane) - 1u))] = s;
-}
-
-// A warp's claimed nodes wait in shared memory and go to the queue in runs
-// of up to SW_RUN slots, one atomicAdd on the tail per run: on a level of
-// many small-degree nodes a per-chunk append puts one same-address atomic
-// in the chain of almost every frontier node.
-constexpr int SW_RUN = 128;
-
-// adds the lanes' claimed nodes to the warp's run, writing the run out when
-// another chunk might not fit (every lane of the warp calls it)
-__device__ __forceinline__ void sw_stage(bool c, uint32_t s, uint32_t* run, int& fill, uint32_t* queue,
-                                         unsigned long long* tail) {
-    const unsigned mask = __ballot_sync(0xffffffffu, c);
-    const int lane = threadIdx.x & 31;
-    if (c) run[fill + __popc(mask & ((1u << lane) - 1u))] = s;
-    fill += __popc(mask);
-    if (fill > SW_RUN - 32) {
-        __syncwarp();
-        unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(tail, (unsigned long long)fill);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        for (int k = lane; k < fill; k += 32) queue[base + k] = run[k];
-        __syncwarp();
-        fill = 0;
-    }
-}
-
-// writes out what is left of the warp's run
-__device__ __forceinline__ void sw_flush(const uint32_t* run, int fill, uint32_t* queue, unsigned long long* tail) {
-    if (fill == 0) return;
-    __syncwarp();
-    const int lane = threadIdx.x & 31;
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(tail, (unsigned long long)fill);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    for (int k = lane; k < fill; k += 32) queue[base + k] = run[k];
-}
-
-// The level state of a visit in device memory, so that the host enqueues
-// several levels before it looks: queue slots [b, e) are the frontier (at
-// distance d - 1), d the distance its successors get, last the largest
-// distance that reached a node.
-struct Level {
-    unsigned long long b, e, d, last;
-};
-
-// level [b, e) of the queue (distance d - 1) -> distance d, appended at *tail
-__global__ void k_sw_expand(const uint64_t* __restrict__ off, const uint32_t* __restrict__ succ,
-                            const uint32_t* __restrict__ comp, uint32_t* dist, uint32_t* queue,
-                            const Level* lev, unsigned long long* tail, uint32_t* heavy,
-                            unsigned long long* heavy_n) {
-    __shared__ uint32_t runs[SW_THREADS / 32][SW_RUN];
-    uint32_t* run = runs[threadIdx.x >> 5];
-    int fill = 0;  // the same in every lane of the warp
-    const uint64_t b = lev->b, e = lev->e;
-    const uint32_t d = (uint32_t)lev->d;
-    const int lane = threadIdx.x & 31;
-    const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t i = b + warp; i < e; i += warps) {
-        const uint32_t v = queue[i];
-        const uint64_t s0 = off[v], s1 = off[v + 1];
-        if (s1 - s0 > SW_HEAVY) {
-            if (lane == 0) heavy[atomicAdd(heavy_n, 1ull)] = v;
-            continue;
-        }
-        const uint32_t cv = comp ? comp[v] : 0u;
-        for (uint64_t a = s0; a < s1; a += 32) {
-            const uint64_t x = a + lane;
-            uint32_t s = 0;
-            bool c = false;
-            if (x < s1) {
-                s = __ldg(succ + x);
-                c = (!comp || __ldg(comp + s) == cv) && sw_claim(dist, s, d);
-            }
-            sw_stage(c, s, run, fill, queue, tail);
-        }
-    }
-    sw_flush(run, fill, queue, tail);
-}
-
-// the deferred nodes of a level, one block each
-__global__ void k_sw_heavy(const uint64_t* __restrict__ off, const uint32_t* __restrict__ succ,
-                           const uint32_t* __restrict__ comp, uint32_t* dist, uint32_t* queue, const Level* lev,
-                           unsigned long long* tail, const uint32_t* heavy, const unsigned long long* heavy_n) {
-    const uint64_t count = *heavy_n;
-    const uint32_t d = (uint32_t)lev->d;
-    for (uint64_t h = blockIdx.x; h < count; h += gridDim.x) {
-        const uint32_t v = heavy[h];
-        const uint64_t s0 = off[v], s1 = off[v + 1];
-        const uint32_t cv = comp ? comp[v] : 0u;
-        for (uint64_t a = s0; a < s1; a += blockDim.x) {
-            const uint64_t x = a + threadIdx.x;
-            uint32_t s = 0;
-            bool c = false;
-            if (x < s1) {
-                s = __ldg(succ + x);
-                c = (!comp || __ldg(comp + s) == cv) && sw_claim(dist, s, d);
-            }
-            sw_append(c, s, queue, tail);
-        }
-    }
-}
-
-// the next level: the nodes just appended become the frontier
-__global__ void k_sw_advance(Level* lev, const unsigned long long* tail, unsigned long long* heavy_n) {
-    const unsigned long long t = *tail;
-    if (t > lev->e) lev->last = lev->d;
-    lev->b = lev->e;
-    lev->e = t;
-    lev->d++;
-    *heavy_n = 0;
-}
-
-// the start nodes of a visit at distance 0 (each start is distinct)
-__global__ void k_sw_roots(const uint32_t* __restrict__ roots, uint64_t count, uint32_t* dist, uint32_t* queue) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t r = roots[i];
-        dist[r] = 0;
-        queue[i] = r;
-    }
-}
-
-// computer.rs:652-678 (forward visit): backward totals and lower bounds
-__global__ void k_sw_fwd_update(const uint32_t* __restrict__ queue, uint64_t count, const uint32_t* __restrict__ dist,
-                                uint64_t* bt, uint64_t* bl, const uint64_t* __restrict__ bh) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t v = queue[i];
-        const uint64_t d = dist[v];
-        bt[v] += d;
-        if (bl[v] != bh[v] && bl[v] < d) bl[v] = d;
-    }
-}
-
-// computer.rs:586-626 (backward visit): forward totals and lower bounds; a
-// node whose bounds meet becomes a radius candidate
-__global__ void k_sw_bwd_update(const uint32_t* __restrict__ queue, uint64_t count, const uint32_t* __restrict__ dist,
-                                uint64_t* ft, uint64_t* fl, const uint64_t* __restrict__ fh,
-                                const uint8_t* __restrict__ radial, unsigned long long* key) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t v = queue[i];
-        const uint64_t d = dist[v];
-        ft[v] += d;
-        if (fl[v] != fh[v] && fl[v] < d) {
-            fl[v] = d;
-            if (d == fh[v] && radial[v]) atomicMin(key, (d << 32) | v);
-        }
-    }
-}
-
-__global__ void k_sw_mark(const uint32_t* __restrict__ queue, uint64_t count, uint8_t* radial) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (uint64_t)gridDim.x * blockDim.x)
-        radial[queue[i]] = 1;
-}
-
-// a pivot's eccentricity inside its component: the largest distance there
-__global__ void k_sw_pivot_ecc(const uint32_t* __restrict__ queue, uint64_t count, const uint32_t* __restrict__ dist,
-                               const uint32_t* __restrict__ comp, unsigned long long* ecc) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t v = queue[i];
-        atomicMax(ecc + comp[v], (unsigned long long)dist[v]);
-    }
-}
 
 struct Best {
     uint64_t val, tie;
     uint64_t idx;  // ~0: none
 };
+
+// What the kernels of a step keep on the device between launches.
+struct Scratch {
+    Best pick;                     // the selected start
+    unsigned long long key;        // radius candidate (~0: none)
+    unsigned long long count[5];   // missing nodes
+    uint32_t ticket;
+};
+
+// What a step tells the host (page-locked memory).
+struct Result {
+    uint64_t done;                 // 0: the visit needs more levels
+    uint64_t start;                // ~0: no node qualified, the step did nothing
+    uint64_t ecc, visited, launches;
+    uint64_t radial;               // the start is a radial vertex
+    uint64_t key;
+    uint64_t count[5];
+};
+
+// One start node (the selected one, or `root` when pick is null): every
+// distance unknown, every bit clear but the start's.
+__global__ void k_sw_begin(const hbl::Level a, uint64_t n, const Scratch* pick, uint32_t root) {
+    hbl::wait_for_launch();
+    const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t r = pick ? pick->pick.idx : root;
+    for (uint64_t v = t0; v < n; v += stride) a.dist[v] = v == r ? 0u : INF;
+    for (uint64_t w = t0; w < (n + 31) / 32; w += stride) a.visited[w] = w == r >> 5 ? 1u << (r & 31) : 0u;
+    if (r != ~0ull)  // the first level is the start's units
+        for (uint64_t t = t0; t * 32 * hbl::UNIT < a.info[r].deg; t += stride) a.tile[0][t] = 0;
+    if (t0 == 0) {
+        hbl::State s{0, 0, 0, 1, 0};
+        if (r != ~0ull) {
+            s.e = 1;
+            a.entry[0] = a.info[r];
+            s.units = (a.entry[0].deg + hbl::UNIT - 1) / hbl::UNIT;
+            a.queue[0] = (uint32_t)r;
+        }
+        a.ctl->st[0] = s;
+        a.ctl->tail = s.e;
+        a.ctl->ticket = 0;
+        a.ctl->launches = 0;
+    }
+}
+
+// the five counts of computer.rs:929-973: radial below the radius bound,
+// incomplete forward and backward above the diameter bound, incomplete forward,
+// incomplete backward
+struct Counts {
+    uint32_t r = 0, df = 0, db = 0, af = 0, ab = 0;
+    __device__ __forceinline__ void add(uint64_t fl, uint64_t fh, uint64_t bl, uint64_t bh, bool radial,
+                                        uint64_t diameter_low, uint64_t radius_high) {
+        if (fl != fh) {
+            af++;
+            df += fh > diameter_low;
+            r += radial && fl < radius_high;
+        }
+        if (bl != bh) {
+            ab++;
+            db += bh > diameter_low;
+        }
+    }
+};
+
+// Adds the block's counts to s->count; the last block to arrive gives the
+// host its result and clears the scratch for the next step.
+__device__ __forceinline__ void finish_counts(Counts c, Scratch* s, const hbl::Control* ctl, const uint8_t* radial,
+                                              bool step, Result* out) {
+    __shared__ uint32_t sum[5][SW_THREADS / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t v[5] = {c.r, c.df, c.db, c.af, c.ab};
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+        const uint32_t t = __reduce_add_sync(0xffffffffu, v[k]);
+        if (lane == 0) sum[k][warp] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x < 5) {
+        unsigned long long t = 0;
+        for (int w = 0; w < SW_THREADS / 32; w++) t += sum[threadIdx.x][w];
+        if (t) atomicAdd(&s->count[threadIdx.x], t);
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x != 0 || atomicAdd(&s->ticket, 1u) != gridDim.x - 1) return;
+    __threadfence();
+    const hbl::State st = ctl->st[0];
+    const uint64_t start = step ? s->pick.idx : ~0ull;
+    out->done = 1;
+    out->start = start;
+    out->ecc = st.last;
+    out->visited = st.e;
+    out->launches = ctl->launches;
+    out->radial = start != ~0ull && radial[start] != 0;
+    out->key = atomicAdd(&s->key, 0ull);
+    for (int k = 0; k < 5; k++) {
+        out->count[k] = atomicAdd(&s->count[k], 0ull);
+        s->count[k] = 0;
+    }
+    s->key = ~0ull;
+    s->ticket = 0;
+}
+
+// true (and the host told) when the visit has not ended
+__device__ __forceinline__ bool unfinished(const hbl::Control* ctl, Result* out) {
+    if (hbl::done(ctl->st[0], INF)) return false;
+    if (blockIdx.x == 0 && threadIdx.x == 0) out->done = 0;
+    return true;
+}
+
+// computer.rs:652-678 (forward visit): backward totals and lower bounds, the
+// start's forward bounds; then the missing counts
+__global__ void __launch_bounds__(SW_THREADS) k_sw_forward(
+    uint64_t n, const uint32_t* __restrict__ dist, uint64_t* bt, uint64_t* bl, const uint64_t* __restrict__ bh,
+    uint64_t* fl, uint64_t* fh, const uint8_t* __restrict__ radial, uint64_t diameter_low, uint64_t radius_high,
+    Scratch* s, const hbl::Control* ctl, Result* out) {
+    hbl::wait_for_launch();
+    if (unfinished(ctl, out)) return;
+    const uint64_t start = s->pick.idx, ecc = ctl->st[0].last;
+    if (start != ~0ull) {
+        diameter_low = max(diameter_low, ecc);
+        if (radial[start] && radius_high > ecc) radius_high = ecc;
+    }
+    Counts c;
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t d = dist[v];
+        uint64_t l = bl[v], f = fl[v], g = fh[v];
+        const uint64_t u = bh[v];
+        if (d != INF) {
+            bt[v] += d;
+            if (l != u && l < d) bl[v] = l = d;
+        }
+        if (v == start) fl[v] = fh[v] = f = g = ecc;
+        c.add(f, g, l, u, radial[v] != 0, diameter_low, radius_high);
+    }
+    finish_counts(c, s, ctl, radial, true, out);
+}
+
+// computer.rs:586-626 (backward visit): forward totals and lower bounds; a
+// node whose bounds meet becomes a radius candidate; the start's backward bounds
+__global__ void __launch_bounds__(SW_THREADS) k_sw_backward(
+    uint64_t n, const uint32_t* __restrict__ dist, uint64_t* ft, uint64_t* fl, const uint64_t* __restrict__ fh,
+    uint64_t* bl, uint64_t* bh, const uint8_t* __restrict__ radial, Scratch* s, const hbl::Control* ctl, Result* out) {
+    hbl::wait_for_launch();
+    if (unfinished(ctl, out)) return;
+    const uint64_t start = s->pick.idx, ecc = ctl->st[0].last;
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t d = dist[v];
+        if (d != INF) {
+            ft[v] += d;
+            const uint64_t l = fl[v], u = fh[v];
+            if (l != u && l < d) {
+                fl[v] = d;
+                if (d == u && radial[v]) atomicMin(&s->key, (unsigned long long)((d << 32) | v));
+            }
+        }
+        if (v == start) bl[v] = bh[v] = ecc;
+    }
+}
+
+// The missing counts alone: after a backward visit (`step`: with the bounds it
+// leaves) or after all_cc_upper_bound.
+__global__ void __launch_bounds__(SW_THREADS) k_sw_missing(
+    uint64_t n, const uint64_t* __restrict__ fl, const uint64_t* __restrict__ fh, const uint64_t* __restrict__ bl,
+    const uint64_t* __restrict__ bh, const uint8_t* __restrict__ radial, uint64_t diameter_low, uint64_t radius_high,
+    int step, Scratch* s, const hbl::Control* ctl, Result* out) {
+    hbl::wait_for_launch();
+    if (step) {
+        if (unfinished(ctl, out)) return;
+        if (s->pick.idx != ~0ull) diameter_low = max(diameter_low, (uint64_t)ctl->st[0].last);
+        if (s->key != ~0ull) radius_high = min(radius_high, (uint64_t)(s->key >> 32));
+    }
+    Counts c;
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x)
+        c.add(fl[v], fh[v], bl[v], bh[v], radial[v] != 0, diameter_low, radius_high);
+    finish_counts(c, s, ctl, radial, step != 0, out);
+}
+
+// the visited nodes become radial vertices
+__global__ void k_sw_mark(uint64_t n, const uint32_t* __restrict__ dist, uint8_t* radial) {
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x)
+        if (dist[v] != INF) radial[v] = 1;
+}
+
+// a pivot's eccentricity inside its component: the largest distance there.
+// Most warps see one component (the giant one), so the warp agrees first; the
+// plain read in front keeps the atomics to the ones that raise the maximum.
+__global__ void k_sw_pivot_ecc(uint64_t n, const uint32_t* __restrict__ dist, const uint32_t* __restrict__ comp,
+                               unsigned long long* ecc) {
+    const uint64_t limit = (n + 31) & ~31ull;
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < limit; v += (uint64_t)gridDim.x * blockDim.x) {
+        const bool in = v < n && dist[v] != INF;
+        const uint32_t c = in ? comp[v] : 0xffffffffu, d = in ? dist[v] : 0u;
+        int same;
+        __match_all_sync(0xffffffffu, c, &same);
+        const uint32_t m = __reduce_max_sync(0xffffffffu, d);
+        if (!in || (same && (threadIdx.x & 31) != 0)) continue;
+        const unsigned long long x = same ? m : d;
+        if (*(volatile unsigned long long*)(ecc + c) < x) atomicMax(ecc + c, x);
+    }
+}
 
 // a better than b: larger (val, tie) when maximizing, smaller when
 // minimizing, then the smaller node (argmax.rs, argmin.rs)
@@ -253,13 +282,37 @@ __device__ __host__ __forceinline__ bool better(const Best& a, const Best& b, bo
     return a.idx < b.idx;
 }
 
+// s[0] = the best of the block's b
+__device__ __forceinline__ void block_best(Best b, Best* s, bool maximize) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto over = [&](int lanes) {
+        for (int o = lanes / 2; o > 0; o >>= 1) {
+            const Best c{__shfl_xor_sync(0xffffffffu, b.val, o), __shfl_xor_sync(0xffffffffu, b.tie, o),
+                         __shfl_xor_sync(0xffffffffu, b.idx, o)};
+            if (better(c, b, maximize)) b = c;
+        }
+    };
+    over(32);
+    __syncthreads();
+    if (lane == 0) s[warp] = b;
+    __syncthreads();
+    if (warp == 0) {
+        b = lane < SW_THREADS / 32 ? s[lane] : Best{0, 0, ~0ull};
+        over(SW_THREADS / 32);
+        if (lane == 0) s[0] = b;
+    }
+    __syncthreads();
+}
+
 // filter: 0 fa[i] != fb[i] (bounds not met), 1 radial[i]; val == nullptr:
 // the out-degree from off (the start of the SumSweep heuristic)
 __global__ void k_sw_select(uint64_t n, const uint64_t* __restrict__ val, const uint64_t* __restrict__ tie,
                             const uint64_t* __restrict__ off, int maximize, int filter,
                             const uint64_t* __restrict__ fa, const uint64_t* __restrict__ fb,
-                            const uint8_t* __restrict__ radial, Best* out) {
-    __shared__ Best s[SW_THREADS];
+                            const uint8_t* __restrict__ radial, Best* part, Scratch* scr, uint64_t* host) {
+    hbl::wait_for_launch();
+    __shared__ Best s[SW_THREADS / 32];
+    __shared__ bool last;
     Best b{0, 0, ~0ull};
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         bool keep = true;
@@ -272,49 +325,26 @@ __global__ void k_sw_select(uint64_t n, const uint64_t* __restrict__ val, const 
         c.idx = i;
         if (better(c, b, maximize)) b = c;
     }
-    s[threadIdx.x] = b;
+    block_best(b, s, maximize);
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = s[0];
+        __threadfence();
+        last = atomicAdd(&scr->ticket, 1u) == gridDim.x - 1;
+    }
     __syncthreads();
-    for (int w = SW_THREADS / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w && better(s[threadIdx.x + w], s[threadIdx.x], maximize))
-            s[threadIdx.x] = s[threadIdx.x + w];
-        __syncthreads();
+    if (!last) return;
+    // the last block: the best of the blocks (written in this launch: not cached)
+    __threadfence();
+    b = Best{0, 0, ~0ull};
+    for (int k = threadIdx.x; k < (int)gridDim.x; k += SW_THREADS) {
+        const Best c{__ldcg(&part[k].val), __ldcg(&part[k].tie), __ldcg(&part[k].idx)};
+        if (better(c, b, maximize)) b = c;
     }
-    if (threadIdx.x == 0) out[blockIdx.x] = s[0];
-}
-
-// computer.rs:929-973: incomplete forward, of them above the diameter bound
-// and radial below the radius bound; incomplete backward, of them above the
-// diameter bound
-__global__ void k_sw_missing(uint64_t n, const uint64_t* __restrict__ fl, const uint64_t* __restrict__ fh,
-                             const uint64_t* __restrict__ bl, const uint64_t* __restrict__ bh,
-                             const uint8_t* __restrict__ radial, uint64_t diameter_low, uint64_t radius_high,
-                             unsigned long long* cnt) {
-    unsigned long long r = 0, df = 0, db = 0, af = 0, ab = 0;
-    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
-        if (fl[v] != fh[v]) {
-            af++;
-            if (fh[v] > diameter_low) df++;
-            if (radial[v] && fl[v] < radius_high) r++;
-        }
-        if (bl[v] != bh[v]) {
-            ab++;
-            if (bh[v] > diameter_low) db++;
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        r += __shfl_xor_sync(0xffffffffu, r, o);
-        df += __shfl_xor_sync(0xffffffffu, df, o);
-        db += __shfl_xor_sync(0xffffffffu, db, o);
-        af += __shfl_xor_sync(0xffffffffu, af, o);
-        ab += __shfl_xor_sync(0xffffffffu, ab, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        if (r) atomicAdd(cnt + 0, r);
-        if (df) atomicAdd(cnt + 1, df);
-        if (db) atomicAdd(cnt + 2, db);
-        if (af) atomicAdd(cnt + 3, af);
-        if (ab) atomicAdd(cnt + 4, ab);
+    block_best(b, s, maximize);
+    if (threadIdx.x == 0) {
+        scr->pick = s[0];
+        scr->ticket = 0;
+        if (host) *host = s[0].idx;
     }
 }
 
@@ -329,17 +359,36 @@ __global__ void k_sw_pivot_pass(int pass, uint64_t n, const uint32_t* __restrict
                                 const uint64_t* __restrict__ bl, const uint64_t* __restrict__ bh,
                                 const uint64_t* __restrict__ ft, const uint64_t* __restrict__ bt,
                                 unsigned long long* best_score, unsigned long long* best_tot, uint32_t* pivot) {
-    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t c = comp[v];
-        const uint64_t sc = pivot_score(v, n, fl, fh, bl, bh);
-        if (pass == 0) {
-            atomicMin(best_score + c, (unsigned long long)sc);
-            continue;
+    // Most warps see one component (the giant one), whose minimum is one word:
+    // such a warp agrees on its own first, and a plain read keeps the atomics
+    // to the ones that lower the minimum.
+    const uint64_t limit = (n + 31) & ~31ull;
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < limit; v += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t c = v < n ? comp[v] : 0xffffffffu;
+        uint64_t x = ~0ull;
+        if (v < n) {
+            const uint64_t sc = pivot_score(v, n, fl, fh, bl, bh);
+            if (pass == 0) {
+                x = sc;
+            } else if (sc == best_score[c]) {
+                const uint64_t tot = ft[v] + bt[v];
+                if (pass == 1) x = tot;
+                else if (tot == best_tot[c]) x = v;
+            }
         }
-        if (sc != best_score[c]) continue;
-        const uint64_t tot = ft[v] + bt[v];
-        if (pass == 1) atomicMin(best_tot + c, (unsigned long long)tot);
-        else if (tot == best_tot[c]) atomicMin(pivot + c, (uint32_t)v);
+        int same;
+        __match_all_sync(0xffffffffu, c, &same);
+        if (same) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) x = min(x, __shfl_xor_sync(0xffffffffu, x, o));
+        }
+        if (x == ~0ull || (same && (threadIdx.x & 31) != 0)) continue;
+        if (pass == 2) {
+            if (*(volatile uint32_t*)(pivot + c) > (uint32_t)x) atomicMin(pivot + c, (uint32_t)x);
+        } else {
+            unsigned long long* best = (pass == 0 ? best_score : best_tot) + c;
+            if (*(volatile unsigned long long*)best > x) atomicMin(best, (unsigned long long)x);
+        }
     }
 }
 
@@ -372,12 +421,6 @@ __global__ void k_sw_refine(uint64_t n, const uint32_t* __restrict__ comp, const
         const uint64_t pb = (uint64_t)df[v] + eb[c];
         if (pb < bh[v]) bh[v] = pb;
     }
-}
-
-// a[i] = b[i] = value (the start node's bounds after its own visit)
-__global__ void k_sw_set2(uint64_t* a, uint64_t* b, uint64_t i, uint64_t value) {
-    a[i] = value;
-    b[i] = value;
 }
 
 __global__ void k_sw_fill64(uint64_t* p, uint64_t count, uint64_t value) {
@@ -524,24 +567,24 @@ struct Sweeper {
     // device state
     u64 *d_off = nullptr, *d_toff = nullptr;
     uint32_t *d_succ = nullptr, *d_tsucc = nullptr;
-    uint32_t *d_dist = nullptr, *d_queue = nullptr, *d_heavy = nullptr, *d_comp = nullptr;
-    uint32_t *d_roots = nullptr, *d_df = nullptr, *d_db = nullptr;
+    uint32_t *d_dist = nullptr, *d_queue = nullptr, *d_visited = nullptr, *d_comp = nullptr;
+    uint32_t *d_df = nullptr, *d_db = nullptr;
     u64 *d_fl = nullptr, *d_fh = nullptr, *d_bl = nullptr, *d_bh = nullptr, *d_ft = nullptr, *d_bt = nullptr;
     uint8_t* d_radial = nullptr;
-    unsigned long long* d_cnt = nullptr;  // [2] radius key [3..7] missing counts
-    hbs::Level* d_lev = nullptr;          // a visit's level, then its tail and deferred-node count
+    hbl::Entry *d_entry = nullptr, *d_info = nullptr, *d_tinfo = nullptr;
+    uint32_t* d_tile[2] = {nullptr, nullptr};
+    hbl::Control* d_ctl = nullptr;
+    hbs::Scratch* d_scr = nullptr;
     unsigned long long *d_ecc_f = nullptr, *d_ecc_b = nullptr, *d_best_score = nullptr, *d_best_tot = nullptr;
     uint32_t* d_pivot = nullptr;
     u64 *d_ef = nullptr, *d_eb = nullptr;
     uint32_t *d_cstart = nullptr, *d_cend = nullptr, *d_gather = nullptr;
     u64* d_gather64 = nullptr;
-    hbs::Best* d_best = nullptr;
-    unsigned long long* h_cnt = nullptr;  // page-locked: [0, 6) a visit's level, 6 root, 7 key, [8, 13) counts
-    hbs::Best* h_best = nullptr;          // page-locked copy of the selection's block results
+    hbs::Best* d_best = nullptr;          // the blocks' results of a selection
+    hbs::Result* h_res = nullptr;         // page-locked
+    int* d_bad = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    static constexpr int LEVELS_AHEAD = 8;
-    cudaGraphExec_t group_graph[2][2] = {};  // [backward][inside components]: LEVELS_AHEAD levels
-    cudaStream_t cap = nullptr;              // capture stream of the groups
+    int ahead[2] = {4, 4};                // launches of the next forward / backward visit
     float device_ms = 0.f;
     u64 sweeps = 0;
     // host state (computer.rs:38-89)
@@ -552,29 +595,23 @@ struct Sweeper {
     u64 diameter_low = 0, radius_high = NONE, diameter_vertex = 0, radius_vertex = 0, iterations = 0;
     u64 radius_it = NONE, diameter_it = NONE, forward_it = NONE, all_it = NONE;
     bool compute_radial = true;
-    std::vector<uint8_t> radial_host;  // the radial vertices (read on the host by forward steps)
     int grid = 1;
 
     ~Sweeper() {
         cudaSetDevice(device);
         if (s) cudaStreamSynchronize(s);
         // a symmetric graph is its own transpose: each block once
-        std::vector<void*> ps = {d_off, d_toff, d_succ, d_tsucc, d_dist, d_queue, d_heavy, d_comp,
-                                 d_roots, d_df, d_db, d_fl, d_fh, d_bl, d_bh, d_ft, d_bt, d_radial,
-                                 d_cnt, d_lev, d_ecc_f, d_ecc_b, d_best_score, d_best_tot, d_pivot, d_ef,
+        std::vector<void*> ps = {d_off, d_toff, d_succ, d_tsucc, d_dist, d_queue, d_entry, d_info, d_tinfo, d_tile[0], d_tile[1], d_visited, d_comp,
+                                 d_df, d_db, d_fl, d_fh, d_bl, d_bh, d_ft, d_bt, d_radial, d_ctl, d_scr, d_bad,
+                                 d_ecc_f, d_ecc_b, d_best_score, d_best_tot, d_pivot, d_ef,
                                  d_eb, d_cstart, d_cend, d_gather, d_gather64, d_best};
         std::sort(ps.begin(), ps.end());
         ps.erase(std::unique(ps.begin(), ps.end()), ps.end());
         for (void* p : ps)
             if (p) cudaFree(p);
-        if (h_cnt) cudaFreeHost(h_cnt);
-        if (h_best) cudaFreeHost(h_best);
+        if (h_res) cudaFreeHost(h_res);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
-        for (auto& row : group_graph)
-            for (cudaGraphExec_t g : row)
-                if (g) cudaGraphExecDestroy(g);
-        if (cap) cudaStreamDestroy(cap);
         if (own_stream && s) cudaStreamDestroy(s);
     }
 
@@ -585,85 +622,86 @@ struct Sweeper {
     int blocks(u64 work) const { return (int)std::min<u64>((work + hbs::SW_THREADS - 1) / hbs::SW_THREADS + 1, (u64)grid); }
     void sync() { ck(cudaStreamSynchronize(s), "cudaStreamSynchronize"); }
 
-    // One visit from the `count` start nodes in d_roots on the graph or its
-    // transpose (inside components when `in_comp`); returns the number of
-    // visited nodes (d_queue[0, visited), distances in d_dist) and the
-    // largest distance in *ecc. Levels are enqueued LEVELS_AHEAD at a time
-    // with their bounds in device memory (a level past the last is empty);
-    // the host looks only between groups. A group is one CUDA graph per kind
-    // of visit (forward or backward, inside components or not), captured
-    // the first time on a private stream and launched on the call's stream.
-    u64 visit(u64 count, bool backward, bool in_comp, u64* ecc) {
-        const u64* off = backward ? d_toff : d_off;
-        const uint32_t* succ = backward ? d_tsucc : d_succ;
-        const uint32_t* cp = in_comp ? d_comp : nullptr;
-        ck(cudaMemsetAsync(d_dist, 0xff, n * 4, s), "cudaMemsetAsync");
-        hbs::k_sw_roots<<<blocks(count), hbs::SW_THREADS, 0, s>>>(d_roots, count, d_dist, d_queue);
-        ck(cudaGetLastError(), "k_sw_roots");
-        hbs::Level* h = reinterpret_cast<hbs::Level*>(h_cnt);
-        *h = hbs::Level{0, count, 1, 0};
-        h_cnt[4] = count;  // tail
-        h_cnt[5] = 0;      // deferred nodes
-        ck(cudaMemcpyAsync(d_lev, h_cnt, 6 * 8, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
-        unsigned long long* tail = reinterpret_cast<unsigned long long*>(d_lev) + 4;
-        unsigned long long* heavy_n = tail + 1;
-        auto enqueue = [&](cudaStream_t x) {
-            for (int k = 0; k < LEVELS_AHEAD; k++) {
-                hbs::k_sw_expand<<<grid, hbs::SW_THREADS, 0, x>>>(off, succ, cp, d_dist, d_queue, d_lev, tail,
-                                                                 d_heavy, heavy_n);
-                hbs::k_sw_heavy<<<sms * 4, hbs::SW_THREADS, 0, x>>>(off, succ, cp, d_dist, d_queue, d_lev, tail,
-                                                                  d_heavy, heavy_n);
-                hbs::k_sw_advance<<<1, 1, 0, x>>>(d_lev, tail, heavy_n);
-            }
-        };
-        cudaGraphExec_t& ge = group_graph[backward ? 1 : 0][in_comp ? 1 : 0];
-        if (!ge) {
-            if (!cap) ck(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking), "cudaStreamCreate");
-            ck(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
-            enqueue(cap);
-            cudaGraph_t graph = nullptr;
-            const cudaError_t e = cudaStreamEndCapture(cap, &graph);
-            if (e == cudaSuccess) ck(cudaGraphInstantiate(&ge, graph, 0), "cudaGraphInstantiate");
-            if (graph) cudaGraphDestroy(graph);
-            ck(e, "cudaStreamEndCapture");
-        }
-        for (;;) {
-            ck(cudaGraphLaunch(ge, s), "cudaGraphLaunch");
-            ck(cudaMemcpyAsync(h_cnt, d_lev, 6 * 8, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
+    hbl::Level level_args(bool backward, bool in_comp) const {
+        hbl::Level a{};
+        a.info = backward ? d_tinfo : d_info;
+        a.succ = backward ? d_tsucc : d_succ;
+        a.comp = in_comp ? d_comp : nullptr;
+        a.visited = d_visited;
+        a.dist = d_dist;
+        a.queue = d_queue;
+        a.entry = d_entry;
+        a.tile[0] = d_tile[0];
+        a.tile[1] = d_tile[1];
+        a.ctl = d_ctl;
+        a.n = n;
+        a.small = hbl::small_units(n, m);
+        a.max_d = hbs::INF;
+        return a;
+    }
+
+    // `count` more level launches of a visit (in: the parity of the next)
+    void levels(const hbl::Level& a, int count, int& in) {
+        ck(a.comp ? hbl::launch_levels<true, false>(a, count, in, sms, s)
+                  : hbl::launch_levels<false, false>(a, count, in, sms, s),
+           "k_level");
+    }
+
+    // after a visit that took `launches` launches with work
+    void learn(bool backward, u64 launches) {
+        // an idle launch costs about 1.4 us, a visit that needs another
+        // synchronisation 20: the estimate falls by one launch a visit at most
+        const int want = (int)std::max<u64>(1, std::min<u64>(launches, 64));
+        ahead[backward] = std::max(want, ahead[backward] - 1);
+    }
+
+    // runs the levels of a visit to its end
+    void run_levels(const hbl::Level& a, bool backward) {
+        int in = 0;
+        for (int k = ahead[backward];; k = 2) {
+            levels(a, k, in);
+            hbl::Control* c = reinterpret_cast<hbl::Control*>(h_res + 1);
+            ck(cudaMemcpyAsync(c, d_ctl, sizeof *c, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
             sync();
-            if (h->b == h->e) break;
+            if (hbl::done(c->st[0], hbs::INF)) {
+                learn(backward, c->launches);
+                return;
+            }
         }
-        if (ecc) *ecc = h->last;
-        return h_cnt[4];
     }
 
-    // small transfers go through page-locked words (a pageable copy would
-    // wait for the stream each time): h_cnt[6] the start node, h_cnt[7]
-    // the radius key
-    void set_root(u64 r) {
-        reinterpret_cast<uint32_t*>(h_cnt + 6)[0] = (uint32_t)r;
-        ck(cudaMemcpyAsync(d_roots, h_cnt + 6, 4, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
+    // A visit from `root` on the graph or its transpose: distances in d_dist.
+    void visit(u64 root, bool backward) {
+        const hbl::Level a = level_args(backward, false);
+        ck(hbl::chain(hbs::k_sw_begin, blocks(n), hbs::SW_THREADS, 0, s, a, n, nullptr, (uint32_t)root), "k_sw_begin");
+        ck(cudaGetLastError(), "k_sw_begin");
+        run_levels(a, backward);
     }
 
-    unsigned long long read_key() {
-        ck(cudaMemcpyAsync(h_cnt + 7, d_cnt + 2, 8, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
-        sync();
-        return h_cnt[7];
+    // One visit from all components' pivots, inside the components.
+    void visit_components(bool backward) {
+        const hbl::Level a = level_args(backward, true);
+        ck(cudaMemsetAsync(d_dist, 0xff, n * 4, s), "cudaMemsetAsync");
+        ck(cudaMemsetAsync(d_visited, 0, (n + 31) / 32 * 4, s), "cudaMemsetAsync");
+        ck(cudaMemsetAsync(d_ctl, 0, sizeof *d_ctl, s), "cudaMemsetAsync");
+        ck(hbl::launch_starts<false>(a, d_pivot, ncomp, 0, true, sms, s), "k_starts");
+        run_levels(a, backward);
     }
-    void reset_key() { ck(cudaMemsetAsync(d_cnt + 2, 0xff, 8, s), "cudaMemsetAsync"); }
 
-    // argmax / argmin over nodes (filter 0: bounds fa, fb not met; 1 radial)
-    u64 select(const u64* val, const u64* tie, bool maximize, int filter, const u64* fa, const u64* fb) {
-        const int g = blocks(n);
-        hbs::k_sw_select<<<g, hbs::SW_THREADS, 0, s>>>(n, val, tie, d_off, maximize ? 1 : 0, filter, fa, fb,
-                                                       d_radial, d_best);
+    // argmax / argmin over nodes (filter 0: bounds fa, fb not met; 1 radial; 2
+    // none); the start stays in d_scr->pick
+    void select(const u64* val, const u64* tie, bool maximize, int filter, const u64* fa, const u64* fb,
+                u64* host = nullptr) {
+        ck(hbl::chain(hbs::k_sw_select, blocks(n), hbs::SW_THREADS, 0, s, n, val, tie, d_off, maximize ? 1 : 0, filter, fa, fb,
+                                                              d_radial, d_best, d_scr, host), "k_sw_select");
         ck(cudaGetLastError(), "k_sw_select");
-        ck(cudaMemcpyAsync(h_best, d_best, g * sizeof(hbs::Best), cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
+    }
+
+    // the node of the largest out-degree
+    u64 largest() {
+        select(nullptr, nullptr, true, 2, nullptr, nullptr, &h_res->start);
         sync();
-        hbs::Best b{0, 0, NONE};
-        for (int k = 0; k < g; k++)
-            if (hbs::better(h_best[k], b, maximize)) b = h_best[k];
-        return b.idx;
+        return h_res->start;
     }
 
     // The strongly connected components of a directed graph, numbered in a
@@ -680,13 +718,11 @@ struct Sweeper {
     // largest size (computer.rs:498-506 takes the first); then the whole
     // graph goes through Tarjan's algorithm in node order instead.
     std::vector<uint32_t> directed_components(const HostCsr& hg) {
-        const u64 p = select(nullptr, nullptr, true, 2, nullptr, nullptr);
+        const u64 p = largest();
         std::vector<uint32_t> fw(n), bw(n);
-        set_root(p);
-        visit(1, false, false, nullptr);
+        visit(p, false);
         ck(cudaMemcpyAsync(fw.data(), d_dist, n * 4, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
-        set_root(p);
-        visit(1, true, false, nullptr);
+        visit(p, true);
         ck(cudaMemcpyAsync(bw.data(), d_dist, n * 4, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
         sync();
         // group 0: reached from p only; 1: the component of p; 2: the rest
@@ -716,10 +752,9 @@ struct Sweeper {
     // components share the largest size; then all of them come from the host
     // in the reference's order.
     std::vector<uint32_t> symmetric_components(const HostCsr& hg) {
-        const u64 p = select(nullptr, nullptr, true, 2, nullptr, nullptr);
+        const u64 p = largest();
         std::vector<uint32_t> d(n);
-        set_root(p);
-        visit(1, false, false, nullptr);
+        visit(p, false);
         ck(cudaMemcpyAsync(d.data(), d_dist, n * 4, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
         sync();
         std::vector<uint32_t> comp(n, 0xffffffffu);
@@ -736,6 +771,48 @@ struct Sweeper {
         return comp;
     }
 
+    // The arcs between components (comp, and d_comp on the device), in arc order.
+    // A host pass over every arc took 5.9 ms on a web-like graph of 2.6 M arcs.
+    void cross_arcs(std::vector<uint32_t>& src, std::vector<uint32_t>& dst) {
+        const u64 nt = hbk::arc_tiles(m);
+        if (nt == 0) return;
+        struct Temp {
+            std::vector<void*> ps;
+            ~Temp() {
+                for (void* p : ps) cudaFree(p);
+            }
+        } temp;
+        auto get = [&](auto** p, u64 count) {
+            alloc(p, count);
+            temp.ps.push_back(*p);
+        };
+        uint32_t *tile = nullptr, *d_src = nullptr, *d_dst = nullptr;
+        unsigned long long *count = nullptr, *scratch = nullptr;
+        u64* at = nullptr;
+        const u64 sl = hbk::scan_scratch_len(nt + 1);
+        get(&tile, nt);
+        get(&count, nt + 1);
+        get(&at, nt + 1);
+        get(&scratch, sl);
+        auto launch = [&](int e, const char* what) { ck((cudaError_t)e, what); };
+        ck(cudaMemsetAsync(count + nt, 0, 8, s), "cudaMemsetAsync");
+        launch(hbk::launch_tile_start(d_off, n, tile, s), "k_tile_start");
+        launch(hbk::launch_cross_arcs(d_off, n, m, tile, d_succ, d_comp, count, nullptr, nullptr, nullptr, s), "k_cross_arcs");
+        launch(hbk::launch_exclusive_scan_u64(count, at, nt + 1, scratch, sl, s), "scan");
+        u64 total = 0;
+        ck(cudaMemcpyAsync(&total, at + nt, 8, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
+        sync();
+        if (total == 0) return;
+        get(&d_src, total);
+        get(&d_dst, total);
+        launch(hbk::launch_cross_arcs(d_off, n, m, tile, d_succ, d_comp, count, at, d_src, d_dst, s), "k_cross_arcs");
+        src.resize(total);
+        dst.resize(total);
+        ck(cudaMemcpyAsync(src.data(), d_src, total * 4, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
+        ck(cudaMemcpyAsync(dst.data(), d_dst, total * 4, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
+        sync();
+    }
+
     // computer.rs:487-542
     void compute_radial_vertices() {
         std::vector<u64> sizes(ncomp, 0);
@@ -748,61 +825,54 @@ struct Sweeper {
             v--;
             if (comp[v] == big) break;
         }
-        set_root(v);
-        const u64 cnt = visit(1, true, false, nullptr);
-        hbs::k_sw_mark<<<blocks(cnt), hbs::SW_THREADS, 0, s>>>(d_queue, cnt, d_radial);
+        visit(v, true);
+        hbs::k_sw_mark<<<blocks(n), hbs::SW_THREADS, 0, s>>>(n, d_dist, d_radial);
         ck(cudaGetLastError(), "k_sw_mark");
         sweeps++;
     }
 
-    // computer.rs:644-693
-    void forward_step(u64 start) {
-        set_root(start);
-        u64 ecc = 0;
-        const u64 cnt = visit(1, false, false, &ecc);
-        sweeps++;
-        hbs::k_sw_fwd_update<<<blocks(cnt), hbs::SW_THREADS, 0, s>>>(d_queue, cnt, d_dist, d_bt, d_bl, d_bh);
-        hbs::k_sw_set2<<<1, 1, 0, s>>>(d_fl, d_fh, start, ecc);
-        ck(cudaGetLastError(), "k_sw_fwd_update");
-        const bool rad = radial_host[start] != 0;
-        if (diameter_low < ecc) {
-            diameter_low = ecc;
-            diameter_vertex = start;
-        }
-        if (rad && radius_high > ecc) {
-            radius_high = ecc;
-            radius_vertex = start;
-        }
-    }
-
-    // computer.rs:572-642
-    void backward_step(u64 start) {
-        set_root(start);
-        u64 ecc = 0;
-        const u64 cnt = visit(1, true, false, &ecc);
-        sweeps++;
-        reset_key();
-        hbs::k_sw_bwd_update<<<blocks(cnt), hbs::SW_THREADS, 0, s>>>(d_queue, cnt, d_dist, d_ft, d_fl, d_fh,
-                                                                    d_radial, d_cnt + 2);
-        hbs::k_sw_set2<<<1, 1, 0, s>>>(d_bl, d_bh, start, ecc);
-        ck(cudaGetLastError(), "k_sw_bwd_update");
-        const unsigned long long key = read_key();
-        if (key != ~0ull && (key >> 32) < radius_high) {
+    void radius_candidate(u64 key) {
+        if (key != NONE && (key >> 32) < radius_high) {
             radius_high = key >> 32;
             radius_vertex = key & 0xffffffffull;
         }
-        if (diameter_low < ecc) {
-            diameter_low = ecc;
-            diameter_vertex = start;
-        }
     }
 
-    // computer.rs:554-570
-    void step(u64 start, bool forward) {
-        if (start == NONE) return;
-        if (forward) forward_step(start);
-        else backward_step(start);
+    // computer.rs:554-570, 572-693: a visit from the selected start (none
+    // qualified: nothing), its bound updates, and the missing counts after it
+    void step(bool forward) {
+        const hbl::Level a = level_args(!forward, false);
+        ck(hbl::chain(hbs::k_sw_begin, blocks(n), hbs::SW_THREADS, 0, s, a, n, d_scr, 0), "k_sw_begin");
+        hbs::Result& r = *h_res;
+        int in = 0;
+        for (int k = ahead[!forward];; k = 2) {
+            levels(a, k, in);
+            if (forward) {
+                ck(hbl::chain(hbs::k_sw_forward, blocks(n), hbs::SW_THREADS, 0, s, n, d_dist, d_bt, d_bl, d_bh, d_fl, d_fh, d_radial,
+                                                                       diameter_low, radius_high, d_scr, d_ctl, h_res), "k_sw_forward");
+            } else {
+                ck(hbl::chain(hbs::k_sw_backward, blocks(n), hbs::SW_THREADS, 0, s, n, d_dist, d_ft, d_fl, d_fh, d_bl, d_bh,
+                                                                        d_radial, d_scr, d_ctl, h_res), "k_sw_backward");
+                ck(hbl::chain(hbs::k_sw_missing, blocks(n), hbs::SW_THREADS, 0, s, n, d_fl, d_fh, d_bl, d_bh, d_radial, diameter_low,
+                                                                       radius_high, 1, d_scr, d_ctl, h_res), "k_sw_missing");
+            }
+            ck(cudaGetLastError(), "k_sw_forward");
+            sync();
+            if (r.done) break;
+        }
+        if (r.start == NONE) return;
+        learn(!forward, r.launches);
+        sweeps++;
         iterations++;
+        if (!forward) radius_candidate(r.key);
+        if (diameter_low < r.ecc) {
+            diameter_low = r.ecc;
+            diameter_vertex = r.start;
+        }
+        if (forward && r.radial && radius_high > r.ecc) {
+            radius_high = r.ecc;
+            radius_vertex = r.start;
+        }
     }
 
     // computer.rs:818-921
@@ -817,16 +887,14 @@ struct Sweeper {
             ck(cudaGetLastError(), "k_sw_pivot_pass");
         }
         // distances from the pivots inside each component, both directions
-        ck(cudaMemcpyAsync(d_roots, d_pivot, nc * 4, cudaMemcpyDeviceToDevice, s), "cudaMemcpyAsync");
-        u64 cnt = visit(nc, false, true, nullptr);
+        visit_components(false);
         ck(cudaMemsetAsync(d_ecc_f, 0, nc * 8, s), "cudaMemsetAsync");
-        hbs::k_sw_pivot_ecc<<<blocks(cnt), hbs::SW_THREADS, 0, s>>>(d_queue, cnt, d_dist, d_comp, d_ecc_f);
+        hbs::k_sw_pivot_ecc<<<blocks(n), hbs::SW_THREADS, 0, s>>>(n, d_dist, d_comp, d_ecc_f);
         ck(cudaGetLastError(), "k_sw_pivot_ecc");
         ck(cudaMemcpyAsync(d_df, d_dist, n * 4, cudaMemcpyDeviceToDevice, s), "cudaMemcpyAsync");
-        ck(cudaMemcpyAsync(d_roots, d_pivot, nc * 4, cudaMemcpyDeviceToDevice, s), "cudaMemcpyAsync");
-        cnt = visit(nc, true, true, nullptr);
+        visit_components(true);
         ck(cudaMemsetAsync(d_ecc_b, 0, nc * 8, s), "cudaMemsetAsync");
-        hbs::k_sw_pivot_ecc<<<blocks(cnt), hbs::SW_THREADS, 0, s>>>(d_queue, cnt, d_dist, d_comp, d_ecc_b);
+        hbs::k_sw_pivot_ecc<<<blocks(n), hbs::SW_THREADS, 0, s>>>(n, d_dist, d_comp, d_ecc_b);
         ck(cudaGetLastError(), "k_sw_pivot_ecc");
         ck(cudaMemcpyAsync(d_db, d_dist, n * 4, cudaMemcpyDeviceToDevice, s), "cudaMemcpyAsync");
         sweeps += 2;
@@ -871,27 +939,24 @@ struct Sweeper {
         }
         ck(cudaMemcpyAsync(d_ef, ef.data(), nc * 8, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
         ck(cudaMemcpyAsync(d_eb, eb.data(), nc * 8, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
-        reset_key();
         hbs::k_sw_refine<<<blocks(n), hbs::SW_THREADS, 0, s>>>(n, d_comp, d_df, d_db, d_ef, d_eb, d_fl, d_fh, d_bh,
-                                                              d_radial, d_cnt + 2);
+                                                              d_radial, &d_scr->key);
         ck(cudaGetLastError(), "k_sw_refine");
-        const unsigned long long key = read_key();
-        if (key != ~0ull && (key >> 32) < radius_high) {
-            radius_high = key >> 32;
-            radius_vertex = key & 0xffffffffull;
-        }
+        unsigned long long* key = reinterpret_cast<unsigned long long*>(&h_res->key);
+        ck(cudaMemcpyAsync(key, &d_scr->key, 8, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
+        ck(cudaMemsetAsync(&d_scr->key, 0xff, 8, s), "cudaMemsetAsync");
+        sync();
+        radius_candidate(*key);
         iterations += 3;
+        ck(hbl::chain(hbs::k_sw_missing, blocks(n), hbs::SW_THREADS, 0, s, n, d_fl, d_fh, d_bl, d_bh, d_radial, diameter_low,
+                                                               radius_high, 0, d_scr, d_ctl, h_res), "k_sw_missing");
+        ck(cudaGetLastError(), "k_sw_missing");
+        sync();
     }
 
     // computer.rs:929-1015
     u64 missing() {
-        ck(cudaMemsetAsync(d_cnt + 3, 0, 5 * 8, s), "cudaMemsetAsync");
-        hbs::k_sw_missing<<<blocks(n), hbs::SW_THREADS, 0, s>>>(n, d_fl, d_fh, d_bl, d_bh, d_radial, diameter_low,
-                                                               radius_high, d_cnt + 3);
-        ck(cudaGetLastError(), "k_sw_missing");
-        unsigned long long* c = h_cnt + 8;
-        ck(cudaMemcpyAsync(c, d_cnt + 3, 5 * 8, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
-        sync();
+        const uint64_t* c = h_res->count;  // of the last step
         const u64 mr = c[0], mdf = c[1], mdb = c[2], maf = c[3], mab = c[4];
         if (mr == 0 && radius_it == NONE) radius_it = iterations;
         if ((mdf == 0 || mdb == 0) && diameter_it == NONE) diameter_it = iterations;
@@ -909,15 +974,16 @@ struct Sweeper {
     // computer.rs:282-409
     void compute() {
         if (compute_radial) compute_radial_vertices();
-        radial_host.resize(n);
-        ck(cudaMemcpyAsync(radial_host.data(), d_radial, n, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
-        sync();
-        step(select(nullptr, nullptr, true, 2, nullptr, nullptr), true);
+        select(nullptr, nullptr, true, 2, nullptr, nullptr);
+        step(true);
         for (int i = 2; i <= 6; i++) {
-            if (i % 2 == 0)
-                step(select(d_bt, d_bl, true, 0, d_bl, d_bh), false);
-            else
-                step(select(d_ft, d_fl, true, 0, d_fl, d_fh), true);
+            if (i % 2 == 0) {
+                select(d_bt, d_bl, true, 0, d_bl, d_bh);
+                step(false);
+            } else {
+                select(d_ft, d_fl, true, 0, d_fl, d_fh);
+                step(true);
+            }
         }
         double points[5];
         for (double& p : points) p = (double)n;
@@ -928,10 +994,22 @@ struct Sweeper {
                 if (points[i] > points[st]) st = i;
             switch (st) {
                 case 0: all_cc_upper_bound(); break;
-                case 1: step(select(d_fh, d_ft, true, 0, d_fl, d_fh), true); break;
-                case 2: step(select(d_fl, d_ft, false, 1, nullptr, nullptr), true); break;
-                case 3: step(select(d_bh, d_bt, true, 0, d_bl, d_bh), false); break;
-                default: step(select(d_bt, d_bh, true, 0, d_bl, d_bh), false); break;
+                case 1:
+                    select(d_fh, d_ft, true, 0, d_fl, d_fh);
+                    step(true);
+                    break;
+                case 2:
+                    select(d_fl, d_ft, false, 1, nullptr, nullptr);
+                    step(true);
+                    break;
+                case 3:
+                    select(d_bh, d_bt, true, 0, d_bl, d_bh);
+                    step(false);
+                    break;
+                default:
+                    select(d_bt, d_bh, true, 0, d_bl, d_bh);
+                    step(false);
+                    break;
             }
             const u64 old = miss;
             miss = missing();
@@ -989,7 +1067,7 @@ int run(const hb_graph_view* g, const hb_graph_view* t, int level, const uint8_t
         w.own_stream = true;
     }
     cudaDeviceGetAttribute(&w.sms, cudaDevAttrMultiProcessorCount, device);
-    w.grid = w.sms * 8;
+    w.grid = w.sms * 4;
     ck(cudaEventCreate(&w.ev0), "cudaEventCreate");
     ck(cudaEventCreate(&w.ev1), "cudaEventCreate");
     // HB_TRACE=1: the phases' host time on stderr
@@ -1014,14 +1092,17 @@ int run(const hb_graph_view* g, const hb_graph_view* t, int level, const uint8_t
         w.d_toff = w.d_off;
         w.d_tsucc = w.d_succ;
     }
-    for (uint32_t** p : {&w.d_dist, &w.d_queue, &w.d_heavy, &w.d_comp, &w.d_roots, &w.d_df, &w.d_db}) w.alloc(p, n);
+    for (uint32_t** p : {&w.d_dist, &w.d_queue, &w.d_comp, &w.d_df, &w.d_db}) w.alloc(p, n);
+    w.alloc(&w.d_visited, (n + 31) / 32);
+    w.alloc(&w.d_entry, n);
+    for (uint32_t** p : {&w.d_tile[0], &w.d_tile[1]}) w.alloc(p, hbl::tiles(n, m));
     for (u64** p : {&w.d_fl, &w.d_fh, &w.d_bl, &w.d_bh, &w.d_ft, &w.d_bt}) w.alloc(p, n);
     w.alloc(&w.d_radial, n);
-    w.alloc(&w.d_cnt, 8);
-    ck(cudaMalloc((void**)&w.d_lev, 6 * 8), "cudaMalloc");
+    w.alloc(&w.d_ctl, 1);
+    w.alloc(&w.d_scr, 1);
+    w.alloc(&w.d_bad, 1);
     w.alloc(&w.d_best, (u64)w.grid);
-    ck(cudaMallocHost((void**)&w.h_cnt, 16 * 8), "cudaMallocHost");
-    ck(cudaMallocHost((void**)&w.h_best, (size_t)w.grid * sizeof(hbs::Best)), "cudaMallocHost");
+    ck(cudaMallocHost((void**)&w.h_res, sizeof(hbs::Result) + sizeof(hbl::Control)), "cudaMallocHost");
     cudaStream_t s = w.s;
     ck(cudaMemcpyAsync(w.d_off, g->offsets, (n + 1) * 8, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
     if (m) ck(cudaMemcpyAsync(w.d_succ, g->successors, m * 4, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
@@ -1032,8 +1113,10 @@ int run(const hb_graph_view* g, const hb_graph_view* t, int level, const uint8_t
     // the CSR is checked before any kernel indexes with it
     {
         int bad = 0;
-        int* d_bad = (int*)(w.d_cnt + 7);
+        int* d_bad = w.d_bad;
         ck(cudaMemsetAsync(d_bad, 0, 4, s), "cudaMemsetAsync");
+        ck(cudaMemsetAsync(w.d_scr, 0, sizeof *w.d_scr, s), "cudaMemsetAsync");
+        ck(cudaMemsetAsync(&w.d_scr->key, 0xff, 8, s), "cudaMemsetAsync");
         hbs::k_sw_validate<<<w.blocks(std::max(n, m)), hbs::SW_THREADS, 0, s>>>(w.d_off, w.d_succ, n, m, d_bad);
         if (t) hbs::k_sw_validate<<<w.blocks(std::max(n, m)), hbs::SW_THREADS, 0, s>>>(w.d_toff, w.d_tsucc, n, m, d_bad);
         ck(cudaGetLastError(), "k_sw_validate");
@@ -1041,42 +1124,50 @@ int run(const hb_graph_view* g, const hb_graph_view* t, int level, const uint8_t
         w.sync();
         if (bad) fail(HB_ERR_INVALID, "graph has decreasing offsets or successors >= num_nodes");
     }
+    w.alloc(&w.d_info, n);
+    hbl::k_info<<<w.blocks(n), hbs::SW_THREADS, 0, s>>>(w.d_off, n, w.d_info);
+    if (t) {
+        w.alloc(&w.d_tinfo, n);
+        hbl::k_info<<<w.blocks(n), hbs::SW_THREADS, 0, s>>>(w.d_toff, n, w.d_tinfo);
+    } else {
+        w.d_tinfo = w.d_info;
+    }
+    ck(cudaGetLastError(), "k_info");
     mark("device graph");
     // components and the arcs between them
     if (w.undirected) w.comp = w.symmetric_components(hg);
     else w.comp = w.directed_components(hg);
     w.seg.assign(w.ncomp, 0);
+    ck(cudaMemcpyAsync(w.d_comp, w.comp.data(), n * 4, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
     mark("components");
     if (!w.undirected) {
-        // scc_graph.rs:118-227; the nodes of each component in increasing
-        // order by a counting sort
+        // scc_graph.rs:118-227, over the arcs between components alone (found
+        // on the device, in arc order), grouped by their component: the order
+        // in which the reference meets them
+        std::vector<uint32_t> src, dst;
+        w.cross_arcs(src, dst);
         std::vector<u64> first(w.ncomp + 1, 0);
-        for (u64 v = 0; v < n; v++) first[w.comp[v] + 1]++;
+        for (uint32_t v : src) first[w.comp[v] + 1]++;
         for (u64 c = 0; c < w.ncomp; c++) first[c + 1] += first[c];
-        std::vector<uint32_t> members(n);
+        std::vector<u64> order(src.size());
         {
             std::vector<u64> at(first.begin(), first.end() - 1);
-            for (u64 v = 0; v < n; v++) members[at[w.comp[v]]++] = (uint32_t)v;
+            for (u64 k = 0; k < src.size(); k++) order[at[w.comp[src[k]]]++] = k;
         }
         std::vector<uint32_t> bs(w.ncomp, 0xffffffffu), be(w.ncomp, 0);
         std::vector<uint32_t> children;
         auto value = [&](u64 a, u64 b) { return ht.deg(a) + hg.deg(b); };
         for (u64 c = 0; c < w.ncomp; c++) {
             for (u64 k = first[c]; k < first[c + 1]; k++) {
-                const uint32_t v = members[k];
-                for (u64 e = hg.off[v]; e < hg.off[v + 1]; e++) {
-                    const uint32_t x = hg.succ[e];
-                    const uint32_t xc = w.comp[x];
-                    if (xc == c) continue;
-                    if (bs[xc] == 0xffffffffu) {
-                        bs[xc] = v;
-                        be[xc] = x;
-                        children.push_back(xc);
-                    }
-                    if (value(v, x) > value(bs[xc], be[xc])) {
-                        bs[xc] = v;
-                        be[xc] = x;
-                    }
+                const uint32_t v = src[order[k]], x = dst[order[k]], xc = w.comp[x];
+                if (bs[xc] == 0xffffffffu) {
+                    bs[xc] = v;
+                    be[xc] = x;
+                    children.push_back(xc);
+                }
+                if (value(v, x) > value(bs[xc], be[xc])) {
+                    bs[xc] = v;
+                    be[xc] = x;
                 }
             }
             w.seg[c] = w.ctarget.size();
@@ -1102,7 +1193,6 @@ int run(const hb_graph_view* g, const hb_graph_view* t, int level, const uint8_t
     w.alloc(&w.d_cstart, nconn);
     w.alloc(&w.d_cend, nconn);
     w.alloc(&w.d_gather, nconn);
-    ck(cudaMemcpyAsync(w.d_comp, w.comp.data(), n * 4, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
     if (nconn) {
         ck(cudaMemcpyAsync(w.d_cstart, w.cstart.data(), nconn * 4, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
         ck(cudaMemcpyAsync(w.d_cend, w.cend.data(), nconn * 4, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");

@@ -274,7 +274,11 @@ struct hb_handle {
     unsigned long long* d_q_scratch = nullptr;
     uint64_t q_scratch_len = 0;
     unsigned long long* d_inst_mod = nullptr;
-    double* d_inst_nf = nullptr;
+    double* d_inst_nf = nullptr;                 // parts of the instances' segments
+    unsigned long long* d_inst_part = nullptr;
+    uint32_t* d_inst_ticket = nullptr;
+    uint2* d_inst_segs = nullptr;                // (instance, segment)
+    uint32_t inst_segs = 0;                      // of all instances
     std::vector<unsigned long long> inst_mod;    // last iteration, per instance
     std::vector<double> inst_sum;                // last iteration, per instance
     std::vector<uint64_t> inst_iters;            // iterations run so far
@@ -287,10 +291,7 @@ struct hb_handle {
     uint64_t n_chunks = 0;
     uint32_t* d_light_bits = nullptr;           // light nodes (device ids)
     uint32_t* d_medium_bits = nullptr;          // medium nodes (device ids)
-    unsigned long long* d_word_cnt = nullptr;   // systolic lists: per bitmap word counts
-    uint64_t* d_word_off = nullptr;             // their exclusive prefix sum (+ totals)
-    unsigned long long* d_list_scratch = nullptr;
-    uint64_t list_scratch_len = 0;
+    unsigned long long* d_list_tiles = nullptr; // systolic lists: counts per tile of the bitmaps, then of all
     uint32_t* d_light_list = nullptr;           // systolic: light nodes to check or copy
     uint32_t* d_medium_list = nullptr;          // systolic: medium nodes to check or copy
     uint32_t* d_heavy = nullptr;
@@ -307,6 +308,7 @@ struct hb_handle {
     int* d_any31 = nullptr;
     bool any31 = false;
     int grid_tile = 1, grid_heavy = 1, grid_mark = 1;
+    int sms = 1;
     int grid_tile_occ = 1;           // the window kernel's grid in its 4-blocks-per-SM variant
     int grid_tile_two = 1;           // ... and in its 2-blocks-per-SM variant
     int grid_staged = 1, grid_staged_occ = 1;  // the staged kernel's grids
@@ -925,36 +927,45 @@ int enqueue_pre(hb_handle* h, hbk::UnionArgs& a, bool first_systolic, cudaStream
         return external ? cudaEventRecordWithFlags(e, s, cudaEventRecordExternal) : cudaEventRecord(e, s);
     };
     HB_CUDA(h, rec(h->ev[0]));
-    HB_CUDA(h, cudaMemsetAsync(h->d_bits[h->mod_cur ^ 1], 0, words * 4, s));
-    if (h->systolic) {
-        HB_CUDA(h, cudaMemsetAsync(h->d_bits[h->mbc_cur ^ 1], 0, words * 4, s));
-        if (first_systolic) {
-            // The reference scans every node in the first systolic iteration
-            // (HB:853-857); scanning the predecessors of the nodes modified in
-            // the previous iteration gives the same counters.
-            HB_CUDA(h, cudaMemsetAsync(h->d_bits[h->mbc_cur], 0, words * 4, s));
-            HB_LAUNCH(h, hbk::launch_mark_preds(h->d_bits[h->mod_cur], h->d_toff, h->d_tsucc,
-                                                h->d_bits[h->mbc_cur], n, h->grid_mark, s));
-        }
+    // The per-iteration constants and, after the union, the totals move between
+    // the pinned host blocks and the device by kernels, not by the copy
+    // engines: a served job's step would otherwise queue behind the other jobs'
+    // CSR uploads and result downloads.
+    hbk::IterBegin ib{};
+    ib.ic_host = h->h_ic;
+    ib.ic = h->d_ic;
+    ib.bits[0] = h->d_bits[h->mod_cur ^ 1];
+    ib.bits[1] = h->systolic ? h->d_bits[h->mbc_cur ^ 1] : nullptr;
+    ib.bits[2] = first_systolic ? h->d_bits[h->mbc_cur] : nullptr;
+    ib.words = words;
+    ib.nf_items = h->d_nf_items;
+    ib.items = h->n_chunks + h->n_heavy;
+    ib.total = h->d_partials;
+    ib.cursor = h->d_cursor;
+    HB_LAUNCH(h, hbk::launch_iter_begin(ib, h->sms, s));
+    if (first_systolic) {
+        // The reference scans every node in the first systolic iteration
+        // (HB:853-857); scanning the predecessors of the nodes modified in
+        // the previous iteration gives the same counters.
+        HB_LAUNCH(h, hbk::launch_mark_preds(h->d_bits[h->mod_cur], h->d_toff, h->d_tsucc,
+                                            h->d_bits[h->mbc_cur], n, h->grid_mark, s));
     }
-    HB_CUDA(h, cudaMemsetAsync(h->d_partials, 0, h->n_partials * sizeof(hbk::TilePartial), s));
-    HB_CUDA(h, cudaMemsetAsync(h->d_nf_items, 0, (h->n_chunks + h->n_heavy) * sizeof(double), s));
-    HB_CUDA(h, cudaMemsetAsync(h->d_cursor, 0, sizeof(unsigned long long), s));
-    // the per-iteration constants and, after the union, the totals move
-    // between the pinned host blocks and the device by a small kernel, not by
-    // the copy engines: a served job's step would otherwise queue behind the
-    // other jobs' CSR uploads and result downloads
-    HB_LAUNCH(h, hbk::launch_copy_u64(reinterpret_cast<const uint64_t*>(h->h_ic),
-                                      reinterpret_cast<uint64_t*>(h->d_ic), sizeof(hbk::IterConsts) / 8, s));
     if (h->systolic && h->n_tiles) {
         // the light and medium nodes to check or to copy
-        HB_LAUNCH(h, hbk::launch_work_lists(a.mbc, a.curr_mod, h->d_medium_bits, h->d_light_bits, n,
-                                            h->d_word_cnt, h->d_word_off, h->d_list_scratch,
-                                            h->list_scratch_len, h->d_light_list,
-                                            h->d_medium_list, s));
+        hbk::WorkLists wl{};
+        wl.mbc = a.mbc;
+        wl.curr_mod = a.curr_mod;
+        wl.medium_bits = h->d_medium_bits;
+        wl.light_bits = h->d_light_bits;
+        wl.nwords = words;
+        wl.tiles = h->d_list_tiles;
+        wl.counts = h->d_list_tiles + hbk::list_tiles(n);
+        wl.light_list = h->d_light_list;
+        wl.medium_list = h->d_medium_list;
+        HB_LAUNCH(h, hbk::launch_work_lists(wl, s));
         a.light_list = h->d_light_list;
         a.medium_list = h->d_medium_list;
-        a.list_counts = h->d_word_off + words;
+        a.list_counts = reinterpret_cast<const uint64_t*>(wl.counts);
     } else if (h->d_queue && h->n_tiles) {
         // a batch's standard iteration scans the instances still running
         const uint32_t ni = (uint32_t)(h->inst_start.size() - 1);
@@ -1013,20 +1024,24 @@ int enqueue_post(hb_handle* h, const hbk::UnionArgs& a, cudaStream_t s, bool ext
     if (h->systolic)
         HB_LAUNCH(h, hbk::launch_mark_preds(h->d_bits[h->mod_cur ^ 1], h->d_toff, h->d_tsucc,
                                             h->d_bits[h->mbc_cur ^ 1], n, h->grid_mark, s));
-    // the neighbourhood-function parts, in a fixed order, into partials[0].nf
-    HB_LAUNCH(h, hbk::launch_sum_f64(h->d_nf_items, h->n_chunks + h->n_heavy, h->d_nf_scratch,
-                                     &h->d_partials[0].nf, s));
     const size_t n_inst = h->inst_start.empty() ? 0 : h->inst_start.size() - 1;
     if (n_inst) {
-        HB_LAUNCH(h, hbk::launch_inst_stats(h->d_bits[h->mod_cur ^ 1], h->d_est, h->d_inst_start,
-                                            (uint32_t)n_inst, h->d_inst_mod, h->d_inst_nf, s));
-        HB_LAUNCH(h, hbk::launch_copy_u64(reinterpret_cast<const uint64_t*>(h->d_inst_mod),
-                                          reinterpret_cast<uint64_t*>(h->h_inst_mod), n_inst, s));
-        HB_LAUNCH(h, hbk::launch_copy_u64(reinterpret_cast<const uint64_t*>(h->d_inst_nf),
-                                          reinterpret_cast<uint64_t*>(h->h_inst_sum), n_inst, s));
+        hbk::InstStats is{};
+        is.next_mod = h->d_bits[h->mod_cur ^ 1];
+        is.est = h->d_est;
+        is.starts = h->d_inst_start;
+        is.mods = h->d_inst_mod;
+        is.host_mods = h->h_inst_mod;
+        is.host_nfs = h->h_inst_sum;
+        is.segs = h->d_inst_segs;
+        is.part_nf = h->d_inst_nf;
+        is.part_mod = h->d_inst_part;
+        is.ticket = h->d_inst_ticket;
+        HB_LAUNCH(h, hbk::launch_inst_stats(is, h->inst_segs, s));
     }
-    HB_LAUNCH(h, hbk::launch_copy_u64(reinterpret_cast<const uint64_t*>(h->d_partials),
-                                      reinterpret_cast<uint64_t*>(h->h_tot), sizeof(hbk::TilePartial) / 8, s));
+    // the neighbourhood-function parts in a fixed order, the totals to the host
+    HB_LAUNCH(h, hbk::launch_iter_end(h->d_nf_items, h->n_chunks + h->n_heavy, h->d_nf_scratch, h->d_partials,
+                                      h->d_cursor + 1, h->h_tot, s));
     HB_CUDA(h, rec(h->ev[3]));
     return HB_OK;
 }
@@ -2284,11 +2299,7 @@ static int create_impl(const hb_graph_view* graph, const hb_graph_view* transpos
         trace.mark("CSR upload + check");
         if ((r = device_partition(hp, off0, win_nodes, per_light, per_medium))) return fail(r);
         trace.mark("work partition");
-        const uint64_t words = (h->n + 31) / 32;
-        if ((r = dalloc(hp, &h->d_word_cnt, words + 1))) return fail(r);
-        if ((r = dalloc(hp, &h->d_word_off, words + 1))) return fail(r);
-        h->list_scratch_len = hbk::scan_scratch_len(words + 1);
-        if ((r = dalloc(hp, &h->d_list_scratch, h->list_scratch_len))) return fail(r);
+        if ((r = dalloc(hp, &h->d_list_tiles, hbk::list_tiles(h->n) + 1))) return fail(r);
         if ((r = dalloc(hp, &h->d_light_list, h->n + 1))) return fail(r);
         if ((r = dalloc(hp, &h->d_medium_list, h->n + 1))) return fail(r);
         if (!h->inst_start.empty()) {
@@ -2301,7 +2312,24 @@ static int create_impl(const hb_graph_view* graph, const hb_graph_view* transpos
                               "cudaMemcpyAsync")))
                 return fail(r);
             if ((r = dalloc(hp, &h->d_inst_mod, ni))) return fail(r);
-            if ((r = dalloc(hp, &h->d_inst_nf, ni))) return fail(r);
+            std::vector<uint2> segs;
+            for (size_t i = 0; i < ni; i++) {
+                const uint64_t nodes = h->inst_start[i + 1] - h->inst_start[i];
+                for (uint64_t q = 0; q == 0 || q * hbk::INST_SEG < nodes; q++)
+                    segs.push_back(make_uint2((uint32_t)i, (uint32_t)q));
+            }
+            h->inst_segs = (uint32_t)segs.size();
+            if ((r = dalloc(hp, &h->d_inst_segs, segs.size()))) return fail(r);
+            if ((r = cuda_err(hp, cudaMemcpyAsync(h->d_inst_segs, segs.data(), segs.size() * sizeof(uint2),
+                                                  cudaMemcpyHostToDevice, h->stream),
+                              "cudaMemcpyAsync")))
+                return fail(r);
+            // segs leaves the scope below
+            if ((r = cuda_err(hp, cudaStreamSynchronize(h->stream), "cudaStreamSynchronize"))) return fail(r);
+            if ((r = dalloc(hp, &h->d_inst_nf, segs.size()))) return fail(r);
+            if ((r = dalloc(hp, &h->d_inst_part, segs.size()))) return fail(r);
+            if ((r = dalloc(hp, &h->d_inst_ticket, ni))) return fail(r);
+            if ((r = cuda_err(hp, cudaMemsetAsync(h->d_inst_ticket, 0, ni * 4, h->stream), "cudaMemsetAsync"))) return fail(r);
             // the chunks of each instance, for the queue of running instances
             if (h->n_chunks && ni && h->n_chunks < (1ull << 32)) {
                 if ((r = dalloc(hp, &h->d_inst_chunk, ni + 1))) return fail(r);
@@ -2432,7 +2460,8 @@ static int create_impl(const hb_graph_view* graph, const hb_graph_view* transpos
     }
     h->grid_heavy = hbk::heavy_grid(h->log2m, h->device);
     if ((uint64_t)h->grid_heavy > h->n_heavy_items + 1) h->grid_heavy = (int)(h->n_heavy_items + 1);
-    h->grid_mark = 8 * hbk::num_sms(h->device);
+    h->sms = hbk::num_sms(h->device);
+    h->grid_mark = 8 * h->sms;
     // integer totals of the union kernels (atomics) and the summed
     // neighbourhood function
     h->n_partials = 1;
@@ -2441,7 +2470,7 @@ static int create_impl(const hb_graph_view* graph, const hb_graph_view* transpos
     if ((r = dalloc(hp, &h->d_nf_scratch, 256))) return fail(r);
     if ((r = dalloc(hp, &h->d_any31, 1))) return fail(r);
     if ((r = dalloc(hp, &h->d_ic, 1))) return fail(r);
-    if ((r = dalloc(hp, &h->d_cursor, 1))) return fail(r);
+    if ((r = dalloc(hp, &h->d_cursor, 2))) return fail(r);
     if ((r = cuda_err(hp, cudaStreamSynchronize(h->stream), "cudaStreamSynchronize"))) return fail(r);
     trace.mark("launch setup");
     *out = h.release();

@@ -132,12 +132,51 @@ struct InitArgs {
     int* any31;               // set to 1 when an initial register holds 30 or 31
 };
 
+// The first kernel of an iteration: bitmaps, totals, cursors and
+// neighbourhood-function parts cleared, the constants fetched.
+struct IterBegin {
+    const IterConsts* ic_host;   // page-locked
+    IterConsts* ic;
+    uint32_t* bits[3];           // bitmaps to clear (null: none)
+    uint64_t words;
+    double* nf_items;
+    uint64_t items;
+    TilePartial* total;
+    unsigned long long* cursor;  // two words
+};
+
+// The per-instance values of a batch's iteration.
+constexpr uint64_t INST_SEG = 8192;
+struct InstStats {
+    const uint32_t* next_mod;
+    const double* est;
+    const uint64_t* starts;           // instances + 1
+    unsigned long long* mods;         // modified counters (0: stopped), also to
+    unsigned long long* host_mods;    // page-locked memory,
+    double* host_nfs;                 // with the neighbourhood function
+    const uint2* segs;                // instance and segment of each block
+    double* part_nf;                  // per segment
+    unsigned long long* part_mod;
+    uint32_t* ticket;                 // per instance, zero between launches
+};
+
+// The work lists of a systolic iteration.
+struct WorkLists {
+    const uint32_t *mbc, *curr_mod, *medium_bits, *light_bits;
+    uint64_t nwords;
+    unsigned long long* tiles;        // list_tiles(n) words
+    unsigned long long* counts;       // light | medium << 32
+    uint32_t *light_list, *medium_list;
+};
+
 static_assert(sizeof(IterConsts) % 8 == 0 && sizeof(TilePartial) % 8 == 0, "copied as 64-bit words");
 
 // Launchers (hb_kernels.cu). All return cudaError_t as int.
-// dst[i] = src[i], i < n, by a kernel (either side may be page-locked host
-// memory, which the device reads and writes through unified addressing)
-int launch_copy_u64(const uint64_t* src, uint64_t* dst, uint64_t n, void* stream);
+int launch_iter_begin(const IterBegin& a, int device_sms, void* stream);
+// fixed-order sum of `count` doubles (part: 256 doubles) into total->nf, and the
+// totals to the host's page-locked copy
+int launch_iter_end(const double* in, uint64_t count, double* part, TilePartial* total, unsigned long long* ticket,
+                    TilePartial* host, void* stream);
 int launch_init(int log2m, const InitArgs& a, void* stream);
 // device counters (one byte per register) -> the reference's packed layout,
 // in caller node order (inv: caller node -> device node)
@@ -211,25 +250,12 @@ int tile_capacity(int log2m, uint32_t* nodes, uint32_t* arcs);
 // heavy nodes, one CTA each
 int launch_union_heavy(int log2m, const UnionArgs& a, int grid, void* stream);
 int heavy_grid(int log2m, int device);
-// batches: per instance [starts[i], starts[i+1]) the modified counters of the
-// iteration (next_mod) and the sum of the cached estimates
-int launch_inst_stats(const uint32_t* next_mod, const double* est, const uint64_t* starts,
-                      uint32_t count, unsigned long long* mods, double* nfs, void* stream);
-// fixed-order sum of count doubles into *out (scratch: 256 doubles)
-int launch_sum_f64(const double* in, uint64_t count, double* scratch, double* out, void* stream);
-// systolic work lists: every light / medium node set in mbc | curr_mod, in
-// node order (medium_bits / light_bits: the medium / light nodes). cnt and
-// off hold nwords + 1 words; off[nwords] gets the counts (light | medium << 32).
-int launch_work_lists(const uint32_t* mbc, const uint32_t* curr_mod, const uint32_t* medium_bits,
-                      const uint32_t* light_bits, uint64_t n, unsigned long long* cnt, uint64_t* off,
-                      unsigned long long* scratch, uint64_t scratch_len, uint32_t* light_list,
-                      uint32_t* medium_list, void* stream);
+int launch_inst_stats(const InstStats& a, uint32_t segs, void* stream);
+uint64_t list_tiles(uint64_t n);
+int launch_work_lists(const WorkLists& a, void* stream);
 // nodes per chunk of the union kernel: light nodes (lane-group each) and
 // medium nodes (team each)
 int chunk_nodes(int log2m, uint32_t* light, uint32_t* medium);
-// fixed-order sum of `count` partials; scratch holds 256 partials
-int launch_reduce_partials(const TilePartial* in, uint64_t count, TilePartial* scratch,
-                           TilePartial* out, void* stream);
 int launch_mark_preds(const uint32_t* next_mod, const uint64_t* toff, const uint32_t* tsucc,
                       uint32_t* next_mbc, uint64_t n, int grid, void* stream);
 int launch_fill_u32(uint32_t* p, uint32_t v, uint64_t count, void* stream);

@@ -1608,87 +1608,157 @@ __global__ void k_add_indeg(unsigned long long* __restrict__ rows, const uint32_
         rows[v] += indeg[v];
 }
 
-// fixed-order sum of doubles: block b sums its contiguous range (strided by
-// thread, then a tree); a second launch sums the block results the same way
-__global__ void k_sum_f64(const double* __restrict__ in, uint64_t count, double* __restrict__ out) {
-    __shared__ double s[256];
+// ---------------------------------------------------------------------------
+// An iteration's first and last kernel. Small graphs' iterations are their
+// launches (a dependent launch costs about 4 us, 1.1 as a node of a captured
+// graph), so everything that stands before the union is one kernel (it was up
+// to five clears and a copy) and everything after it another (two sums and a
+// copy).
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void clear(uint32_t* p, uint64_t words, uint64_t t0, uint64_t stride) {
+    if (!p) return;
+    uint4* q = reinterpret_cast<uint4*>(p);  // allocations are 256-byte aligned
+    for (uint64_t i = t0; i < words / 4; i += stride) q[i] = make_uint4(0u, 0u, 0u, 0u);
+    const uint64_t i = words / 4 * 4 + t0;
+    if (i < words) p[i] = 0u;
+}
+
+__global__ void k_iter_begin(const IterBegin a) {
+    const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    // the iteration's constants, from page-locked memory
+    if (t0 < sizeof(IterConsts) / 8)
+        reinterpret_cast<uint64_t*>(a.ic)[t0] = reinterpret_cast<const volatile uint64_t*>(a.ic_host)[t0];
+    if (t0 == 0) {
+        *a.total = TilePartial{};
+        a.cursor[0] = 0;  // the union kernels' cursor
+        a.cursor[1] = 0;  // k_iter_end's ticket
+    }
+    clear(a.bits[0], a.words, t0, stride);
+    clear(a.bits[1], a.words, t0, stride);
+    clear(a.bits[2], a.words, t0, stride);
+    clear(reinterpret_cast<uint32_t*>(a.nf_items), 2 * a.items, t0, stride);
+}
+
+// The neighbourhood-function parts in a fixed order: block b sums its
+// contiguous range (strided by thread, then a tree); the last block to finish
+// sums the blocks' results the same way and gives the iteration's totals to the
+// host (page-locked memory).
+constexpr int SUM_THREADS = 256;
+
+__device__ __forceinline__ double tree_sum(double x, double* s) {
+    // (t, t + 128), (t, t + 64), ... as a tree in shared memory; the last five
+    // levels are the first warp's
+    s[threadIdx.x] = x;
+    __syncthreads();
+#pragma unroll
+    for (int w = SUM_THREADS / 2; w >= 32; w >>= 1) {
+        if ((int)threadIdx.x < w) s[threadIdx.x] = x = __dadd_rn(s[threadIdx.x], s[threadIdx.x + w]);
+        __syncthreads();
+    }
+    if (threadIdx.x < 32) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) x = __dadd_rn(x, __shfl_down_sync(0xffffffffu, x, o));
+    }
+    return x;  // thread 0's
+}
+
+__global__ void __launch_bounds__(SUM_THREADS) k_iter_end(const double* __restrict__ in, uint64_t count,
+                                                          double* __restrict__ part, TilePartial* __restrict__ total,
+                                                          unsigned long long* __restrict__ ticket,
+                                                          TilePartial* __restrict__ host) {
+    __shared__ double s[SUM_THREADS];
+    __shared__ bool last;
     const uint64_t per = (count + gridDim.x - 1) / gridDim.x;
     const uint64_t b = (uint64_t)blockIdx.x * per, e = min(count, b + per);
     double x = 0.0;
-    for (uint64_t i = b + threadIdx.x; i < e; i += blockDim.x) x = __dadd_rn(x, in[i]);
-    s[threadIdx.x] = x;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) s[threadIdx.x] = __dadd_rn(s[threadIdx.x], s[threadIdx.x + w]);
-        __syncthreads();
+    for (uint64_t i = b + threadIdx.x; i < e; i += SUM_THREADS) x = __dadd_rn(x, in[i]);
+    const double sum = tree_sum(x, s);
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = sum;
+        __threadfence();
+        last = atomicAdd(ticket, 1ull) == gridDim.x - 1;
     }
-    if (threadIdx.x == 0) out[blockIdx.x] = s[0];
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    x = 0.0;
+    for (uint64_t i = threadIdx.x; i < gridDim.x; i += SUM_THREADS) x = __dadd_rn(x, __ldcg(part + i));
+    const double nf = tree_sum(x, s);
+    if (threadIdx.x == 0) {
+        TilePartial t = *total;
+        t.nf = nf;
+        *total = t;
+        *host = t;
+    }
 }
 
 // ---------------------------------------------------------------------------
 // batches: per instance (a device id range) the number of modified counters
 // and the neighbourhood function (sum of the cached estimates) of the
-// iteration just run; one block per running instance, fixed order
+// iteration just run, to the device and to the host's page-locked arrays. An
+// instance is cut into segments of INST_SEG nodes, a block each (one block for
+// the largest instance took 45 us); the last of them adds the segments' parts
+// in order. Instances whose previous iteration modified nothing have stopped:
+// their values stay.
 // ---------------------------------------------------------------------------
-constexpr int INST_THREADS = 512;
-__global__ void __launch_bounds__(INST_THREADS) k_inst_stats(const uint32_t* __restrict__ next_mod,
-                                                             const double* __restrict__ est,
-                                                             const uint64_t* __restrict__ starts,
-                                                             uint32_t count,
-                                                             unsigned long long* __restrict__ mods,
-                                                             double* __restrict__ nfs) {
-    // One block per instance, a fixed order: thread t keeps four running
-    // sums (nodes b + t + 512 (4j + k) go to sum k, so four loads are in
-    // flight), adds them as (s0 + s1) + (s2 + s3), then a fixed tree. (With
-    // one sum, 256 threads, the largest instance's block took most of the
-    // kernel's time.) An instance whose previous iteration modified nothing
-    // has stopped: its values stay.
+constexpr int INST_THREADS = 256;
+__global__ void __launch_bounds__(INST_THREADS) k_inst_stats(const InstStats a) {
+    __shared__ double s_nf[INST_THREADS];
+    __shared__ unsigned long long s_mc[INST_THREADS / 32];
     constexpr int T = INST_THREADS;
-    __shared__ double s_nf[T];
-    __shared__ unsigned long long s_mc[T];
-    for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
-        if (mods[i] == 0) continue;  // uniform over the block
-        __syncthreads();
-        const uint64_t b = __ldg(starts + i), e = __ldg(starts + i + 1);
-        double s4[4] = {0.0, 0.0, 0.0, 0.0};
-        uint64_t v = b + threadIdx.x;
-        for (; v + 3 * T < e; v += 4 * T) {
-            double x[4];
+    const uint2 is = __ldg(a.segs + blockIdx.x);
+    const uint32_t i = is.x, seg = is.y;
+    if (a.mods[i] == 0) return;  // written below only when every block has read it
+    const uint64_t b0 = __ldg(a.starts + i), e0 = __ldg(a.starts + i + 1);
+    const uint64_t b = b0 + (uint64_t)seg * INST_SEG, e = min(e0, b + INST_SEG);
+    const uint32_t nseg = (uint32_t)((e0 - b0 + INST_SEG - 1) / INST_SEG);  // 0: one block all the same
+    // thread t keeps four running sums (nodes b + t + T (4j + k) go to sum k, so
+    // four loads are in flight), adds them as (s0 + s1) + (s2 + s3), then a tree
+    double s4[4] = {0.0, 0.0, 0.0, 0.0};
+    for (uint64_t v = b + threadIdx.x; v < e; v += 4 * T) {
+        double x[4];
 #pragma unroll
-            for (int k = 0; k < 4; k++) x[k] = __ldg(est + v + k * T);
+        for (int k = 0; k < 4; k++) x[k] = v + k * T < e ? __ldg(a.est + v + k * T) : 0.0;
 #pragma unroll
-            for (int k = 0; k < 4; k++) s4[k] = __dadd_rn(s4[k], x[k]);
-        }
-        // at most three nodes left for this thread
-#pragma unroll
-        for (int k = 0; k < 3; k++)
-            if (v + k * T < e) s4[k] = __dadd_rn(s4[k], __ldg(est + v + k * T));
-        const double sum = __dadd_rn(__dadd_rn(s4[0], s4[1]), __dadd_rn(s4[2], s4[3]));
-        unsigned long long mc = 0;
-        if (e > b) {
-            const uint64_t w0 = b >> 5, w1 = (e - 1) >> 5;
-            for (uint64_t w = w0 + threadIdx.x; w <= w1; w += blockDim.x) {
-                uint32_t bits = __ldg(next_mod + w);
-                if (w == w0) bits &= 0xffffffffu << (b & 31);
-                if (w == w1 && ((e & 31) != 0)) bits &= 0xffffffffu >> (32 - (e & 31));
-                mc += __popc(bits);
-            }
-        }
-        s_nf[threadIdx.x] = sum;
-        s_mc[threadIdx.x] = mc;
-        __syncthreads();
-        for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-            if ((int)threadIdx.x < w) {
-                s_nf[threadIdx.x] = __dadd_rn(s_nf[threadIdx.x], s_nf[threadIdx.x + w]);
-                s_mc[threadIdx.x] += s_mc[threadIdx.x + w];
-            }
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) {
-            mods[i] = s_mc[0];
-            nfs[i] = s_nf[0];
+        for (int k = 0; k < 4; k++) s4[k] = __dadd_rn(s4[k], x[k]);
+    }
+    unsigned long long mc = 0;
+    if (e > b) {
+        const uint64_t w0 = b >> 5, w1 = (e - 1) >> 5;
+        for (uint64_t w = w0 + threadIdx.x; w <= w1; w += T) {
+            uint32_t bits = __ldg(a.next_mod + w);
+            if (w == w0) bits &= 0xffffffffu << (b & 31);
+            if (w == w1 && ((e & 31) != 0)) bits &= 0xffffffffu >> (32 - (e & 31));
+            mc += __popc(bits);
         }
     }
+    mc = __reduce_add_sync(0xffffffffu, (uint32_t)mc);
+    if ((threadIdx.x & 31) == 0) s_mc[threadIdx.x >> 5] = mc;
+    static_assert(INST_THREADS == SUM_THREADS, "tree_sum");
+    const double sum = tree_sum(__dadd_rn(__dadd_rn(s4[0], s4[1]), __dadd_rn(s4[2], s4[3])), s_nf);
+    if (threadIdx.x != 0) return;
+    mc = 0;
+    for (int w = 0; w < T / 32; w++) mc += s_mc[w];
+    double nf = sum;
+    if (nseg > 1) {
+        double* pn = a.part_nf + (blockIdx.x - seg);
+        unsigned long long* pm = a.part_mod + (blockIdx.x - seg);
+        pn[seg] = sum;
+        pm[seg] = mc;
+        __threadfence();
+        if (atomicAdd(a.ticket + i, 1u) != nseg - 1) return;
+        __threadfence();
+        a.ticket[i] = 0;
+        nf = 0.0;
+        mc = 0;
+        for (uint32_t q = 0; q < nseg; q++) {
+            nf = __dadd_rn(nf, __ldcg(pn + q));
+            mc += __ldcg(pm + q);
+        }
+    }
+    a.mods[i] = mc;
+    a.host_mods[i] = mc;
+    a.host_nfs[i] = nf;
 }
 
 // ---------------------------------------------------------------------------
@@ -1927,90 +1997,82 @@ __global__ void __launch_bounds__(256) k_mark_preds(const uint32_t* __restrict__
     }
 }
 
-// Fixed-order reduction of the per-tile / per-block partials: stage 1 sums
-// contiguous ranges (one block each), stage 2 sums the stage-1 results, so
-// the neighbourhood function is reproducible run to run.
 constexpr int REDUCE_BLOCKS = 256;
 
-__global__ void k_reduce_partials(const TilePartial* __restrict__ in, uint64_t count,
-                                  TilePartial* __restrict__ out) {
-    __shared__ double s_nf[256];
-    __shared__ unsigned long long s_v[256], s_m[256], s_s[256], s_a[256];
-    const uint64_t per = (count + gridDim.x - 1) / gridDim.x;
-    const uint64_t b = (uint64_t)blockIdx.x * per, e = min(count, b + per);
-    double nf = 0.0;
-    unsigned long long v = 0, mo = 0, sc = 0, sa = 0;
-    for (uint64_t i = b + threadIdx.x; i < e; i += blockDim.x) {
-        nf = __dadd_rn(nf, in[i].nf);
-        v += in[i].vis;
-        mo += in[i].mod;
-        sc += in[i].scanned;
-        sa += in[i].sarcs;
+// ---------------------------------------------------------------------------
+// Systolic iterations: the light and medium nodes to check or to copy, in node
+// order. The bitmap words are cut into tiles of LIST_TILE; the first kernel
+// counts each tile's nodes (light | medium << 32), the second adds up the tiles
+// in front of its own, scans its words' counts and writes the nodes. (Counts a
+// word, a three-launch scan and a fill were five launches.)
+// ---------------------------------------------------------------------------
+constexpr int LIST_THREADS = 256, LIST_ITEMS = 4, LIST_TILE = LIST_THREADS * LIST_ITEMS;
+
+// light and medium bits of words [w, w + LIST_ITEMS) and their counts
+__device__ __forceinline__ unsigned long long list_words(const WorkLists& a, uint64_t w, uint32_t (&lb)[LIST_ITEMS],
+                                                         uint32_t (&mb)[LIST_ITEMS]) {
+    unsigned long long c = 0;
+#pragma unroll
+    for (int k = 0; k < LIST_ITEMS; k++) {
+        const bool in = w + k < a.nwords;
+        const uint32_t bits = in ? __ldg(a.mbc + w + k) | __ldg(a.curr_mod + w + k) : 0u;
+        lb[k] = bits ? bits & __ldg(a.light_bits + w + k) : 0u;
+        mb[k] = bits ? bits & __ldg(a.medium_bits + w + k) : 0u;
+        c += (unsigned long long)__popc(lb[k]) | ((unsigned long long)__popc(mb[k]) << 32);
     }
-    s_nf[threadIdx.x] = nf;
-    s_v[threadIdx.x] = v;
-    s_m[threadIdx.x] = mo;
-    s_s[threadIdx.x] = sc;
-    s_a[threadIdx.x] = sa;
+    return c;
+}
+
+__device__ __forceinline__ unsigned long long warp_sum(unsigned long long x) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+
+__global__ void __launch_bounds__(LIST_THREADS) k_list_count(const WorkLists a) {
+    __shared__ unsigned long long s[LIST_THREADS / 32];
+    uint32_t lb[LIST_ITEMS], mb[LIST_ITEMS];
+    const unsigned long long c =
+        warp_sum(list_words(a, (uint64_t)blockIdx.x * LIST_TILE + threadIdx.x * LIST_ITEMS, lb, mb));
+    if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = c;
     __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) {
-            s_nf[threadIdx.x] = __dadd_rn(s_nf[threadIdx.x], s_nf[threadIdx.x + w]);
-            s_v[threadIdx.x] += s_v[threadIdx.x + w];
-            s_m[threadIdx.x] += s_m[threadIdx.x + w];
-            s_s[threadIdx.x] += s_s[threadIdx.x + w];
-            s_a[threadIdx.x] += s_a[threadIdx.x + w];
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[blockIdx.x] = TilePartial{s_nf[0], s_v[0], s_m[0], s_s[0], s_a[0]};
-}
-
-// Systolic iterations: flags the windows holding a node that must be checked
-// or copied; the union kernel skips the chunks of the other windows.
-// bits of word i split into light and medium nodes
-__device__ __forceinline__ void split_word(uint64_t i, uint32_t bits, const uint32_t* medium_bits,
-                                           const uint32_t* light_bits, uint32_t& lb, uint32_t& mb) {
-    lb = bits & __ldg(light_bits + i);
-    mb = bits & __ldg(medium_bits + i);
-}
-
-__global__ void k_list_count(const uint32_t* __restrict__ mbc, const uint32_t* __restrict__ curr_mod,
-                             const uint32_t* __restrict__ medium_bits,
-                             const uint32_t* __restrict__ light_bits, uint64_t nwords,
-                             unsigned long long* __restrict__ cnt) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= nwords;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        if (i == nwords) {
-            cnt[i] = 0;
-            continue;
-        }
-        uint32_t lb, mb;
-        split_word(i, __ldg(mbc + i) | __ldg(curr_mod + i), medium_bits, light_bits, lb, mb);
-        cnt[i] = (unsigned long long)__popc(lb) | ((unsigned long long)__popc(mb) << 32);
+    if (threadIdx.x == 0) {
+        unsigned long long t = 0;
+        for (int w = 0; w < LIST_THREADS / 32; w++) t += s[w];
+        a.tiles[blockIdx.x] = t;
     }
 }
 
-__global__ void k_list_fill(const uint32_t* __restrict__ mbc, const uint32_t* __restrict__ curr_mod,
-                            const uint32_t* __restrict__ medium_bits,
-                            const uint32_t* __restrict__ light_bits, uint64_t nwords,
-                            const uint64_t* __restrict__ off, uint32_t* __restrict__ light_list,
-                            uint32_t* __restrict__ medium_list) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nwords;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t lb, mb;
-        split_word(i, __ldg(mbc + i) | __ldg(curr_mod + i), medium_bits, light_bits, lb, mb);
-        const uint64_t o = off[i];
-        uint32_t ol = (uint32_t)o, om = (uint32_t)(o >> 32);
-        const uint32_t lo = (uint32_t)(i << 5);
-        while (lb) {
-            light_list[ol++] = lo + (uint32_t)(__ffs(lb) - 1);
-            lb &= lb - 1u;
-        }
-        while (mb) {
-            medium_list[om++] = lo + (uint32_t)(__ffs(mb) - 1);
-            mb &= mb - 1u;
-        }
+__global__ void __launch_bounds__(LIST_THREADS) k_list_fill(const WorkLists a) {
+    __shared__ unsigned long long s[LIST_THREADS / 32], s_base[LIST_THREADS / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t w = (uint64_t)blockIdx.x * LIST_TILE + threadIdx.x * LIST_ITEMS;
+    uint32_t lb[LIST_ITEMS], mb[LIST_ITEMS];
+    const unsigned long long own = list_words(a, w, lb, mb);
+    unsigned long long before = 0;  // the tiles in front
+    for (uint32_t t = threadIdx.x; t < blockIdx.x; t += LIST_THREADS) before += a.tiles[t];
+    before = warp_sum(before);
+    unsigned long long x = own;  // inclusive scan
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) s[warp] = x;
+    if (lane == 0) s_base[warp] = before;
+    __syncthreads();
+    unsigned long long at = x - own;
+    for (int q = 0; q < LIST_THREADS / 32; q++) {
+        at += s_base[q];
+        if (q < warp) at += s[q];
+    }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == LIST_THREADS - 1) *a.counts = at + own;
+    uint32_t ol = (uint32_t)at, om = (uint32_t)(at >> 32);
+#pragma unroll
+    for (int k = 0; k < LIST_ITEMS; k++) {
+        const uint32_t lo = (uint32_t)((w + k) << 5);
+        for (uint32_t b = lb[k]; b; b &= b - 1u) a.light_list[ol++] = lo + (uint32_t)(__ffs(b) - 1);
+        for (uint32_t b = mb[k]; b; b &= b - 1u) a.medium_list[om++] = lo + (uint32_t)(__ffs(b) - 1);
     }
 }
 
@@ -2437,19 +2499,6 @@ int launch_pack_counters(int log2m, const uint8_t* src, const uint32_t* inv, uin
 #undef CALL
 }
 
-__global__ void k_copy_u64(const uint64_t* src, uint64_t* dst, uint64_t n) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        dst[i] = src[i];
-}
-
-int launch_copy_u64(const uint64_t* src, uint64_t* dst, uint64_t n, void* stream) {
-    if (n == 0) return 0;
-    const int grid = (int)std::min<uint64_t>((n + 255) / 256, 1024);
-    ++t_launches;
-    k_copy_u64<<<grid, 256, 0, (cudaStream_t)stream>>>(src, dst, n);
-    return (int)cudaGetLastError();
-}
-
 int launch_add_indeg(unsigned long long* rows, const uint32_t* indeg, uint64_t n, void* stream) {
     if (n == 0) return 0;
     const int grid = (int)std::min<uint64_t>((n + 255) / 256, 8192);
@@ -2458,21 +2507,25 @@ int launch_add_indeg(unsigned long long* rows, const uint32_t* indeg, uint64_t n
     return (int)cudaGetLastError();
 }
 
-int launch_inst_stats(const uint32_t* next_mod, const double* est, const uint64_t* starts,
-                      uint32_t count, unsigned long long* mods, double* nfs, void* stream) {
-    const int grid = (int)std::min<uint64_t>((uint64_t)count, 16384);
+int launch_iter_begin(const IterBegin& a, int device_sms, void* stream) {
+    const uint64_t work = a.words / 4 + a.items / 2 + 64;
+    const int grid = (int)std::min<uint64_t>((work + 255) / 256, (uint64_t)device_sms * 8);
     ++t_launches;
-    if (grid)
-        k_inst_stats<<<grid, INST_THREADS, 0, (cudaStream_t)stream>>>(next_mod, est, starts, count, mods, nfs);
+    k_iter_begin<<<grid, 256, 0, (cudaStream_t)stream>>>(a);
     return (int)cudaGetLastError();
 }
 
-int launch_sum_f64(const double* in, uint64_t count, double* scratch, double* out, void* stream) {
-    cudaStream_t s = (cudaStream_t)stream;
+int launch_iter_end(const double* in, uint64_t count, double* part, TilePartial* total, unsigned long long* ticket,
+                    TilePartial* host, void* stream) {
     ++t_launches;
-    k_sum_f64<<<REDUCE_BLOCKS, 256, 0, s>>>(in, count, scratch);
+    k_iter_end<<<REDUCE_BLOCKS, SUM_THREADS, 0, (cudaStream_t)stream>>>(in, count, part, total, ticket, host);
+    return (int)cudaGetLastError();
+}
+
+int launch_inst_stats(const InstStats& a, uint32_t segs, void* stream) {
+    if (!segs) return 0;
     ++t_launches;
-    k_sum_f64<<<1, 256, 0, s>>>(scratch, REDUCE_BLOCKS, out);
+    k_inst_stats<<<segs, INST_THREADS, 0, (cudaStream_t)stream>>>(a);
     return (int)cudaGetLastError();
 }
 
@@ -2645,33 +2698,17 @@ int chunk_nodes(int log2m, uint32_t* light, uint32_t* medium) {
 #undef CALL
 }
 
-int launch_work_lists(const uint32_t* mbc, const uint32_t* curr_mod, const uint32_t* medium_bits,
-                      const uint32_t* light_bits, uint64_t n, unsigned long long* cnt, uint64_t* off,
-                      unsigned long long* scratch, uint64_t scratch_len, uint32_t* light_list,
-                      uint32_t* medium_list, void* stream) {
+uint64_t list_tiles(uint64_t n) { return std::max<uint64_t>(((n + 31) / 32 + LIST_TILE - 1) / LIST_TILE, 1); }
+
+int launch_work_lists(const WorkLists& a, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
-    const uint64_t nwords = (n + 31) / 32;
-    const int grid = (int)std::min<uint64_t>((nwords + 256) / 256 + 1, 8192);
+    const unsigned grid = (unsigned)list_tiles(a.nwords * 32);
     ++t_launches;
-    k_list_count<<<grid, 256, 0, s>>>(mbc, curr_mod, medium_bits, light_bits, nwords, cnt);
-    int e = (int)cudaGetLastError();
-    if (e) return e;
-    e = launch_exclusive_scan_u64(cnt, off, nwords + 1, scratch, scratch_len, stream);
+    k_list_count<<<grid, LIST_THREADS, 0, s>>>(a);
+    const int e = (int)cudaGetLastError();
     if (e) return e;
     ++t_launches;
-    k_list_fill<<<grid, 256, 0, s>>>(mbc, curr_mod, medium_bits, light_bits, nwords, off, light_list,
-                                     medium_list);
-    return (int)cudaGetLastError();
-}
-
-
-int launch_reduce_partials(const TilePartial* in, uint64_t count, TilePartial* scratch,
-                           TilePartial* out, void* stream) {
-    cudaStream_t s = (cudaStream_t)stream;
-    ++t_launches;
-    k_reduce_partials<<<REDUCE_BLOCKS, 256, 0, s>>>(in, count, scratch);
-    ++t_launches;
-    k_reduce_partials<<<1, 256, 0, s>>>(scratch, REDUCE_BLOCKS, out);
+    k_list_fill<<<grid, LIST_THREADS, 0, s>>>(a);
     return (int)cudaGetLastError();
 }
 

@@ -1,6 +1,6 @@
 """GPU tests of what an iteration runs around its union: the systolic work
 lists at the bounds of their tiles, and a batch's statistics at the bounds of
-the instances' segments."""
+the instances' segments, and the marks of the predecessors of modified nodes."""
 import numpy as np
 import pytest
 
@@ -20,6 +20,35 @@ def test_work_list_tiles(hb, oracle, n):
     off = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.uint64)
     g = hb.Graph.from_csr(off, np.concatenate(rows).astype(np.uint32))
     lockstep(hb, oracle, g, 4, transpose_on_device=True, buckets=(4, 1024), max_iters=40)
+
+
+@pytest.mark.parametrize("hubs", [3, 64, 65, 100])
+@pytest.mark.parametrize("in_degree", [1023, 1024, 3000])
+def test_marks_of_hubs(hb, oracle, hubs, in_degree):
+    """Nodes with in-degrees around the bound of what a warp takes alone, up to
+    more of them than one block notes; a chain behind them keeps them changing
+    while a few thousand nodes change in all."""
+    n = 20_000
+    chain = list(range(hubs, hubs + 40))
+    rows = [[chain[0]] for _ in range(hubs)] + [[c + 1] for c in chain] + [[]] * (n - hubs - 40)
+    for v in range(n - in_degree, n):
+        rows[v] = list(range(hubs))
+    off = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.uint64)
+    g = hb.Graph.from_csr(off, np.concatenate([np.asarray(r, dtype=np.uint32) for r in rows]))
+    lockstep(hb, oracle, g, 4, transpose_on_device=True)
+
+
+def test_marks_of_sparse_words(hb, oracle):
+    """More nodes than one pass of the warps over single words of the bitmap
+    takes, few of them with arcs; the last node is one."""
+    n = 10_200_007
+    rng = np.random.default_rng(1)
+    src = np.unique(np.append(rng.integers(0, n, size=30_000), [0, n - 1]))
+    dst = rng.permutation(src)  # long paths over the nodes with arcs
+    off = np.zeros(n + 1, dtype=np.uint64)
+    off[src + 1] = 1
+    g = hb.Graph.from_csr(np.cumsum(off, dtype=np.uint64), dst.astype(np.uint32))
+    lockstep(hb, oracle, g, 4, transpose_on_device=True, max_iters=8, check_next=False)
 
 
 @pytest.mark.parametrize("large", [8191, 8192, 8193, 16_384, 16_385, 70_001])

@@ -173,6 +173,7 @@ constexpr UnionVariant kVariants[] = {{0, 0, 0, 0}, {2, 2, 0, 0}, {0, 0, 1, 0}, 
                                       {0, 0, 1, 2}, {0, 0, 2, 0}};
 constexpr int kNumVariants = (int)(sizeof(kVariants) / sizeof(kVariants[0]));
 constexpr int kTunedClasses = 2;  // gather-all standard, filtered standard
+constexpr uint64_t kEventMinArcs = 1ull << 26;  // larger graphs' iterations are timed by events
 constexpr uint64_t kTuneMinArcs = 1ull << 22;  // smaller graphs keep the first variant
 constexpr double kTuneMargin = 0.97;
 
@@ -309,6 +310,7 @@ struct hb_handle {
     bool any31 = false;
     int grid_tile = 1, grid_heavy = 1, grid_mark = 1;
     int sms = 1;
+    bool events = true;                         // iterations timed by events
     int grid_tile_occ = 1;           // the window kernel's grid in its 4-blocks-per-SM variant
     int grid_tile_two = 1;           // ... and in its 2-blocks-per-SM variant
     int grid_staged = 1, grid_staged_occ = 1;  // the staged kernel's grids
@@ -918,15 +920,18 @@ int do_init(hb_handle* h) {
 // enqueue_union (the union kernels of this handle alone) and enqueue_post
 // (predecessor marks, the fixed-order NF sum, totals to the host). Several
 // handles can run their pre and post parts around one shared union launch
-// (multi_iterate).
+// (multi_iterate). `chained`: the three parts follow each other on s, launched
+// directly, so a kernel may be set up while the one in front of it runs. A
+// kernel behind an event is launched plainly. (As nodes of a graph they are
+// plain too: the node's gap is 1.1 us.)
 int enqueue_pre(hb_handle* h, hbk::UnionArgs& a, bool first_systolic, cudaStream_t s,
-                bool external) {
+                bool external, bool chained) {
     const uint64_t n = h->n;
     const uint64_t words = (n + 31) / 32;
     auto rec = [&](cudaEvent_t e) {
         return external ? cudaEventRecordWithFlags(e, s, cudaEventRecordExternal) : cudaEventRecord(e, s);
     };
-    HB_CUDA(h, rec(h->ev[0]));
+    if (h->events) HB_CUDA(h, rec(h->ev[0]));
     // The per-iteration constants and, after the union, the totals move between
     // the pinned host blocks and the device by kernels, not by the copy
     // engines: a served job's step would otherwise queue behind the other jobs'
@@ -948,7 +953,7 @@ int enqueue_pre(hb_handle* h, hbk::UnionArgs& a, bool first_systolic, cudaStream
         // (HB:853-857); scanning the predecessors of the nodes modified in
         // the previous iteration gives the same counters.
         HB_LAUNCH(h, hbk::launch_mark_preds(h->d_bits[h->mod_cur], h->d_toff, h->d_tsucc,
-                                            h->d_bits[h->mbc_cur], n, h->grid_mark, s));
+                                            h->d_bits[h->mbc_cur], n, h->grid_mark, nullptr, s, chained));
     }
     if (h->systolic && h->n_tiles) {
         // the light and medium nodes to check or to copy
@@ -962,7 +967,7 @@ int enqueue_pre(hb_handle* h, hbk::UnionArgs& a, bool first_systolic, cudaStream
         wl.counts = h->d_list_tiles + hbk::list_tiles(n);
         wl.light_list = h->d_light_list;
         wl.medium_list = h->d_medium_list;
-        HB_LAUNCH(h, hbk::launch_work_lists(wl, s));
+        HB_LAUNCH(h, hbk::launch_work_lists(wl, s, chained));
         a.light_list = h->d_light_list;
         a.medium_list = h->d_medium_list;
         a.list_counts = reinterpret_cast<const uint64_t*>(wl.counts);
@@ -977,12 +982,13 @@ int enqueue_pre(hb_handle* h, hbk::UnionArgs& a, bool first_systolic, cudaStream
         a.queue_len = h->d_queue_len;
         a.staged = 0;
     }
-    HB_CUDA(h, rec(h->ev[1]));
+    if (h->events) HB_CUDA(h, rec(h->ev[1]));
     return HB_OK;
 }
 
 // The heavy-node kernel (side stream) and the window kernel of this handle.
-int enqueue_union(hb_handle* h, const hbk::UnionArgs& a, cudaStream_t s, bool window) {
+int enqueue_union(hb_handle* h, const hbk::UnionArgs& a, cudaStream_t s, bool window, bool chained) {
+    if (h->events || h->n_heavy) chained = false;
     if (h->n_heavy) {
         // The heavy nodes (one CTA each) start first on the side stream; the
         // window kernel's blocks take the SMs as they free up, so the long
@@ -1001,11 +1007,12 @@ int enqueue_union(hb_handle* h, const hbk::UnionArgs& a, cudaStream_t s, bool wi
         HB_CUDA(h, cudaEventRecord(h->join, h->side));
     }
     if (window && h->n_tiles && a.staged)
-        HB_LAUNCH(h, hbk::launch_union_staged(h->log2m, a, a.occ ? h->grid_staged_occ : h->grid_staged, s));
+        HB_LAUNCH(h, hbk::launch_union_staged(h->log2m, a, a.occ ? h->grid_staged_occ : h->grid_staged, s,
+                                              chained));
     else if (window && h->n_tiles)
         HB_LAUNCH(h, hbk::launch_union_tile(h->log2m, a,
                                             a.occ == 2 ? h->grid_tile_two : a.occ ? h->grid_tile_occ : h->grid_tile,
-                                            s));
+                                            s, chained));
     return HB_OK;
 }
 
@@ -1014,16 +1021,18 @@ int enqueue_join(hb_handle* h, cudaStream_t s) {
     return HB_OK;
 }
 
-int enqueue_post(hb_handle* h, const hbk::UnionArgs& a, cudaStream_t s, bool external) {
+int enqueue_post(hb_handle* h, const hbk::UnionArgs& a, cudaStream_t s, bool external, bool chained) {
+    const bool behind = chained && !h->events && !h->n_heavy;
     const uint64_t n = h->n;
     auto rec = [&](cudaEvent_t e) {
         return external ? cudaEventRecordWithFlags(e, s, cudaEventRecordExternal) : cudaEventRecord(e, s);
     };
     (void)a;
-    HB_CUDA(h, rec(h->ev[2]));
+    if (h->events) HB_CUDA(h, rec(h->ev[2]));
     if (h->systolic)
         HB_LAUNCH(h, hbk::launch_mark_preds(h->d_bits[h->mod_cur ^ 1], h->d_toff, h->d_tsucc,
-                                            h->d_bits[h->mbc_cur ^ 1], n, h->grid_mark, s));
+                                            h->d_bits[h->mbc_cur ^ 1], n, h->grid_mark, h->d_partials, s,
+                                            behind));
     const size_t n_inst = h->inst_start.empty() ? 0 : h->inst_start.size() - 1;
     if (n_inst) {
         hbk::InstStats is{};
@@ -1033,16 +1042,17 @@ int enqueue_post(hb_handle* h, const hbk::UnionArgs& a, cudaStream_t s, bool ext
         is.mods = h->d_inst_mod;
         is.host_mods = h->h_inst_mod;
         is.host_nfs = h->h_inst_sum;
+        is.total = h->d_partials;
         is.segs = h->d_inst_segs;
         is.part_nf = h->d_inst_nf;
         is.part_mod = h->d_inst_part;
         is.ticket = h->d_inst_ticket;
-        HB_LAUNCH(h, hbk::launch_inst_stats(is, h->inst_segs, s));
+        HB_LAUNCH(h, hbk::launch_inst_stats(is, h->inst_segs, s, h->systolic ? chained : behind));
     }
     // the neighbourhood-function parts in a fixed order, the totals to the host
     HB_LAUNCH(h, hbk::launch_iter_end(h->d_nf_items, h->n_chunks + h->n_heavy, h->d_nf_scratch, h->d_partials,
-                                      h->d_cursor + 1, h->h_tot, s));
-    HB_CUDA(h, rec(h->ev[3]));
+                                      h->d_cursor + 1, h->h_tot, s, h->systolic || n_inst ? chained : behind));
+    if (h->events) HB_CUDA(h, rec(h->ev[3]));
     return HB_OK;
 }
 
@@ -1053,10 +1063,10 @@ int enqueue_post(hb_handle* h, const hbk::UnionArgs& a, cudaStream_t s, bool ext
 // synchronised; the per-iteration constants come from h->h_ic.
 int enqueue_iteration(hb_handle* h, hbk::UnionArgs a, bool first_systolic, cudaStream_t s,
                       bool external) {
-    int r = enqueue_pre(h, a, first_systolic, s, external);
-    if (!r) r = enqueue_union(h, a, s, true);
+    int r = enqueue_pre(h, a, first_systolic, s, external, !external);
+    if (!r) r = enqueue_union(h, a, s, true, !external);
     if (!r) r = enqueue_join(h, s);
-    if (!r) r = enqueue_post(h, a, s, external);
+    if (!r) r = enqueue_post(h, a, s, external, !external);
     return r;
 }
 
@@ -1222,8 +1232,13 @@ int iter_finish(hb_handle* h, IterPlan& p, bool from_graph, double union_ms, hb_
     st.local = h->local;
     st.pre_local = h->pre_local;
     float ms_union = 0.f, ms_all = 0.f;
-    cudaEventElapsedTime(&ms_union, h->ev[1], h->ev[2]);
-    cudaEventElapsedTime(&ms_all, h->ev[0], h->ev[3]);
+    if (h->events) {
+        cudaEventElapsedTime(&ms_union, h->ev[1], h->ev[2]);
+        cudaEventElapsedTime(&ms_all, h->ev[0], h->ev[3]);
+    } else {
+        if (tot.union_end > tot.union_begin) ms_union = (float)((double)(tot.union_end - tot.union_begin) * 1e-6);
+        ms_all = (float)((double)(tot.end - tot.begin) * 1e-6);
+    }
     st.union_ms = union_ms >= 0.0 ? union_ms : ms_union;
     st.iteration_ms = ms_all;
     st.scanned_arcs = host.st[3];
@@ -1389,7 +1404,7 @@ static int multi_enqueue(std::vector<hb_handle*>& hs, std::vector<IterPlan>& pla
         const cudaStream_t y = own(j) ? hs[j]->stream : x;
         if (y != x)
             if (cudaError_t e = fork(j); e != cudaSuccess) return fail(e);
-        if ((r = enqueue_pre(hs[j], plans[j].a, plans[j].first_systolic, y, external))) return r;
+        if ((r = enqueue_pre(hs[j], plans[j].a, plans[j].first_systolic, y, external, false))) return r;
         if (y != x)
             if (cudaError_t e = join(j); e != cudaSuccess) return fail(e);
     }
@@ -1420,7 +1435,7 @@ static int multi_enqueue(std::vector<hb_handle*>& hs, std::vector<IterPlan>& pla
         hb_handle* h = hs[j];
         // handles outside the shared kernel launch their own window kernel
         const bool own = h->n_tiles && (!job_kernel_log2m(h->log2m) || plans[j].a.far_tma);
-        if ((r = enqueue_union(h, plans[j].a, x, own))) return r;
+        if ((r = enqueue_union(h, plans[j].a, x, own, false))) return r;
     }
     if (J) {
         const int e = hbk::launch_union_jobs(p, mc.grid, x);
@@ -1439,7 +1454,7 @@ static int multi_enqueue(std::vector<hb_handle*>& hs, std::vector<IterPlan>& pla
         const cudaStream_t y = own(j) ? hs[j]->stream : x;
         if (y != x)
             if (cudaError_t e = fork(j); e != cudaSuccess) return fail(e);
-        if ((r = enqueue_post(hs[j], plans[j].a, y, external))) return r;
+        if ((r = enqueue_post(hs[j], plans[j].a, y, external, false))) return r;
         if (y != x)
             if (cudaError_t e = join(j); e != cudaSuccess) return fail(e);
     }
@@ -2461,6 +2476,13 @@ static int create_impl(const hb_graph_view* graph, const hb_graph_view* transpos
     h->grid_heavy = hbk::heavy_grid(h->log2m, h->device);
     if ((uint64_t)h->grid_heavy > h->n_heavy_items + 1) h->grid_heavy = (int)(h->n_heavy_items + 1);
     h->sms = hbk::num_sms(h->device);
+    // Four timing events an iteration stand between its launches and keep them
+    // from being chained. Below kEventMinArcs the kernels read the device's
+    // clock instead (steps of 32 ns): an iteration on 1e4 nodes takes 25 instead
+    // of 36 us, ones on 1e6 nodes (1.2e7 arcs) 11 us less of 50 to 200. From
+    // 6.7e7 arcs on an iteration that merges all takes over 0.5 ms, where that
+    // is 2% and less.
+    h->events = h->m >= kEventMinArcs;
     h->grid_mark = 8 * h->sms;
     // integer totals of the union kernels (atomics) and the summed
     // neighbourhood function

@@ -38,6 +38,8 @@ struct TilePartial {
     unsigned long long scanned;   // scanned nodes
     unsigned long long sarcs;     // arcs of the scanned nodes
     unsigned long long timeouts;  // bounded mbarrier waits that gave up (an error)
+    // moments of the iteration, in nanoseconds of the device's clock
+    unsigned long long begin, union_begin, union_end, end;
 };
 
 // The values of one iteration t that the kernels read from device memory, so
@@ -155,6 +157,7 @@ struct InstStats {
     unsigned long long* host_mods;    // page-locked memory,
     double* host_nfs;                 // with the neighbourhood function
     const uint2* segs;                // instance and segment of each block
+    TilePartial* total;
     double* part_nf;                  // per segment
     unsigned long long* part_mod;
     uint32_t* ticket;                 // per instance, zero between launches
@@ -172,11 +175,13 @@ struct WorkLists {
 static_assert(sizeof(IterConsts) % 8 == 0 && sizeof(TilePartial) % 8 == 0, "copied as 64-bit words");
 
 // Launchers (hb_kernels.cu). All return cudaError_t as int.
+// chained: the kernel in front of it on the stream is one of these, and it may be
+// set up while that one runs (launch_chain.cuh)
 int launch_iter_begin(const IterBegin& a, int device_sms, void* stream);
 // fixed-order sum of `count` doubles (part: 256 doubles) into total->nf, and the
 // totals to the host's page-locked copy
 int launch_iter_end(const double* in, uint64_t count, double* part, TilePartial* total, unsigned long long* ticket,
-                    TilePartial* host, void* stream);
+                    TilePartial* host, void* stream, bool chained);
 int launch_init(int log2m, const InitArgs& a, void* stream);
 // device counters (one byte per register) -> the reference's packed layout,
 // in caller node order (inv: caller node -> device node)
@@ -211,14 +216,14 @@ int launch_cross_arcs(const uint64_t* off, uint64_t n, uint64_t m, const uint32_
 int launch_gather_f64(const double* src, const uint32_t* inv, double* dst, uint64_t n,
                       void* stream);
 // persistent tile kernel over the worklist (or all tiles)
-int launch_union_tile(int log2m, const UnionArgs& a, int grid, void* stream);
+int launch_union_tile(int log2m, const UnionArgs& a, int grid, void* stream, bool chained);
 // A TMA descriptor for a counter array (n rows of 2^log2m bytes) as the union
 // kernel's far gathers read it; nonzero when the TMA path is not available
 // for this size (log2m > 8, n >= 2^31) or the driver cannot encode it.
 int encode_far_map(int log2m, const uint8_t* counters, uint64_t n, CUtensorMap* out);
 int tile_grid(int log2m, int device, int occ);
 // standard iterations on the staged window kernel (items table; m < 2^32)
-int launch_union_staged(int log2m, const UnionArgs& a, int grid, void* stream);
+int launch_union_staged(int log2m, const UnionArgs& a, int grid, void* stream, bool chained);
 int staged_grid(int log2m, int device, int occ);
 // the window work of several handles in one launch (log2m 4, 6 or 8 each):
 // every job's arguments travel as kernel parameters (constant bank), so at
@@ -250,14 +255,14 @@ int tile_capacity(int log2m, uint32_t* nodes, uint32_t* arcs);
 // heavy nodes, one CTA each
 int launch_union_heavy(int log2m, const UnionArgs& a, int grid, void* stream);
 int heavy_grid(int log2m, int device);
-int launch_inst_stats(const InstStats& a, uint32_t segs, void* stream);
+int launch_inst_stats(const InstStats& a, uint32_t segs, void* stream, bool chained);
 uint64_t list_tiles(uint64_t n);
-int launch_work_lists(const WorkLists& a, void* stream);
+int launch_work_lists(const WorkLists& a, void* stream, bool chained);
 // nodes per chunk of the union kernel: light nodes (lane-group each) and
 // medium nodes (team each)
 int chunk_nodes(int log2m, uint32_t* light, uint32_t* medium);
 int launch_mark_preds(const uint32_t* next_mod, const uint64_t* toff, const uint32_t* tsucc,
-                      uint32_t* next_mbc, uint64_t n, int grid, void* stream);
+                      uint32_t* next_mbc, uint64_t n, int grid, TilePartial* total, void* stream, bool chained);
 int launch_fill_u32(uint32_t* p, uint32_t v, uint64_t count, void* stream);
 int launch_transpose_count(const uint32_t* succ, uint64_t m, unsigned long long* indeg,
                            void* stream);

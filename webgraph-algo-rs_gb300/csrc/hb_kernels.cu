@@ -33,6 +33,7 @@
 
 #include "hb_internal.h"
 #include "hll_device.cuh"
+#include "launch_chain.cuh"
 
 using namespace hbd;
 
@@ -42,6 +43,22 @@ namespace hbk {
 static thread_local uint64_t t_launches = 0;
 uint64_t launch_count() { return t_launches; }
 void count_launches(int64_t delta) { t_launches += (uint64_t)delta; }
+
+// nanoseconds (in steps of 32)
+__device__ __forceinline__ unsigned long long clock_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+
+// the union's first and last moment (one thread of each union kernel's first
+// block; of the kernel behind the union)
+__device__ __forceinline__ void stamp_union(const UnionArgs& a) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicMin(&a.partials[a.acc_slot].union_begin, clock_ns());
+}
+__device__ __forceinline__ void stamp_after(TilePartial* t) {
+    if (blockIdx.x == 0 && threadIdx.x == 0 && t->union_end == 0) t->union_end = clock_ns();
+}
 
 // ---------------------------------------------------------------------------
 // block-level publish of per-thread statistics into one partial slot
@@ -786,6 +803,8 @@ __device__ __forceinline__ uint2 item_at(const UnionArgs& a, const WorkItems& w,
 // build has the registers for 2 at 16 words per lane)
 template <int LOG2M, bool FAR, int MINB, int PIPEX = 0>
 __global__ void __launch_bounds__(256, MINB) k_union_window(const __grid_constant__ UnionArgs a) {
+    hbl::wait_for_launch();
+    stamp_union(a);
     using Gm = Geo<LOG2M>;
     constexpr int G = Gm::CHUNKS;
     constexpr int TB_MED = team_lanes<LOG2M>();
@@ -1252,6 +1271,8 @@ __device__ __forceinline__ void staged_nodes(const UnionArgs& a, uint32_t buf, i
 // IDS: successor ids staged too (else read from global memory in the loop)
 template <int LOG2M, int MINB, int PIPE_L, bool IDS>
 __global__ void __launch_bounds__(256, MINB) k_union_staged(const __grid_constant__ UnionArgs a) {
+    hbl::wait_for_launch();
+    stamp_union(a);
     using Gm = Geo<LOG2M>;
     using SG = StageGeo<LOG2M>;
     constexpr int G = Gm::CHUNKS;
@@ -1347,6 +1368,7 @@ __global__ void k_chunk_items(const uint2* __restrict__ chunks, uint64_t n_chunk
 // ---------------------------------------------------------------------------
 template <int LOG2M>
 __global__ void __launch_bounds__(256) k_union_heavy(const __grid_constant__ UnionArgs a) {
+    stamp_union(a);
     using Gm = Geo<LOG2M>;
     constexpr int G = Gm::CHUNKS, NW = Gm::NW, M4 = Gm::M / 4;
     constexpr int TEAM = 256, P = TEAM / G, WARPS = TEAM / 32;
@@ -1624,12 +1646,16 @@ __device__ __forceinline__ void clear(uint32_t* p, uint64_t words, uint64_t t0, 
 }
 
 __global__ void k_iter_begin(const IterBegin a) {
+    const unsigned long long now = clock_ns();
     const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
     // the iteration's constants, from page-locked memory
     if (t0 < sizeof(IterConsts) / 8)
         reinterpret_cast<uint64_t*>(a.ic)[t0] = reinterpret_cast<const volatile uint64_t*>(a.ic_host)[t0];
     if (t0 == 0) {
-        *a.total = TilePartial{};
+        TilePartial t{};
+        t.begin = now;
+        t.union_begin = ~0ull;
+        *a.total = t;
         a.cursor[0] = 0;  // the union kernels' cursor
         a.cursor[1] = 0;  // k_iter_end's ticket
     }
@@ -1668,6 +1694,8 @@ __global__ void __launch_bounds__(SUM_THREADS) k_iter_end(const double* __restri
                                                           TilePartial* __restrict__ host) {
     __shared__ double s[SUM_THREADS];
     __shared__ bool last;
+    hbl::wait_for_launch();
+    stamp_after(total);
     const uint64_t per = (count + gridDim.x - 1) / gridDim.x;
     const uint64_t b = (uint64_t)blockIdx.x * per, e = min(count, b + per);
     double x = 0.0;
@@ -1694,6 +1722,7 @@ __global__ void __launch_bounds__(SUM_THREADS) k_iter_end(const double* __restri
     if (threadIdx.x == 0) {
         TilePartial t = *total;
         t.nf = nf;
+        t.end = clock_ns();
         *total = t;
         *host = t;
     }
@@ -1713,6 +1742,8 @@ __global__ void __launch_bounds__(INST_THREADS) k_inst_stats(const InstStats a) 
     __shared__ double s_nf[INST_THREADS];
     __shared__ unsigned long long s_mc[INST_THREADS / 32];
     constexpr int T = INST_THREADS;
+    hbl::wait_for_launch();
+    stamp_after(a.total);
     const uint2 is = __ldg(a.segs + blockIdx.x);
     const uint32_t i = is.x, seg = is.y;
     if (a.mods[i] == 0) return;  // written below only when every block has read it
@@ -1986,9 +2017,12 @@ constexpr int MARK_THREADS = 256, MARK_HUB = 1024, MARK_HUBS = 64;
 __global__ void __launch_bounds__(MARK_THREADS) k_mark_preds(const uint32_t* __restrict__ next_mod,
                                                              const uint64_t* __restrict__ toff,
                                                              const uint32_t* __restrict__ tsucc,
-                                                             uint32_t* __restrict__ next_mbc, uint64_t n, int lg) {
+                                                             uint32_t* __restrict__ next_mbc, uint64_t n, int lg,
+                                                             TilePartial* total) {
     __shared__ uint64_t hub[MARK_HUBS][2];
     __shared__ int hubs;
+    hbl::wait_for_launch();
+    if (total) stamp_after(total);
     if (threadIdx.x == 0) hubs = 0;
     __syncthreads();
     const int lane = threadIdx.x & 31;
@@ -2117,6 +2151,7 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long x) {
 }
 
 __global__ void __launch_bounds__(LIST_THREADS) k_list_count(const WorkLists a) {
+    hbl::wait_for_launch();
     __shared__ unsigned long long s[LIST_THREADS / 32];
     uint32_t lb[LIST_ITEMS], mb[LIST_ITEMS];
     const unsigned long long c =
@@ -2131,6 +2166,7 @@ __global__ void __launch_bounds__(LIST_THREADS) k_list_count(const WorkLists a) 
 }
 
 __global__ void __launch_bounds__(LIST_THREADS) k_list_fill(const WorkLists a) {
+    hbl::wait_for_launch();
     __shared__ unsigned long long s[LIST_THREADS / 32], s_base[LIST_THREADS / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t w = (uint64_t)blockIdx.x * LIST_TILE + threadIdx.x * LIST_ITEMS;
@@ -2475,8 +2511,14 @@ int encode_far_map(int log2m, const uint8_t* counters, uint64_t n, CUtensorMap* 
 #undef CALL
 }
 
+// a launch's error, which is also the thread's last error (cleared here)
+static int launched(cudaError_t e) {
+    if (e != cudaSuccess) cudaGetLastError();
+    return (int)e;
+}
+
 template <int LOG2M, bool FAR, int MINB, int PIPEX = 0>
-static int tile_launch(const UnionArgs& a, int grid, cudaStream_t s) {
+static int tile_launch(const UnionArgs& a, int grid, cudaStream_t s, bool chained) {
     constexpr int smem = far_bytes<LOG2M, FAR>();
     if constexpr (smem > 48 * 1024) {
         static const cudaError_t attr = cudaFuncSetAttribute(
@@ -2484,21 +2526,20 @@ static int tile_launch(const UnionArgs& a, int grid, cudaStream_t s) {
         if (attr != cudaSuccess) return (int)attr;
     }
     ++t_launches;
-    k_union_window<LOG2M, FAR, MINB, PIPEX><<<grid, 256, smem, s>>>(a);
-    return (int)cudaGetLastError();
+    return launched(hbl::launch(chained, k_union_window<LOG2M, FAR, MINB, PIPEX>, grid, 256, smem, s, a));
 }
 
 template <int LOG2M>
-static int tile_impl(const UnionArgs& a, int grid, cudaStream_t s) {
+static int tile_impl(const UnionArgs& a, int grid, cudaStream_t s, bool chained) {
     if constexpr (FarGeo<LOG2M>::ON)
-        if (a.far_tma) return tile_launch<LOG2M, true, 3>(a, grid, s);
-    if (a.occ == 2) return tile_launch<LOG2M, false, 2, Geo<LOG2M>::NW >= 16 ? 2 : 0>(a, grid, s);
-    if (a.occ) return tile_launch<LOG2M, false, 4>(a, grid, s);
-    return tile_launch<LOG2M, false, 3>(a, grid, s);
+        if (a.far_tma) return tile_launch<LOG2M, true, 3>(a, grid, s, chained);
+    if (a.occ == 2) return tile_launch<LOG2M, false, 2, Geo<LOG2M>::NW >= 16 ? 2 : 0>(a, grid, s, chained);
+    if (a.occ) return tile_launch<LOG2M, false, 4>(a, grid, s, chained);
+    return tile_launch<LOG2M, false, 3>(a, grid, s, chained);
 }
 
 template <int LOG2M, int MINB, bool IDS>
-static int staged_launch(const UnionArgs& a, int grid, cudaStream_t s) {
+static int staged_launch(const UnionArgs& a, int grid, cudaStream_t s, bool chained) {
     constexpr int smem = staged_smem_bytes<LOG2M>();
     constexpr int PIPE_L = pipe_depth<Geo<LOG2M>::NW>();
     if constexpr (smem > 48 * 1024) {
@@ -2507,19 +2548,18 @@ static int staged_launch(const UnionArgs& a, int grid, cudaStream_t s) {
         if (attr != cudaSuccess) return (int)attr;
     }
     ++t_launches;
-    k_union_staged<LOG2M, MINB, PIPE_L, IDS><<<grid, 256, smem, s>>>(a);
-    return (int)cudaGetLastError();
+    return launched(hbl::launch(chained, k_union_staged<LOG2M, MINB, PIPE_L, IDS>, grid, 256, smem, s, a));
 }
 
 // a.staged: 1 = ids staged, 2 = ids from global memory
 template <int LOG2M>
-static int staged_impl(const UnionArgs& a, int grid, cudaStream_t s) {
+static int staged_impl(const UnionArgs& a, int grid, cudaStream_t s, bool chained) {
     if (a.staged == 2) {
-        if (a.occ) return staged_launch<LOG2M, 4, false>(a, grid, s);
-        return staged_launch<LOG2M, 3, false>(a, grid, s);
+        if (a.occ) return staged_launch<LOG2M, 4, false>(a, grid, s, chained);
+        return staged_launch<LOG2M, 3, false>(a, grid, s, chained);
     }
-    if (a.occ) return staged_launch<LOG2M, 4, true>(a, grid, s);
-    return staged_launch<LOG2M, 3, true>(a, grid, s);
+    if (a.occ) return staged_launch<LOG2M, 4, true>(a, grid, s, chained);
+    return staged_launch<LOG2M, 3, true>(a, grid, s, chained);
 }
 
 template <int LOG2M>
@@ -2603,21 +2643,20 @@ int launch_iter_begin(const IterBegin& a, int device_sms, void* stream) {
 }
 
 int launch_iter_end(const double* in, uint64_t count, double* part, TilePartial* total, unsigned long long* ticket,
-                    TilePartial* host, void* stream) {
+                    TilePartial* host, void* stream, bool chained) {
     // a block a 2,048 parts, eight loads a thread in flight; one block alone needs
     // no second pass (8 iterations on 1e4 nodes: 5.9 us each with 256 blocks)
     static_assert(REDUCE_BLOCKS <= SUM_THREADS, "one part a thread");
     const int grid = (int)std::min<uint64_t>(std::max<uint64_t>((count + 2047) / 2048, 1), REDUCE_BLOCKS);
     ++t_launches;
-    k_iter_end<<<grid, SUM_THREADS, 0, (cudaStream_t)stream>>>(in, count, part, total, ticket, host);
-    return (int)cudaGetLastError();
+    return launched(hbl::launch(chained, k_iter_end, grid, SUM_THREADS, 0, (cudaStream_t)stream, in, count, part, total,
+                                ticket, host));
 }
 
-int launch_inst_stats(const InstStats& a, uint32_t segs, void* stream) {
+int launch_inst_stats(const InstStats& a, uint32_t segs, void* stream, bool chained) {
     if (!segs) return 0;
     ++t_launches;
-    k_inst_stats<<<segs, INST_THREADS, 0, (cudaStream_t)stream>>>(a);
-    return (int)cudaGetLastError();
+    return launched(hbl::launch(chained, k_inst_stats, (int)segs, INST_THREADS, 0, (cudaStream_t)stream, a));
 }
 
 int launch_perm_degree(const uint64_t* off0, const uint32_t* perm, uint64_t n,
@@ -2681,14 +2720,14 @@ int launch_gather_f64(const double* src, const uint32_t* inv, double* dst, uint6
     return (int)cudaGetLastError();
 }
 
-int launch_union_tile(int log2m, const UnionArgs& a, int grid, void* stream) {
-#define CALL(L) tile_impl<L>(a, grid, (cudaStream_t)stream)
+int launch_union_tile(int log2m, const UnionArgs& a, int grid, void* stream, bool chained) {
+#define CALL(L) tile_impl<L>(a, grid, (cudaStream_t)stream, chained)
     HB_DISPATCH_LOG2M(log2m, CALL)
 #undef CALL
 }
 
-int launch_union_staged(int log2m, const UnionArgs& a, int grid, void* stream) {
-#define CALL(L) staged_impl<L>(a, grid, (cudaStream_t)stream)
+int launch_union_staged(int log2m, const UnionArgs& a, int grid, void* stream, bool chained) {
+#define CALL(L) staged_impl<L>(a, grid, (cudaStream_t)stream, chained)
     HB_DISPATCH_LOG2M(log2m, CALL)
 #undef CALL
 }
@@ -2791,20 +2830,18 @@ int chunk_nodes(int log2m, uint32_t* light, uint32_t* medium) {
 
 uint64_t list_tiles(uint64_t n) { return std::max<uint64_t>(((n + 31) / 32 + LIST_TILE - 1) / LIST_TILE, 1); }
 
-int launch_work_lists(const WorkLists& a, void* stream) {
+int launch_work_lists(const WorkLists& a, void* stream, bool chained) {
     cudaStream_t s = (cudaStream_t)stream;
-    const unsigned grid = (unsigned)list_tiles(a.nwords * 32);
+    const int grid = (int)list_tiles(a.nwords * 32);
     ++t_launches;
-    k_list_count<<<grid, LIST_THREADS, 0, s>>>(a);
-    const int e = (int)cudaGetLastError();
+    const int e = launched(hbl::launch(chained, k_list_count, grid, LIST_THREADS, 0, s, a));
     if (e) return e;
     ++t_launches;
-    k_list_fill<<<grid, LIST_THREADS, 0, s>>>(a);
-    return (int)cudaGetLastError();
+    return launched(hbl::launch(chained, k_list_fill, grid, LIST_THREADS, 0, s, a));
 }
 
 int launch_mark_preds(const uint32_t* next_mod, const uint64_t* toff, const uint32_t* tsucc,
-                      uint32_t* next_mbc, uint64_t n, int grid, void* stream) {
+                      uint32_t* next_mbc, uint64_t n, int grid, TilePartial* total, void* stream, bool chained) {
     const uint64_t nwords = (n + 31) / 32;
     constexpr uint64_t warps = MARK_THREADS / 32;
     grid = (int)std::min<uint64_t>((uint64_t)grid, (nwords + warps - 1) / warps);
@@ -2813,8 +2850,8 @@ int launch_mark_preds(const uint32_t* next_mod, const uint64_t* toff, const uint
     int lg = 0;
     while (lg < 3 && nwords > (uint64_t)grid * warps * 32 << lg) lg++;
     ++t_launches;
-    k_mark_preds<<<grid, MARK_THREADS, 0, (cudaStream_t)stream>>>(next_mod, toff, tsucc, next_mbc, n, lg);
-    return (int)cudaGetLastError();
+    return launched(hbl::launch(chained, k_mark_preds, grid, MARK_THREADS, 0, (cudaStream_t)stream, next_mod, toff, tsucc,
+                                next_mbc, n, lg, total));
 }
 
 int launch_fill_u32(uint32_t* p, uint32_t v, uint64_t count, void* stream) {

@@ -36,6 +36,8 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "launch_chain.cuh"
+
 namespace hbl {
 
 constexpr uint32_t UNIT = 8;
@@ -51,26 +53,6 @@ constexpr uint32_t SMALL = 2048, SMALL_GLOBAL = 512;
 constexpr uint32_t TINY = 16384;       // any level of a graph of at most this many units
 constexpr uint32_t CAP = 512;          // entries of a level in shared memory
 constexpr uint32_t BITS = 512 * 1024;  // nodes whose visited bits fit shared memory
-
-// Launches in a chain: every kernel waits for the one in front of it at its
-// first instruction, so it may be set up while that one still runs. A launch
-// then costs 1.4 us instead of 4.1 (152 to 1216 blocks, measured back to back).
-__device__ __forceinline__ void wait_for_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
-template <class... P, class... A>
-inline cudaError_t chain(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
-}
 
 // The frontier is queue slots [b, e) with `units` units; d is the distance its
 // successors get, last the largest distance that reached a node.

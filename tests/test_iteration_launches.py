@@ -76,3 +76,22 @@ def test_instance_segments(hb, large):
             np.testing.assert_allclose(b.sum_of_distances(i), h.sum_of_distances(), rtol=1e-12)
             h.close()
     b.close()
+
+
+@pytest.mark.parametrize("n,cap", [(50, 10), (5000, 10), (60_000, 5000)])
+def test_iteration_times(hb, n, cap):
+    """The device's times of directly launched and of replayed iterations, with
+    and without heavy nodes: the union lies within the iteration, and both
+    within the wall time of the run."""
+    import time
+    g = hb.Graph.weblike(n, cap=cap, window=32, seed=1)
+    logic = hb.HyperLogLogBuilder(n).log_2_num_reg(6).build()
+    h = hb.HyperBallBuilder.new(g, logic).transpose_on_device(True).build()
+    for _ in range(3):
+        t0 = time.perf_counter()
+        h.run_until_done()
+        wall = (time.perf_counter() - t0) * 1e3
+        st = h.iteration_stats()
+        assert all(0 < s["union_ms"] < s["iteration_ms"] for s in st)
+        assert sum(s["iteration_ms"] for s in st) < wall
+    h.close()

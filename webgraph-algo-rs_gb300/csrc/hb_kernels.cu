@@ -1722,9 +1722,12 @@ __global__ void __launch_bounds__(SUM_THREADS) k_iter_end(const double* __restri
     if (threadIdx.x == 0) {
         TilePartial t = *total;
         t.nf = nf;
-        t.end = clock_ns();
-        *total = t;
+        t.end = 0;
         *host = t;
+        __threadfence_system();
+        // the host may go on once it sees this
+        *reinterpret_cast<volatile unsigned long long*>(&host->end) = t.end = clock_ns();
+        *total = t;
     }
 }
 

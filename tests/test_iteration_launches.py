@@ -95,3 +95,25 @@ def test_iteration_times(hb, n, cap):
         assert all(0 < s["union_ms"] < s["iteration_ms"] for s in st)
         assert sum(s["iteration_ms"] for s in st) < wall
     h.close()
+
+
+@pytest.mark.parametrize("log2ms", [[4], [9], [4, 6, 8], [5, 4, 10, 7, 8, 6, 9]])
+def test_groups_side_by_side(hb, log2ms):
+    """A batch's groups, one for each counter size, with heavy nodes in some and
+    runs of different lengths: as alone, first launched and then replayed."""
+    gs = [hb.Graph.weblike(9000, cap=3000, window=32, seed=k) if k % 2 else hb.Graph.erdos_renyi(700 * (k + 1), 4, k)
+          for k in range(len(log2ms))]
+    b = hb.HyperBallBatch(gs, log2ms, sum_of_distances=True)
+    for _ in range(3):
+        b.run_until_done()
+        for i, (g, m) in enumerate(zip(gs, log2ms)):
+            logic = hb.HyperLogLogBuilder(g.num_nodes).log_2_num_reg(m).build()
+            h = hb.HyperBallBuilder.new(g, logic).transpose_on_device(True).sum_of_distances(True).build()
+            h.run_until_done()
+            assert b.iterations(i) == h.iteration, i
+            np.testing.assert_array_equal(b.registers(i), h.registers())
+            np.testing.assert_allclose(b.neighborhood_function(i), h.neighborhood_function(), rtol=1e-12)
+            np.testing.assert_allclose(b.sum_of_distances(i), h.sum_of_distances(), rtol=1e-12)
+            h.close()
+    assert b.stats()["union_ms"] > 0
+    b.close()

@@ -131,7 +131,19 @@ struct InitArgs {
     double alpha_m_m;
     const double* ln_table;
     int quirk;
-    int* any31;               // set to 1 when an initial register holds 30 or 31
+    int* any31;               // page-locked; set to 1 when an initial register holds 30 or 31
+};
+
+// Before init: arrays to zero (8 and a discount's each), the modified bitmap to
+// set, a batch's modified counts to set.
+struct ResetArgs {
+    uint32_t* p[8 + MAX_DISCOUNT];
+    uint64_t words[8 + MAX_DISCOUNT];
+    int count;
+    uint32_t* ones;
+    uint64_t n;                      // bits of it
+    unsigned long long* inst_mod;
+    uint64_t n_inst;
 };
 
 // The first kernel of an iteration: bitmaps, totals, cursors and
@@ -182,6 +194,8 @@ int launch_iter_begin(const IterBegin& a, int device_sms, void* stream);
 // totals to the host's page-locked copy
 int launch_iter_end(const double* in, uint64_t count, double* part, TilePartial* total, unsigned long long* ticket,
                     TilePartial* host, void* stream, bool chained);
+int launch_reset(const ResetArgs& a, int device_sms, void* stream);
+// (behind launch_reset on the stream)
 int launch_init(int log2m, const InitArgs& a, void* stream);
 // device counters (one byte per register) -> the reference's packed layout,
 // in caller node order (inv: caller node -> device node)
@@ -263,7 +277,6 @@ int launch_work_lists(const WorkLists& a, void* stream, bool chained);
 int chunk_nodes(int log2m, uint32_t* light, uint32_t* medium);
 int launch_mark_preds(const uint32_t* next_mod, const uint64_t* toff, const uint32_t* tsucc,
                       uint32_t* next_mbc, uint64_t n, int grid, TilePartial* total, void* stream, bool chained);
-int launch_fill_u32(uint32_t* p, uint32_t v, uint64_t count, void* stream);
 int launch_transpose_count(const uint32_t* succ, uint64_t m, unsigned long long* indeg,
                            void* stream);
 int launch_exclusive_scan_u64(const unsigned long long* in, uint64_t* out, uint64_t count,

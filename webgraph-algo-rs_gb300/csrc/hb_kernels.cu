@@ -1542,6 +1542,7 @@ __device__ __forceinline__ uint32_t add_hash(uint8_t* counter, uint64_t x, uint3
 
 template <int LOG2M>
 __global__ void __launch_bounds__(256) k_init(InitArgs a) {
+    hbl::wait_for_launch();
     using Gm = Geo<LOG2M>;
     bool saw_big = false;
     for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < a.n;
@@ -1592,7 +1593,7 @@ __global__ void __launch_bounds__(256) k_init(InitArgs a) {
     }
     // Registers only ever take values some initial register had; remember
     // whether 30 or 31 occurs, which the fast form of the counts excludes.
-    if (__syncthreads_or(saw_big) && threadIdx.x == 0) atomicOr(a.any31, 1);
+    if (__syncthreads_or(saw_big) && threadIdx.x == 0) *reinterpret_cast<volatile int*>(a.any31) = 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -1643,6 +1644,18 @@ __device__ __forceinline__ void clear(uint32_t* p, uint64_t words, uint64_t t0, 
     for (uint64_t i = t0; i < words / 4; i += stride) q[i] = make_uint4(0u, 0u, 0u, 0u);
     const uint64_t i = words / 4 * 4 + t0;
     if (i < words) p[i] = 0u;
+}
+
+// What init starts from, in one launch (with a clear for each, up to eleven of
+// them and two copies, init of 1e4 nodes took 50 us, now 16; 1e6 nodes at log2m
+// 6 took 100, now 57).
+__global__ void k_reset(const __grid_constant__ ResetArgs a) {
+    const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    for (int k = 0; k < a.count; k++) clear(a.p[k], a.words[k], t0, stride);
+    const uint64_t words = (a.n + 31) / 32;
+    for (uint64_t w = t0; w < words; w += stride)
+        a.ones[w] = w == a.n / 32 ? (1u << (a.n % 32)) - 1u : 0xffffffffu;
+    for (uint64_t i = t0; i < a.n_inst; i += stride) a.inst_mod[i] = ~0ull;
 }
 
 __global__ void k_iter_begin(const IterBegin a) {
@@ -2202,11 +2215,6 @@ __global__ void __launch_bounds__(LIST_THREADS) k_list_fill(const WorkLists a) {
     }
 }
 
-__global__ void k_fill_u32(uint32_t* p, uint32_t v, uint64_t count) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count;
-         i += (uint64_t)gridDim.x * blockDim.x)
-        p[i] = v;
-}
 
 // ---------------------------------------------------------------------------
 // transpose on the device: in-degree count, exclusive scan, scatter
@@ -2445,12 +2453,17 @@ int num_sms(int device) {
         default: return (int)cudaErrorInvalidValue; \
     }
 
+// a launch's error, which is also the thread's last error (cleared here)
+static int launched(cudaError_t e) {
+    if (e != cudaSuccess) cudaGetLastError();
+    return (int)e;
+}
+
 template <int LOG2M>
 static int init_impl(const InitArgs& a, cudaStream_t s) {
     const int grid = (int)std::min<uint64_t>((a.n + 255) / 256 + 1, 65535);
     ++t_launches;
-    k_init<LOG2M><<<grid, 256, 0, s>>>(a);
-    return (int)cudaGetLastError();
+    return launched(hbl::launch(true, k_init<LOG2M>, grid, 256, 0, s, a));
 }
 
 template <int LOG2M>
@@ -2512,12 +2525,6 @@ int encode_far_map(int log2m, const uint8_t* counters, uint64_t n, CUtensorMap* 
 #define CALL(L) encode_far_impl<L>(counters, n, out)
     HB_DISPATCH_LOG2M(log2m, CALL)
 #undef CALL
-}
-
-// a launch's error, which is also the thread's last error (cleared here)
-static int launched(cudaError_t e) {
-    if (e != cudaSuccess) cudaGetLastError();
-    return (int)e;
 }
 
 template <int LOG2M, bool FAR, int MINB, int PIPEX = 0>
@@ -2634,6 +2641,15 @@ int launch_add_indeg(unsigned long long* rows, const uint32_t* indeg, uint64_t n
     const int grid = (int)std::min<uint64_t>((n + 255) / 256, 8192);
     ++t_launches;
     k_add_indeg<<<grid, 256, 0, (cudaStream_t)stream>>>(rows, indeg, n);
+    return (int)cudaGetLastError();
+}
+
+int launch_reset(const ResetArgs& a, int device_sms, void* stream) {
+    uint64_t words = a.n / 32 + a.n_inst + 1;
+    for (int i = 0; i < a.count; i++) words += a.words[i];
+    const int grid = (int)std::min<uint64_t>((words + 1023) / 1024, (uint64_t)device_sms * 8);
+    ++t_launches;
+    k_reset<<<grid, 256, 0, (cudaStream_t)stream>>>(a);
     return (int)cudaGetLastError();
 }
 
@@ -2857,13 +2873,6 @@ int launch_mark_preds(const uint32_t* next_mod, const uint64_t* toff, const uint
                                 next_mbc, n, lg, total));
 }
 
-int launch_fill_u32(uint32_t* p, uint32_t v, uint64_t count, void* stream) {
-    if (count == 0) return 0;
-    const int grid = (int)std::min<uint64_t>((count + 255) / 256, 4096);
-    ++t_launches;
-    k_fill_u32<<<grid, 256, 0, (cudaStream_t)stream>>>(p, v, count);
-    return (int)cudaGetLastError();
-}
 
 int launch_transpose_count(const uint32_t* succ, uint64_t m, unsigned long long* indeg,
                            void* stream) {

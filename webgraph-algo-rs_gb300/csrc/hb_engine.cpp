@@ -301,7 +301,7 @@ struct hb_handle {
     uint64_t n_heavy_items = 0;
     uint8_t* d_heavy_part = nullptr;    // partial counters of split nodes' segments
     uint32_t* d_heavy_arrive = nullptr; // arrival counts of split nodes
-    hbk::TilePartial* d_partials = nullptr;  // one per tile, then one per heavy block
+    hbk::TilePartial* d_partials = nullptr;  // the iteration's totals
     uint64_t n_partials = 0;
     double* d_nf_items = nullptr;     // neighbourhood-function part per work item / heavy node
     double* d_nf_scratch = nullptr;
@@ -1302,8 +1302,9 @@ int do_iterate(hb_handle* h, hb_iter_stats* out) {
 // ---------------------------------------------------------------------------
 // Several handles, one step of an iteration each (no reference counterpart).
 // The log2m groups of a batch advance together, each on a branch of its own.
-// The running jobs of a server share one union launch: each handle's pre part (clears, work lists, queue), one
-// k_union_jobs launch that drains every handle's window work from one cursor
+// The running jobs of a server share one union launch: each handle's pre part
+// (clears, work lists, queue), one k_union_jobs launch that drains every
+// handle's window work from one cursor
 // (the heavy-node kernels beside it on the handles' side streams), each
 // handle's post part, one synchronisation, each handle's bookkeeping. The
 // launch sequence of a set of shapes is captured as a CUDA graph the second

@@ -29,11 +29,11 @@ constexpr uint64_t HEAVY_SEG = 4096;
 // arcs of a segment of a node of `arcs` arcs in nseg segments
 __host__ __device__ constexpr uint64_t heavy_seg_arcs(uint64_t arcs, uint64_t nseg) { return (arcs + nseg - 1) / nseg; }
 
-// What one tile (or one block of the heavy-node kernel) contributes to an
-// iteration; summed in a fixed order after the union kernels.
+// The totals of an iteration: integers added up by the union kernels, the
+// neighbourhood function and the last moment by k_iter_end.
 struct TilePartial {
-    double nf;                    // neighbourhood-function contribution
-    unsigned long long vis;       // arcs the next iteration visits (k_finalize)
+    double nf;                    // neighbourhood function
+    unsigned long long vis;       // arcs the next iteration visits
     unsigned long long mod;       // modified counters
     unsigned long long scanned;   // scanned nodes
     unsigned long long sarcs;     // arcs of the scanned nodes
@@ -103,7 +103,7 @@ struct UnionArgs {
     const uint32_t* queue_len;
     const uint4* items;       // staged kernel: {first node, count | medium << 31, first arc, arcs}
     uint32_t staged;          // 1: standard iteration on the staged kernel (k_union_staged)
-    int gather_all;           // merge every successor (nearly all changed before)
+    int gather_all;           // merge every successor (many changed before)
     const uint32_t* indeg;    // in-degree without self-loops
     double* nf_items;         // neighbourhood-function part of each work item, then of each heavy node
     uint64_t heavy_item_base; // index of the first heavy node's part
@@ -115,7 +115,7 @@ struct UnionArgs {
     uint32_t occ;             // window kernel sized for 4 resident blocks per SM instead of 3
     uint32_t tile_max_degree; // nodes above this out-degree are listed as heavy
     uint32_t acc_slot;        // partial slot accumulating the union kernels' integer totals
-    TilePartial* partials;    // one per finalize block, then acc_slot
+    TilePartial* partials;    // the totals stand at acc_slot
 };
 
 struct InitArgs {
@@ -239,7 +239,7 @@ int tile_grid(int log2m, int device, int occ);
 // standard iterations on the staged window kernel (items table; m < 2^32)
 int launch_union_staged(int log2m, const UnionArgs& a, int grid, void* stream, bool chained);
 int staged_grid(int log2m, int device, int occ);
-// the window work of several handles in one launch (log2m 4, 6 or 8 each):
+// the window work of several handles (a server's jobs) in one launch (log2m 4, 6 or 8 each):
 // every job's arguments travel as kernel parameters (constant bank), so at
 // most 48 jobs fit the 32 KB parameter space
 constexpr int MAX_JOBS = 48;

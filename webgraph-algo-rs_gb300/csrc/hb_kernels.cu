@@ -2,7 +2,8 @@
 //
 // One HyperBall iteration (reference: HyperBall::iterate / parallel_task,
 // src/algo/hyperball/hyperball_impl.rs:775-1152) runs as
-//   1. k_list_count,     — systolic iterations only: the light and medium
+//   1. k_iter_begin      — bitmaps and totals cleared, the constants fetched;
+//      k_list_count,     — systolic iterations only: the light and medium
 //      k_list_fill         nodes to check or to copy, in node order;
 //   2. k_union_window    — one warp per chunk of nodes, chunks taken in node
 //                          order from a global cursor; every node of
@@ -11,11 +12,12 @@
 //                          store, and for changed counters the exact count,
 //                          neighbourhood-function part and per-node f64 sums
 //                          (finish_node) while the counter is in registers;
-//   3. k_union_heavy     — the same for the heavy nodes, one CTA per node;
-//   4. k_sum_f64         — the neighbourhood-function parts summed in a fixed
-//                          order (reproducible);
-//   5. k_mark_preds      — systolic iterations: predecessors of modified nodes
-//                          (through the transpose) into next-must-be-checked.
+//   3. k_union_heavy     — the same for the heavy nodes, one CTA per node or
+//                          segment of one, beside the window kernel;
+//   4. k_mark_preds      — systolic iterations: predecessors of modified nodes
+//                          (through the transpose) into next-must-be-checked;
+//   5. k_iter_end        — the neighbourhood-function parts summed in a fixed
+//                          order (reproducible), the totals to the host.
 // Only successors flagged in the previous iteration's modified bitmap are
 // merged (HB:1038), or all of them where that gives the same counters. The
 // count of an unchanged counter is the cached estimate of the previous
@@ -300,7 +302,8 @@ __device__ __forceinline__ double warp_sum_f64(double x) {
 // length; each lane keeps PIPE counter gathers in flight while the ids and
 // modified bits of the next PIPE successors load.
 //
-// In iterations where nearly every counter changed before (`gather_all`), a
+// In iterations where at least a quarter of the counters changed before
+// (`gather_all`), a
 // successor's counter is merged without its modified bit: an unmodified
 // successor's counter is already contained in the node's own
 // (c_{t-1}(u) = c_{t-2}(u) <= c_{t-1}(v)), and so is the node's own counter,

@@ -110,6 +110,8 @@ cudaError_t pool_alloc(int device, void** p, size_t bytes, cudaStream_t s) {
 // handle. Freed blocks are kept for the next handle instead of going back
 // through cudaFreeHost, which may synchronise the device under the other
 // handles' work (the job server destroys handles while others run).
+// Of the large ones, which stage results, kStagesKept at most are kept.
+constexpr size_t kStageBytes = 1u << 20, kStagesKept = 8;
 std::mutex g_pinned_mu;
 std::multimap<size_t, void*> g_pinned_free;
 
@@ -135,8 +137,15 @@ cudaError_t pinned_alloc(void** p, size_t bytes) {
 
 void pinned_free(void* p, size_t bytes) {
     if (!p) return;
-    std::lock_guard<std::mutex> lk(g_pinned_mu);
-    g_pinned_free.emplace(pinned_class(bytes), p);
+    const size_t c = pinned_class(bytes);
+    {
+        std::lock_guard<std::mutex> lk(g_pinned_mu);
+        if (c < kStageBytes || g_pinned_free.count(c) < kStagesKept) {
+            g_pinned_free.emplace(c, p);
+            return;
+        }
+    }
+    cudaFreeHost(p);
 }
 
 }  // namespace
@@ -1650,8 +1659,6 @@ int copy_d2h(const hb_handle* h, const void* src, void* dst, size_t bytes) {
     HB_CUDA(hh, cudaStreamSynchronize(h->stream));
     return HB_OK;
 }
-
-constexpr size_t kStageBytes = 1u << 20;
 
 // Caller nodes [start, start + count) of a per-node device array (device node
 // order) into dst on the host, in caller order.

@@ -108,7 +108,9 @@ __global__ void k_sw_begin(const hbl::Level a, uint64_t n, const Scratch* pick, 
             s.units = (a.entry[0].deg + hbl::UNIT - 1) / hbl::UNIT;
             a.queue[0] = (uint32_t)r;
         }
-        a.ctl->st[0] = s;
+        // in both: of a start without arcs no launch has a level to expand, and
+        // each writes nothing
+        a.ctl->st[0] = a.ctl->st[1] = s;
         a.ctl->tail = s.e;
         a.ctl->ticket = 0;
         a.ctl->launches = 0;

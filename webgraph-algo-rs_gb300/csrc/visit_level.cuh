@@ -407,7 +407,7 @@ static __global__ void k_info(const uint64_t* __restrict__ off, uint64_t n, Entr
 }
 
 // The start nodes not yet visited, at distance 0: the first level of a visit,
-// in st[0]. They are queued from slot `from` on, where ctl->tail stood before
+// in st[0] and st[1]. They are queued from slot `from` on, where ctl->tail stood before
 // the first of the launches that bring them; `last` marks the last one.
 template <bool PRED>
 __global__ void __launch_bounds__(THREADS, 1) k_starts(const Level a, const uint32_t* __restrict__ starts, uint64_t count,
@@ -439,7 +439,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_starts(const Level a, const uint
             ctl->launches = 0;
             if (last) {
                 const unsigned long long tail = atomicAdd(&ctl->tail, 0ull);
-                ctl->st[0] = State{from, (uint32_t)tail, (uint32_t)(tail >> 32), 1, 0};
+                // in both: a first level without units is the end
+                ctl->st[0] = ctl->st[1] = State{from, (uint32_t)tail, (uint32_t)(tail >> 32), 1, 0};
                 ctl->tail = (uint32_t)tail;
             }
         }

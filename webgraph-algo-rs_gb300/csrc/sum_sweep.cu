@@ -177,7 +177,7 @@ __device__ __forceinline__ void finish_counts(Counts c, Scratch* s, const hbl::C
 
 // true (and the host told) when the visit has not ended
 __device__ __forceinline__ bool unfinished(const hbl::Control* ctl, Result* out) {
-    if (hbl::done(ctl->st[0], INF)) return false;
+    if (hbl::done(ctl->st[0])) return false;
     if (blockIdx.x == 0 && threadIdx.x == 0) out->done = 0;
     return true;
 }
@@ -665,7 +665,7 @@ struct Sweeper {
             hbl::Control* c = reinterpret_cast<hbl::Control*>(h_res + 1);
             ck(cudaMemcpyAsync(c, d_ctl, sizeof *c, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
             sync();
-            if (hbl::done(c->st[0], hbs::INF)) {
+            if (hbl::done(c->st[0])) {
                 learn(backward, c->launches);
                 return;
             }

@@ -37,6 +37,7 @@
 #include <cstdint>
 
 #include "launch_chain.cuh"
+#include "visit_state.h"
 
 namespace hbl {
 
@@ -53,12 +54,6 @@ constexpr uint32_t SMALL = 2048, SMALL_GLOBAL = 512;
 constexpr uint32_t TINY = 16384;       // any level of a graph of at most this many units
 constexpr uint32_t CAP = 512;          // entries of a level in shared memory
 constexpr uint32_t BITS = 512 * 1024;  // nodes whose visited bits fit shared memory
-
-// The frontier is queue slots [b, e) with `units` units; d is the distance its
-// successors get, last the largest distance that reached a node.
-struct State {
-    uint32_t b, e, units, d, last;
-};
 
 // A node's arcs and, where it is queued, the units before it in its level. One
 // such 16-byte word per node (Level::info) replaces two reads of the offsets: a
@@ -309,20 +304,6 @@ __device__ __forceinline__ void expand(const Level& a, const State& s, unsigned 
     flush<PRED>(a, tail, run, fill, true, s.d, loc, side, s.e, a.tile[s.d & 1]);
 }
 
-// the state after level s, whose nodes' queue ends at `tail`
-__device__ __forceinline__ State advance(const State& s, unsigned long long tail) {
-    State t;
-    t.b = s.e;
-    t.e = (uint32_t)tail;
-    t.units = (uint32_t)(tail >> 32);
-    t.last = t.e > t.b ? s.d : s.last;
-    t.d = s.d + 1;
-    return t;
-}
-
-// nothing left to expand
-__device__ __host__ __forceinline__ bool done(const State& s, uint32_t max_d) { return s.units == 0 || s.d > max_d; }
-
 template <bool COMP, bool PRED>
 __global__ void __launch_bounds__(THREADS, 1) k_level(const Level a, int in) {
     extern __shared__ __align__(16) uint8_t smem[];
@@ -332,7 +313,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_level(const Level a, int in) {
     Control* ctl = a.ctl;
     State s = ctl->st[in];
     const bool small = s.units <= a.small;
-    if (done(s, a.max_d) || (small && blockIdx.x != 0)) return;
+    if (done(s) || (small && blockIdx.x != 0)) return;
     unsigned long long known = 0;
     if (small) {
         Local* loc = reinterpret_cast<Local*>(smem + sizeof(Run<PRED>) * WARPS);
@@ -361,18 +342,18 @@ __global__ void __launch_bounds__(THREADS, 1) k_level(const Level a, int in) {
             __syncthreads();
             const unsigned long long t = s_tail;
             __syncthreads();
-            s = advance(s, t);
+            s = advance(s, t, a.max_d);
             if (threadIdx.x == 0) s_tail = s.e;  // read again behind the barriers of the next level
             side ^= 1;
             __syncthreads();
-        } while (--left > 0 && !done(s, a.max_d) && s.units <= a.small);
+        } while (--left > 0 && !done(s) && s.units <= a.small);
         if (mine)
             for (uint32_t i = threadIdx.x; i < words; i += THREADS) a.visited[i] = bits[i];
         if (threadIdx.x == 0) {
             ctl->st[in ^ 1] = s;
-            // an ended visit stands in both: whoever still reads st[in] has
-            // nothing to do either way
-            if (done(s, a.max_d)) ctl->st[in] = s;
+            // an ended visit stands in both: a block that still reads st[in] finds
+            // no units there, or those of the level that was small
+            if (done(s)) ctl->st[in] = s;
             ctl->tail = s.e;
             ctl->launches++;
         }
@@ -384,9 +365,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_level(const Level a, int in) {
             __threadfence();
             if (atomicAdd(&ctl->ticket, 1u) == gridDim.x - 1) {
                 // the last block: the queue is complete
-                const State t = advance(s, atomicAdd(&ctl->tail, 0ull));
+                const State t = advance(s, atomicAdd(&ctl->tail, 0ull), a.max_d);
                 ctl->st[in ^ 1] = t;
-                if (done(t, a.max_d)) ctl->st[in] = t;
+                if (done(t)) ctl->st[in] = t;
                 ctl->tail = t.e;
                 ctl->ticket = 0;
                 ctl->launches++;
@@ -440,7 +421,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_starts(const Level a, const uint
             if (last) {
                 const unsigned long long tail = atomicAdd(&ctl->tail, 0ull);
                 // in both: a first level without units is the end
-                ctl->st[0] = ctl->st[1] = State{from, (uint32_t)tail, (uint32_t)(tail >> 32), 1, 0};
+                ctl->st[0] = ctl->st[1] = first_level(from, (uint32_t)tail, (uint32_t)(tail >> 32), a.max_d);
                 ctl->tail = (uint32_t)tail;
             }
         }

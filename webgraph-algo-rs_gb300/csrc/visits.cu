@@ -136,7 +136,7 @@ static int visit_levels(hb_visit* v, const uint64_t* roots, size_t nroots, uint6
         VC(v, cudaEventRecord(v->ev1, s), "cudaEventRecord");
         VC(v, cudaMemcpyAsync(v->h_ctl, v->d_ctl, sizeof(hbl::Control), cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
         VC(v, cudaStreamSynchronize(s), "cudaStreamSynchronize");
-        if (hbl::done(v->h_ctl->st[0], a.max_d)) break;
+        if (hbl::done(v->h_ctl->st[0])) break;
     }
     const hbl::Control& c = *v->h_ctl;
     v->ahead = (int)std::max<uint32_t>(1, std::min<uint32_t>(c.launches, 64));

@@ -25,6 +25,7 @@ HEADERS = [
     os.path.join(CSRC, "visit_level.cuh"),
     os.path.join(CSRC, "visit_state.h"),
     os.path.join(CSRC, "launch_chain.cuh"),
+    os.path.join(CSRC, "once_per_device.h"),
     os.path.join(CSRC, "graph_gen.h"),
     os.path.join(REPO, "include", "hyperball_gb300.h"),
 ]

@@ -2534,9 +2534,9 @@ template <int LOG2M, bool FAR, int MINB, int PIPEX = 0>
 static int tile_launch(const UnionArgs& a, int grid, cudaStream_t s, bool chained) {
     constexpr int smem = far_bytes<LOG2M, FAR>();
     if constexpr (smem > 48 * 1024) {
-        static const cudaError_t attr = cudaFuncSetAttribute(
-            k_union_window<LOG2M, FAR, MINB, PIPEX>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (attr != cudaSuccess) return (int)attr;
+        static hbl::OncePerDevice once;
+        const cudaError_t e = hbl::allow_shared(once, k_union_window<LOG2M, FAR, MINB, PIPEX>, smem);
+        if (e != cudaSuccess) return launched(e);
     }
     ++t_launches;
     return launched(hbl::launch(chained, k_union_window<LOG2M, FAR, MINB, PIPEX>, grid, 256, smem, s, a));
@@ -2556,9 +2556,9 @@ static int staged_launch(const UnionArgs& a, int grid, cudaStream_t s, bool chai
     constexpr int smem = staged_smem_bytes<LOG2M>();
     constexpr int PIPE_L = pipe_depth<Geo<LOG2M>::NW>();
     if constexpr (smem > 48 * 1024) {
-        static const cudaError_t attr = cudaFuncSetAttribute(
-            k_union_staged<LOG2M, MINB, PIPE_L, IDS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (attr != cudaSuccess) return (int)attr;
+        static hbl::OncePerDevice once;
+        const cudaError_t e = hbl::allow_shared(once, k_union_staged<LOG2M, MINB, PIPE_L, IDS>, smem);
+        if (e != cudaSuccess) return launched(e);
     }
     ++t_launches;
     return launched(hbl::launch(chained, k_union_staged<LOG2M, MINB, PIPE_L, IDS>, grid, 256, smem, s, a));

@@ -1,6 +1,9 @@
-// Launches that are set up while the kernel in front of them still runs.
+// Launches that are set up while the kernel in front of them still runs, and
+// kernels with more than 48 KB of dynamic shared memory.
 #pragma once
 #include <cuda_runtime.h>
+
+#include "once_per_device.h"
 
 namespace hbl {
 
@@ -30,6 +33,18 @@ inline cudaError_t launch(bool chained, void (*kernel)(P...), int grid, int bloc
 template <class... P, class... A>
 inline cudaError_t chain(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
     return launch(true, kernel, grid, block, smem, s, args...);
+}
+
+// Lets `kernel` take `bytes` of dynamic shared memory on the current device (from
+// 48 KB on a device refuses the launch otherwise). `once` is the kernel's own.
+template <class... P>
+inline cudaError_t allow_shared(OncePerDevice& once, void (*kernel)(P...), size_t bytes) {
+    int device = -1;
+    const cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    return (cudaError_t)once(device, [&] {
+        return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    });
 }
 
 }  // namespace hbl

@@ -432,9 +432,8 @@ template <bool PRED>
 inline cudaError_t launch_starts(const Level& a, const uint32_t* starts, uint64_t count, uint32_t from, bool last, int sms,
                                  cudaStream_t s) {
     constexpr size_t smem = sizeof(Run<PRED>) * WARPS;
-    static const cudaError_t ok =
-        cudaFuncSetAttribute(k_starts<PRED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (ok != cudaSuccess) return ok;
+    static OncePerDevice once;
+    if (const cudaError_t e = allow_shared(once, k_starts<PRED>, smem); e != cudaSuccess) return e;
     const int grid = (int)std::min<uint64_t>((count + THREADS - 1) / THREADS, (uint64_t)sms);
     k_starts<PRED><<<grid, THREADS, smem, s>>>(a, starts, count, from, last);
     return cudaGetLastError();
@@ -448,9 +447,8 @@ inline cudaError_t launch_levels(const Level& a, int count, int& in, int sms, cu
     // whose bits would not fit it takes less
     constexpr size_t base = sizeof(Run<PRED>) * WARPS + sizeof(Local), most = base + BITS / 8;
     static_assert(most <= 227 * 1024 - 64, "one block per SM");
-    static const cudaError_t ok =
-        cudaFuncSetAttribute(k_level<COMP, PRED>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    if (ok != cudaSuccess) return ok;
+    static OncePerDevice once;
+    if (const cudaError_t e = allow_shared(once, k_level<COMP, PRED>, most); e != cudaSuccess) return e;
     const size_t smem = a.n <= BITS ? base + ((a.n + 31) / 32 * 4 + 15) / 16 * 16 : base;
     const int grid = a.small == TINY ? 1 : sms;  // TINY: every level is the first block's
     for (int k = 0; k < count; k++) {

@@ -41,3 +41,20 @@ def test_roots_in_pieces(hb, oracle):
     assert st["visited"] == n and st["levels"] == 2
     assert np.array_equal(np.sort(nodes[dists == 1]), np.arange(1, n, 2)) and np.all(preds[dists == 1] + 1 == nodes[dists == 1])
     v.close()
+
+
+def test_lean_arrays(hb):
+    """Without room for the rows and entries a visit holds no more than its graph and
+    24 bytes a node: offsets, queue, predecessors, units, tiles, bitmap and a piece of roots."""
+    g = hb.Graph.weblike(4_000_003, seed=1)
+    n, m = g.num_nodes, g.num_arcs
+
+    def make():
+        hb.debug_fail_allocations(0)
+        try:
+            return hb.ParFair(g)
+        finally:
+            hb.debug_fail_allocations(-1)
+
+    want = 4 * m + 20 * n + n // 8 + n // 2 + min(4 * n, 16 << 20)
+    assert _held(make) <= min(want + (8 << 20), 4 * m + 24 * n + n // 8 + (8 << 20))

@@ -355,6 +355,14 @@ struct hb_handle {
     std::string err;
 };
 
+// hb_debug_fail_allocations: the device allocation that brings this count to zero
+// fails (once); -1: none
+static std::atomic<long long> g_fail_alloc_after{-1};
+
+bool hbk::fail_allocation() {
+    return g_fail_alloc_after.load(std::memory_order_relaxed) >= 0 && g_fail_alloc_after.fetch_sub(1) == 0;
+}
+
 namespace {
 
 int set_err(hb_handle* h, int code, const std::string& msg) {
@@ -390,15 +398,10 @@ struct NvtxRange {
     ~NvtxRange() { nvtxRangePop(); }
 };
 
-// hb_debug_fail_allocations: the device allocation of a handle that brings
-// this count to zero fails (once); -1: none
-std::atomic<long long> g_fail_alloc_after{-1};
-
 template <class T>
 int dalloc(hb_handle* h, T** out, size_t count) {
     *out = nullptr;
-    if (g_fail_alloc_after.load(std::memory_order_relaxed) >= 0 &&
-        g_fail_alloc_after.fetch_sub(1) == 0)
+    if (hbk::fail_allocation())
         return set_err(h, HB_ERR_OOM, "device allocation failed (injected by hb_debug_fail_allocations)");
     size_t bytes = std::max<size_t>(count * sizeof(T), 256);
     void* p = nullptr;

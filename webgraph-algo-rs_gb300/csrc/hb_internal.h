@@ -21,6 +21,9 @@ int load_bvgraph(const std::string& basename, Csr& g, std::string& err, uint64_t
 // ---------------------------------------------------------------------------
 namespace hbk {
 
+// hb_debug_fail_allocations: counts a device allocation; true when it is the one to fail
+bool fail_allocation();
+
 constexpr int MAX_DISCOUNT = 8;
 // heavy nodes with more arcs than HEAVY_SPLIT run as equal segments of at most
 // HEAVY_SEG arcs, one CTA each (k_union_heavy)

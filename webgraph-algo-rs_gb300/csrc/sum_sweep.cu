@@ -98,14 +98,17 @@ __global__ void k_sw_begin(const hbl::Level a, uint64_t n, const Scratch* pick, 
     const uint64_t r = pick ? pick->pick.idx : root;
     for (uint64_t v = t0; v < n; v += stride) a.dist[v] = v == r ? 0u : INF;
     for (uint64_t w = t0; w < (n + 31) / 32; w += stride) a.visited[w] = w == r >> 5 ? 1u << (r & 31) : 0u;
-    if (r != ~0ull)  // the first level is the start's units
-        for (uint64_t t = t0; t * 32 * hbl::UNIT < a.info[r].deg; t += stride) a.tile[0][t] = 0;
+    uint64_t units = 0;  // the first level is the start's units
+    if (r != ~0ull) units = a.off ? (a.off[r + 1] - a.off[r] + (1ull << a.lg) - 1) >> a.lg
+                                  : ((uint64_t)a.info[r].deg + hbl::UNIT - 1) / hbl::UNIT;
+    for (uint64_t t = t0; t * 32 < units; t += stride) a.tile[0][t] = 0;
     if (t0 == 0) {
         hbl::State s{0, 0, 0, 1, 0};
         if (r != ~0ull) {
             s.e = 1;
-            a.entry[0] = a.info[r];
-            s.units = (a.entry[0].deg + hbl::UNIT - 1) / hbl::UNIT;
+            s.units = (uint32_t)units;
+            if (a.off) a.unit[0] = 0;
+            else a.entry[0] = a.info[r];
             a.queue[0] = (uint32_t)r;
         }
         // in both: of a start without arcs no launch has a level to expand, and
@@ -573,6 +576,8 @@ struct Sweeper {
     uint32_t *d_df = nullptr, *d_db = nullptr;
     u64 *d_fl = nullptr, *d_fh = nullptr, *d_bl = nullptr, *d_bh = nullptr, *d_ft = nullptr, *d_bt = nullptr;
     uint8_t* d_radial = nullptr;
+    hbl::Form form{false, hbl::UNIT_LG};
+    void* wide = nullptr;                 // the wide form's arrays:
     hbl::Entry *d_entry = nullptr, *d_info = nullptr, *d_tinfo = nullptr;
     uint32_t* d_tile[2] = {nullptr, nullptr};
     hbl::Control* d_ctl = nullptr;
@@ -603,7 +608,7 @@ struct Sweeper {
         cudaSetDevice(device);
         if (s) cudaStreamSynchronize(s);
         // a symmetric graph is its own transpose: each block once
-        std::vector<void*> ps = {d_off, d_toff, d_succ, d_tsucc, d_dist, d_queue, d_entry, d_info, d_tinfo, d_tile[0], d_tile[1], d_visited, d_comp,
+        std::vector<void*> ps = {d_off, d_toff, d_succ, d_tsucc, d_dist, d_queue, wide, d_tile[0], d_tile[1], d_visited, d_comp,
                                  d_df, d_db, d_fl, d_fh, d_bl, d_bh, d_ft, d_bt, d_radial, d_ctl, d_scr, d_bad,
                                  d_ecc_f, d_ecc_b, d_best_score, d_best_tot, d_pivot, d_ef,
                                  d_eb, d_cstart, d_cend, d_gather, d_gather64, d_best};
@@ -627,6 +632,9 @@ struct Sweeper {
     hbl::Level level_args(bool backward, bool in_comp) const {
         hbl::Level a{};
         a.info = backward ? d_tinfo : d_info;
+        a.off = form.lean ? backward ? d_toff : d_off : nullptr;
+        a.lg = form.lg;
+        a.unit = d_db;  // (lean) written between visits alone
         a.succ = backward ? d_tsucc : d_succ;
         a.comp = in_comp ? d_comp : nullptr;
         a.visited = d_visited;
@@ -637,9 +645,39 @@ struct Sweeper {
         a.tile[1] = d_tile[1];
         a.ctl = d_ctl;
         a.n = n;
-        a.small = hbl::small_units(n, m);
+        a.small = hbl::small_units(n, m, form.lg);
         a.max_d = hbs::INF;
         return a;
+    }
+
+    // The wide form's arrays, in one allocation: the entries, and every node's row
+    // forward and backward. The transpose's offsets stand where the entries come
+    // once its rows are known. Without room for them beside the program's other
+    // data the visits take the lean form (hbl::choose_form).
+    void alloc_rows(const u64* off, const u64* toff) {
+        const u64 entries = std::max<u64>(n * sizeof(hbl::Entry), (n + 1) * 8), rows = n * sizeof(hbl::Entry);
+        const u64 bytes = entries + (undirected ? 1 : 2) * rows;
+        const u64 more = bytes - (undirected ? 0 : (n + 1) * 8);
+        size_t free_bytes = 0, all = 0;
+        if (more > hbl::WIDE_BYTES) ck(cudaMemGetInfo(&free_bytes, &all), "cudaMemGetInfo");
+        const u64 longest = std::max(hbl::longest_row(off, n, m), undirected ? 0 : hbl::longest_row(toff, n, m));
+        form = hbl::choose_form(n, m, longest, more, free_bytes);
+        if (!form.lean) {
+            const cudaError_t e = hbk::fail_allocation() ? cudaErrorMemoryAllocation : cudaMalloc(&wide, bytes);
+            if (e == cudaErrorMemoryAllocation) {
+                cudaGetLastError();
+                wide = nullptr;
+                form = hbl::choose_form(n, m, UINT64_MAX, 0, 0);
+            } else {
+                ck(e, "cudaMalloc");
+                char* p = static_cast<char*>(wide);
+                d_entry = reinterpret_cast<hbl::Entry*>(p);
+                d_info = reinterpret_cast<hbl::Entry*>(p + entries);
+                d_tinfo = undirected ? d_info : d_info + n;
+            }
+        }
+        if (undirected) d_toff = d_off;
+        else if (form.lean) alloc(&d_toff, n + 1);
     }
 
     // `count` more level launches of a visit (in: the parity of the next)
@@ -1087,29 +1125,26 @@ int run(const hb_graph_view* g, const hb_graph_view* t, int level, const uint8_t
     // the graph on the device first: the components use its visits
     w.alloc(&w.d_off, n + 1);
     w.alloc(&w.d_succ, m);
-    if (t) {
-        w.alloc(&w.d_toff, n + 1);
-        w.alloc(&w.d_tsucc, m);
-    } else {
-        w.d_toff = w.d_off;
-        w.d_tsucc = w.d_succ;
-    }
+    if (t) w.alloc(&w.d_tsucc, m);
+    else w.d_tsucc = w.d_succ;
     for (uint32_t** p : {&w.d_dist, &w.d_queue, &w.d_comp, &w.d_df, &w.d_db}) w.alloc(p, n);
     w.alloc(&w.d_visited, (n + 31) / 32);
-    w.alloc(&w.d_entry, n);
-    for (uint32_t** p : {&w.d_tile[0], &w.d_tile[1]}) w.alloc(p, hbl::tiles(n, m));
     for (u64** p : {&w.d_fl, &w.d_fh, &w.d_bl, &w.d_bh, &w.d_ft, &w.d_bt}) w.alloc(p, n);
     w.alloc(&w.d_radial, n);
     w.alloc(&w.d_ctl, 1);
     w.alloc(&w.d_scr, 1);
     w.alloc(&w.d_bad, 1);
     w.alloc(&w.d_best, (u64)w.grid);
+    // the rest of the state, and what the components and the levels need
+    w.alloc_rows(g->offsets, t ? t->offsets : nullptr);
+    for (uint32_t** p : {&w.d_tile[0], &w.d_tile[1]}) w.alloc(p, hbl::tiles(n, m, w.form.lg));
+    u64* d_toff = w.form.lean ? w.d_toff : reinterpret_cast<u64*>(w.d_entry);
     ck(cudaMallocHost((void**)&w.h_res, sizeof(hbs::Result) + sizeof(hbl::Control)), "cudaMallocHost");
     cudaStream_t s = w.s;
     ck(cudaMemcpyAsync(w.d_off, g->offsets, (n + 1) * 8, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
     if (m) ck(cudaMemcpyAsync(w.d_succ, g->successors, m * 4, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
     if (t) {
-        ck(cudaMemcpyAsync(w.d_toff, t->offsets, (n + 1) * 8, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
+        ck(cudaMemcpyAsync(d_toff, t->offsets, (n + 1) * 8, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
         if (m) ck(cudaMemcpyAsync(w.d_tsucc, t->successors, m * 4, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
     }
     // the CSR is checked before any kernel indexes with it
@@ -1120,21 +1155,17 @@ int run(const hb_graph_view* g, const hb_graph_view* t, int level, const uint8_t
         ck(cudaMemsetAsync(w.d_scr, 0, sizeof *w.d_scr, s), "cudaMemsetAsync");
         ck(cudaMemsetAsync(&w.d_scr->key, 0xff, 8, s), "cudaMemsetAsync");
         hbs::k_sw_validate<<<w.blocks(std::max(n, m)), hbs::SW_THREADS, 0, s>>>(w.d_off, w.d_succ, n, m, d_bad);
-        if (t) hbs::k_sw_validate<<<w.blocks(std::max(n, m)), hbs::SW_THREADS, 0, s>>>(w.d_toff, w.d_tsucc, n, m, d_bad);
+        if (t) hbs::k_sw_validate<<<w.blocks(std::max(n, m)), hbs::SW_THREADS, 0, s>>>(d_toff, w.d_tsucc, n, m, d_bad);
         ck(cudaGetLastError(), "k_sw_validate");
         ck(cudaMemcpyAsync(&bad, d_bad, 4, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
         w.sync();
         if (bad) fail(HB_ERR_INVALID, "graph has decreasing offsets or successors >= num_nodes");
     }
-    w.alloc(&w.d_info, n);
-    hbl::k_info<<<w.blocks(n), hbs::SW_THREADS, 0, s>>>(w.d_off, n, w.d_info);
-    if (t) {
-        w.alloc(&w.d_tinfo, n);
-        hbl::k_info<<<w.blocks(n), hbs::SW_THREADS, 0, s>>>(w.d_toff, n, w.d_tinfo);
-    } else {
-        w.d_tinfo = w.d_info;
+    if (!w.form.lean) {
+        hbl::k_info<<<w.blocks(n), hbs::SW_THREADS, 0, s>>>(w.d_off, n, w.d_info);
+        if (t) hbl::k_info<<<w.blocks(n), hbs::SW_THREADS, 0, s>>>(d_toff, n, w.d_tinfo);
+        ck(cudaGetLastError(), "k_info");
     }
-    ck(cudaGetLastError(), "k_info");
     mark("device graph");
     // components and the arcs between them
     if (w.undirected) w.comp = w.symmetric_components(hg);

@@ -25,7 +25,7 @@
 // changes under it; an ended visit's state is left in both.
 //
 // Measured: the visit of a web-like graph of 4e6 nodes (42 M arcs) from one node
-// takes 0.47 ms of kernels, where a warp per frontier node, a block per node
+// takes 0.41 ms of kernels (0.54 in the lean form, see visit_state.h), where a warp per frontier node, a block per node
 // above 4096 arcs and a host round trip per level took 2.6 ms. What bounds its two widest
 // levels (160 and 121 us of it) is the SM's load unit, at one lane a cycle for
 // scattered words: a test an arc, and a claim, an entry and a distance a node.
@@ -35,13 +35,13 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <type_traits>
 
 #include "launch_chain.cuh"
 #include "visit_state.h"
 
 namespace hbl {
 
-constexpr uint32_t UNIT = 8;
 constexpr int THREADS = 1024, WARPS = THREADS / 32;
 constexpr int MAX_SMALL = 1024;  // small levels of one launch
 // a warp queues its claimed nodes GROUP at a time, and when it holds as many; it
@@ -72,34 +72,42 @@ struct Control {
 };
 
 struct Level {
-    const Entry* info;     // every node's arcs (k_info)
+    const Entry* info;     // every node's arcs (k_info), or, in the lean form,
+    const uint64_t* off;   // the offsets
     const uint32_t* succ;
     const uint32_t* comp;  // a visit stays inside its start nodes' components (COMP)
     uint32_t* visited;     // bitmap
     uint32_t* dist;        // distance and
     uint32_t* pred;        // predecessor (PRED) of every node visited, or null
     uint32_t* queue;       // visited nodes in visit order,
-    Entry* entry;          // their entries,
+    Entry* entry;          // their entries, or, in the lean form,
+    uint32_t* unit;        // the units before them in their level (see end_of_level),
     uint32_t* tile[2];     // a level's slots by units / 32, and the next level's (tiles() words each)
     uint32_t* qpred;       // their predecessors and
-    uint32_t* qdist;       // their distances (PRED)
+    uint32_t* qdist;       // their distances (PRED; not in the lean form)
     Control* ctl;
     uint64_t n;
+    uint32_t lg;           // a unit's arcs (lean; else UNIT_LG)
     uint32_t max_d;        // nodes farther away are not visited
     uint32_t small;        // units of a level that the first block takes alone
 };
 
-// units of a graph, and the tiles of its largest possible level
-inline uint64_t units(uint64_t n, uint64_t m) { return m / UNIT + n; }
-inline uint64_t tiles(uint64_t n, uint64_t m) { return units(n, m) / 32 + 1; }
-inline uint32_t small_units(uint64_t n, uint64_t m) {
-    return units(n, m) <= TINY ? TINY : n <= BITS ? SMALL : SMALL_GLOBAL;
+inline uint32_t small_units(uint64_t n, uint64_t m, uint32_t lg) {
+    if (units(n, m, UNIT_LG) <= TINY) return TINY;
+    return std::max<uint32_t>((n <= BITS ? SMALL : SMALL_GLOBAL) >> std::min(lg - UNIT_LG, 31u), 1);
 }
 
+// what the queue keeps beside a node
+template <bool LEAN>
+using Slot = std::conditional_t<LEAN, uint32_t, Entry>;
+__device__ __forceinline__ uint32_t unit_of(const Entry& e) { return e.unit; }
+__device__ __forceinline__ uint32_t unit_of(uint32_t u) { return u; }
+
 // The entries and tiles of a level and of the next, in a block that goes on alone.
+template <bool LEAN>
 struct Local {
     uint32_t tile[2][SMALL / 32];
-    Entry entry[2][CAP];
+    Slot<LEAN> entry[2][CAP];
     uint32_t node[2][CAP];
 };
 
@@ -127,23 +135,28 @@ __device__ __forceinline__ bool claim(uint32_t* bits, uint32_t s) {
 // Queues nodes [from, fill) of the warp's run, at most GROUP of them, as nodes
 // at distance d (every lane). With `next`, the first CAP entries from slot
 // `first` on also go to next->entry[side].
-template <bool PRED>
+template <bool PRED, bool LEAN>
 __device__ __forceinline__ void put_group(const Level& a, unsigned long long* tail, const Run<PRED>& run, int from, int fill,
-                                          uint32_t d, Local* next, int side, uint32_t first, uint32_t* tile) {
+                                          uint32_t d, Local<LEAN>* next, int side, uint32_t first, uint32_t* tile) {
     constexpr int G = GROUP / 32;
     const int lane = threadIdx.x & 31;
-    uint32_t v[G], units = 0;
+    uint32_t v[G], own[G], units = 0;
     Entry en[G];
 #pragma unroll
     for (int i = 0; i < G; i++) {
         const int k = from + i * 32 + lane;
         v[i] = k < fill ? run.node[k] : 0u;
         en[i] = Entry{0, 0, 0};
-        if (k < fill) en[i] = load_entry(a.info + v[i]);
+        if constexpr (LEAN) {
+            own[i] = k < fill ? (uint32_t)((__ldg(a.off + v[i] + 1) - __ldg(a.off + v[i]) + (1ull << a.lg) - 1) >> a.lg) : 0u;
+        } else {
+            if (k < fill) en[i] = load_entry(a.info + v[i]);
+            own[i] = (en[i].deg + UNIT - 1) / UNIT;
+        }
     }
 #pragma unroll
     for (int i = 0; i < G; i++) {
-        const uint32_t u = (en[i].deg + UNIT - 1) / UNIT;
+        const uint32_t u = own[i];
         uint32_t x = u;  // inclusive scan
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -163,18 +176,21 @@ __device__ __forceinline__ void put_group(const Level& a, unsigned long long* ta
         uint32_t t0 = 0, t1 = 0;  // the tiles that start in the node's units
         if (k < fill) {
             en[i].unit += (uint32_t)(at >> 32);
-            t0 = (en[i].unit + 31) / 32;
-            t1 = (en[i].unit + (en[i].deg + UNIT - 1) / UNIT + 31) / 32;
+            using Sum = std::conditional_t<LEAN, uint64_t, uint32_t>;
+            t0 = (uint32_t)(((Sum)en[i].unit + 31) / 32);
+            t1 = (uint32_t)(((Sum)en[i].unit + own[i] + 31) / 32);
+            Slot<LEAN> kept;
+            if constexpr (LEAN) a.unit[slot] = kept = en[i].unit;
+            else a.entry[slot] = kept = en[i];
             a.queue[slot] = v[i];
-            a.entry[slot] = en[i];
             if (next && slot - first < CAP) {
-                next->entry[side][slot - first] = en[i];
+                next->entry[side][slot - first] = kept;
                 next->node[side][slot - first] = v[i];
             }
             if (a.dist) a.dist[v[i]] = d;
             if constexpr (PRED) {
                 a.qpred[slot] = run.pred[k];
-                a.qdist[slot] = d;
+                if constexpr (!LEAN) a.qdist[slot] = d;
                 if (a.pred) a.pred[v[i]] = run.pred[k];
             }
             if (t1 == t0 + 1) {
@@ -195,13 +211,13 @@ __device__ __forceinline__ void put_group(const Level& a, unsigned long long* ta
 }
 
 // Queues the warp's run down to fewer than GROUP nodes, or all of it.
-template <bool PRED>
+template <bool PRED, bool LEAN>
 __device__ __forceinline__ void flush(const Level& a, unsigned long long* tail, const Run<PRED>& run, int& fill, bool all,
-                                      uint32_t d, Local* next, int side, uint32_t first, uint32_t* tile) {
+                                      uint32_t d, Local<LEAN>* next, int side, uint32_t first, uint32_t* tile) {
     __syncwarp();
     while (fill >= GROUP || (all && fill > 0)) {
         const int from = max(fill - GROUP, 0);
-        put_group<PRED>(a, tail, run, from, fill, d, next, side, first, tile);
+        put_group<PRED, LEAN>(a, tail, run, from, fill, d, next, side, first, tile);
         fill = from;
     }
     __syncwarp();
@@ -210,101 +226,132 @@ __device__ __forceinline__ void flush(const Level& a, unsigned long long* tail, 
 // Warp w of nw: its share of the level s, whose entries come from the queue
 // or, with `local`, from loc->entry[side ^ 1]; what it claims goes to the queue and,
 // with loc, to loc->entry[side].
-template <bool COMP, bool PRED>
+template <bool COMP, bool PRED, bool LEAN>
 __device__ __forceinline__ void expand(const Level& a, const State& s, unsigned long long* tail, uint32_t w,
-                                       uint32_t nw, Run<PRED>& run, unsigned long long& known, uint32_t* bits, Local* loc,
-                                       int side, bool local) {
+                                       uint32_t nw, Run<PRED>& run, unsigned long long& known, uint32_t* bits,
+                                       Local<LEAN>* loc, int side, bool local) {
+    using Sum = std::conditional_t<LEAN, uint64_t, uint32_t>;  // of units
     const int lane = threadIdx.x & 31;
-    const uint32_t ntiles = (s.units + 31) / 32, per = (ntiles + nw - 1) / nw;
+    const uint32_t lg = LEAN ? a.lg : UNIT_LG;
+    const Sum ntiles = ((Sum)s.units + 31) / 32, per = (ntiles + nw - 1) / nw;
     if ((uint64_t)w * per >= ntiles) return;
-    uint32_t u = w * per * 32;
-    const uint32_t u1 = min(u + per * 32, s.units);
-    const Entry* entry = local ? loc->entry[side ^ 1] - s.b : a.entry;
+    Sum u = w * per * 32;
+    const Sum u1 = min(u + per * 32, (Sum)s.units);
+    const Slot<LEAN>* entry;
+    if constexpr (LEAN) entry = a.unit;
+    else entry = a.entry;
+    if (local) entry = loc->entry[side ^ 1] - s.b;
     const uint32_t* queue = local ? loc->node[side ^ 1] - s.b : a.queue;
     int fill = 0;
     for (uint32_t base = (local ? loc->tile[side ^ 1] : a.tile[(s.d & 1) ^ 1])[u / 32]; u < u1; base += 32) {
         // 32 slots at a time, one per lane
         const uint32_t slot = base + lane;
-        uint32_t qu = 0xffffffffu, v = 0, deg = 0, cv = 0;
+        uint32_t v = 0, cv = 0;
+        Sum qu = ~(Sum)0;
+        std::conditional_t<LEAN, uint64_t, uint32_t> deg = 0;
         uint64_t o = 0;
         if (slot < s.e) {
-            const Entry en = entry[slot];
-            qu = en.unit;
-            o = en.off;
-            deg = en.deg;
-            if constexpr (PRED || COMP) v = queue[slot];
+            const Slot<LEAN> en = entry[slot];
+            qu = unit_of(en);
+            if constexpr (PRED || COMP || LEAN) v = queue[slot];
+            if constexpr (LEAN) {
+                o = __ldg(a.off + v);
+                deg = __ldg(a.off + v + 1) - o;
+            } else {
+                o = en.off;
+                deg = en.deg;
+            }
             if constexpr (COMP) cv = __ldg(a.comp + v);
         }
-        const uint32_t lim = s.e - base > 32 ? min(u1, entry[base + 32].unit) : u1;
-        for (; u < lim; u += min(32u, lim - u)) {
+        const Sum lim = s.e - base > 32 ? min(u1, (Sum)unit_of(entry[base + 32])) : u1;
+        for (; u < lim; u += min((Sum)32, lim - u)) {
             // lane l: unit u + l, in the last of the slots that starts at or before it
-            const uint32_t x = u + lane;
+            const Sum x = u + lane;
             int idx = 0;
 #pragma unroll
             for (int st = 16; st > 0; st >>= 1)
                 if (__shfl_sync(0xffffffffu, qu, idx + st) <= x) idx += st;
-            const uint32_t skip = (x - __shfl_sync(0xffffffffu, qu, idx)) * UNIT;
-            const uint64_t first = __shfl_sync(0xffffffffu, o, idx) + skip;
-            const uint32_t rest = __shfl_sync(0xffffffffu, deg, idx) - skip;
-            const uint32_t len = x < lim ? min(rest, UNIT) : 0u;
-            run.unit[lane] = make_ulonglong2(first, COMP ? len | ((uint64_t)__shfl_sync(0xffffffffu, cv, idx) << 32) : len);
+            const auto skip = (x - __shfl_sync(0xffffffffu, qu, idx)) << lg;
+            uint64_t first = __shfl_sync(0xffffffffu, o, idx) + skip;
+            const auto rest = __shfl_sync(0xffffffffu, deg, idx) - skip;
+            uint64_t left = x < lim ? min(rest, (Sum)1 << lg) : (Sum)0;
+            const uint32_t c0 = COMP ? __shfl_sync(0xffffffffu, cv, idx) : 0u;
             if constexpr (PRED) run.unit_pred[lane] = __shfl_sync(0xffffffffu, v, idx);
-            __syncwarp();
-            uint32_t src[UNIT], cw[COMP ? UNIT : 1];
-            uint32_t have = 0, hit = 0;
+            // UNIT arcs of each of the 32 units at a time (the lean form's may be longer)
+            for (bool more = true; more;) {
+                const uint32_t len = LEAN ? (uint32_t)min(left, (uint64_t)UNIT) : (uint32_t)left;
+                run.unit[lane] = make_ulonglong2(first, COMP ? len | ((uint64_t)c0 << 32) : len);
+                __syncwarp();
+                uint32_t src[UNIT], cw[COMP ? UNIT : 1];
+                uint32_t have = 0, hit = 0;
 #pragma unroll
-            for (int j = 0; j < (int)UNIT; j++) {
-                const ulonglong2 un = run.unit[j * 4 + (lane >> 3)];  // eight lanes per unit
-                src[j] = 0;
-                if constexpr (COMP) cw[j] = (uint32_t)(un.y >> 32);
-                if ((lane & 7u) < (uint32_t)un.y) {
-                    src[j] = __ldg(a.succ + un.x + (lane & 7));
-                    have |= 1u << j;
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < (int)UNIT; j++) {
-                bool c = ((have >> j) & 1u) && !visited(bits, src[j]);
-                if constexpr (COMP) c = c && __ldg(a.comp + src[j]) == cw[j];
-                hit |= (uint32_t)c << j;
-            }
-            if (hit) {
-#pragma unroll
-                for (int j = 0; j < (int)UNIT; j++)
-                    if (((hit >> j) & 1u) && !claim(bits, src[j])) hit &= ~(1u << j);
-            }
-            if constexpr (PRED) known += __popc(have & ~hit);
-            if (__any_sync(0xffffffffu, hit != 0u)) {
-#pragma unroll
-                for (int half = 0; half < 2; half++) {
-                    // the lanes' claimed nodes, one lane after the other, into the run
-                    constexpr int H = UNIT / 2;
-                    const uint32_t mine = __popc((hit >> (half * H)) & ((1u << H) - 1u));
-                    uint32_t y = mine;
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const uint32_t z = __shfl_up_sync(0xffffffffu, y, o);
-                        if (lane >= o) y += z;
+                for (int j = 0; j < (int)UNIT; j++) {
+                    const ulonglong2 un = run.unit[j * 4 + (lane >> 3)];  // eight lanes per unit
+                    src[j] = 0;
+                    if constexpr (COMP) cw[j] = (uint32_t)(un.y >> 32);
+                    if ((lane & 7u) < (uint32_t)un.y) {
+                        src[j] = __ldg(a.succ + un.x + (lane & 7));
+                        have |= 1u << j;
                     }
-                    uint32_t at = fill + y - mine;
+                }
 #pragma unroll
-                    for (int j = half * H; j < half * H + H; j++)
-                        if ((hit >> j) & 1u) {
-                            run.node[at] = src[j];
-                            if constexpr (PRED) run.pred[at] = run.unit_pred[j * 4 + (lane >> 3)];
-                            at++;
+                for (int j = 0; j < (int)UNIT; j++) {
+                    bool c = ((have >> j) & 1u) && !visited(bits, src[j]);
+                    if constexpr (COMP) c = c && __ldg(a.comp + src[j]) == cw[j];
+                    hit |= (uint32_t)c << j;
+                }
+                if (hit) {
+#pragma unroll
+                    for (int j = 0; j < (int)UNIT; j++)
+                        if (((hit >> j) & 1u) && !claim(bits, src[j])) hit &= ~(1u << j);
+                }
+                if constexpr (PRED) known += __popc(have & ~hit);
+                if (__any_sync(0xffffffffu, hit != 0u)) {
+#pragma unroll
+                    for (int half = 0; half < 2; half++) {
+                        // the lanes' claimed nodes, one lane after the other, into the run
+                        constexpr int H = UNIT / 2;
+                        const uint32_t mine = __popc((hit >> (half * H)) & ((1u << H) - 1u));
+                        uint32_t y = mine;
+#pragma unroll
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const uint32_t z = __shfl_up_sync(0xffffffffu, y, o);
+                            if (lane >= o) y += z;
                         }
-                    fill += __shfl_sync(0xffffffffu, y, 31);
-                    flush<PRED>(a, tail, run, fill, false, s.d, loc, side, s.e, a.tile[s.d & 1]);
+                        uint32_t at = fill + y - mine;
+#pragma unroll
+                        for (int j = half * H; j < half * H + H; j++)
+                            if ((hit >> j) & 1u) {
+                                run.node[at] = src[j];
+                                if constexpr (PRED) run.pred[at] = run.unit_pred[j * 4 + (lane >> 3)];
+                                at++;
+                            }
+                        fill += __shfl_sync(0xffffffffu, y, 31);
+                        flush<PRED, LEAN>(a, tail, run, fill, false, s.d, loc, side, s.e, a.tile[s.d & 1]);
+                    }
+                }
+                __syncwarp();
+                more = false;
+                if constexpr (LEAN) {
+                    first += len;
+                    left -= len;
+                    more = __any_sync(0xffffffffu, left != 0);
                 }
             }
-            __syncwarp();
         }
     }
-    flush<PRED>(a, tail, run, fill, true, s.d, loc, side, s.e, a.tile[s.d & 1]);
+    flush<PRED, LEAN>(a, tail, run, fill, true, s.d, loc, side, s.e, a.tile[s.d & 1]);
 }
 
-template <bool COMP, bool PRED>
+// In the lean form an expanded level leaves its end where its first slot's units
+// (none) stood, so that the host can tell the levels of a visit's events apart: a
+// zero there is the last level's.
+template <bool PRED, bool LEAN>
+__device__ __forceinline__ void end_of_level(const Level& a, const State& s) {
+    if constexpr (PRED && LEAN) a.unit[s.b] = s.e;
+}
+
+template <bool COMP, bool PRED, bool LEAN>
 __global__ void __launch_bounds__(THREADS, 1) k_level(const Level a, int in) {
     extern __shared__ __align__(16) uint8_t smem[];
     Run<PRED>& run = reinterpret_cast<Run<PRED>*>(smem)[threadIdx.x >> 5];
@@ -316,7 +363,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_level(const Level a, int in) {
     if (done(s) || (small && blockIdx.x != 0)) return;
     unsigned long long known = 0;
     if (small) {
-        Local* loc = reinterpret_cast<Local*>(smem + sizeof(Run<PRED>) * WARPS);
+        Local<LEAN>* loc = reinterpret_cast<Local<LEAN>*>(smem + sizeof(Run<PRED>) * WARPS);
         uint32_t* bits = a.visited;
         const uint32_t words = (uint32_t)((a.n + 31) / 32);
         const bool mine = a.n <= BITS;
@@ -328,7 +375,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_level(const Level a, int in) {
         auto fits = [&] { return s.e - s.b <= CAP && s.units <= SMALL; };
         if (fits()) {
             for (uint32_t i = threadIdx.x; i < s.e - s.b; i += THREADS) {
-                loc->entry[0][i] = a.entry[s.b + i];
+                if constexpr (LEAN) loc->entry[0][i] = a.unit[s.b + i];
+                else loc->entry[0][i] = a.entry[s.b + i];
                 loc->node[0][i] = a.queue[s.b + i];
             }
             for (uint32_t i = threadIdx.x; i * 32 < s.units; i += THREADS)
@@ -338,10 +386,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_level(const Level a, int in) {
         __syncthreads();
         int left = MAX_SMALL;
         do {
-            expand<COMP, PRED>(a, s, &s_tail, threadIdx.x >> 5, WARPS, run, known, bits, loc, side, fits());
+            expand<COMP, PRED, LEAN>(a, s, &s_tail, threadIdx.x >> 5, WARPS, run, known, bits, loc, side, fits());
             __syncthreads();
             const unsigned long long t = s_tail;
             __syncthreads();
+            if (threadIdx.x == 0) end_of_level<PRED, LEAN>(a, s);
             s = advance(s, t, a.max_d);
             if (threadIdx.x == 0) s_tail = s.e;  // read again behind the barriers of the next level
             side ^= 1;
@@ -358,13 +407,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_level(const Level a, int in) {
             ctl->launches++;
         }
     } else {
-        expand<COMP, PRED>(a, s, &ctl->tail, blockIdx.x * WARPS + (threadIdx.x >> 5), gridDim.x * WARPS, run, known,
-                           a.visited, nullptr, 0, false);
+        expand<COMP, PRED, LEAN>(a, s, &ctl->tail, blockIdx.x * WARPS + (threadIdx.x >> 5), gridDim.x * WARPS, run, known,
+                                 a.visited, nullptr, 0, false);
         __syncthreads();
         if (threadIdx.x == 0) {
             __threadfence();
             if (atomicAdd(&ctl->ticket, 1u) == gridDim.x - 1) {
                 // the last block: the queue is complete
+                end_of_level<PRED, LEAN>(a, s);
                 const State t = advance(s, atomicAdd(&ctl->tail, 0ull), a.max_d);
                 ctl->st[in ^ 1] = t;
                 if (done(t)) ctl->st[in] = t;
@@ -390,7 +440,7 @@ static __global__ void k_info(const uint64_t* __restrict__ off, uint64_t n, Entr
 // The start nodes not yet visited, at distance 0: the first level of a visit,
 // in st[0] and st[1]. They are queued from slot `from` on, where ctl->tail stood before
 // the first of the launches that bring them; `last` marks the last one.
-template <bool PRED>
+template <bool PRED, bool LEAN>
 __global__ void __launch_bounds__(THREADS, 1) k_starts(const Level a, const uint32_t* __restrict__ starts, uint64_t count,
                                                        uint32_t from, bool last) {
     extern __shared__ __align__(16) uint8_t smem[];
@@ -409,9 +459,9 @@ __global__ void __launch_bounds__(THREADS, 1) k_starts(const Level a, const uint
             if constexpr (PRED) run.pred[k] = r;
         }
         fill += __popc(mask);
-        flush<PRED>(a, &ctl->tail, run, fill, false, 0, nullptr, 0, 0, a.tile[0]);
+        flush<PRED, LEAN>(a, &ctl->tail, run, fill, false, 0, nullptr, 0, 0, a.tile[0]);
     }
-    flush<PRED>(a, &ctl->tail, run, fill, true, 0, nullptr, 0, 0, a.tile[0]);
+    flush<PRED, LEAN>(a, &ctl->tail, run, fill, true, 0, nullptr, 0, 0, a.tile[0]);
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
@@ -428,35 +478,48 @@ __global__ void __launch_bounds__(THREADS, 1) k_starts(const Level a, const uint
     }
 }
 
+template <bool PRED, bool LEAN>
+inline cudaError_t launch_starts_as(const Level& a, const uint32_t* starts, uint64_t count, uint32_t from, bool last,
+                                    int sms, cudaStream_t s) {
+    constexpr size_t smem = sizeof(Run<PRED>) * WARPS;
+    static OncePerDevice once;
+    if (const cudaError_t e = allow_shared(once, k_starts<PRED, LEAN>, smem); e != cudaSuccess) return e;
+    const int grid = (int)std::min<uint64_t>((count + THREADS - 1) / THREADS, (uint64_t)sms);
+    k_starts<PRED, LEAN><<<grid, THREADS, smem, s>>>(a, starts, count, from, last);
+    return cudaGetLastError();
+}
+
 template <bool PRED>
 inline cudaError_t launch_starts(const Level& a, const uint32_t* starts, uint64_t count, uint32_t from, bool last, int sms,
                                  cudaStream_t s) {
-    constexpr size_t smem = sizeof(Run<PRED>) * WARPS;
+    return a.off ? launch_starts_as<PRED, true>(a, starts, count, from, last, sms, s)
+                 : launch_starts_as<PRED, false>(a, starts, count, from, last, sms, s);
+}
+
+template <bool COMP, bool PRED, bool LEAN>
+inline cudaError_t launch_levels_as(const Level& a, int count, int& in, int sms, cudaStream_t s) {
+    // shared memory comes out of L1, which answers a wide level's tests: a graph
+    // whose bits would not fit it takes less
+    constexpr size_t base = sizeof(Run<PRED>) * WARPS + sizeof(Local<LEAN>), most = base + BITS / 8;
+    static_assert(most <= 227 * 1024 - 64, "one block per SM");
     static OncePerDevice once;
-    if (const cudaError_t e = allow_shared(once, k_starts<PRED>, smem); e != cudaSuccess) return e;
-    const int grid = (int)std::min<uint64_t>((count + THREADS - 1) / THREADS, (uint64_t)sms);
-    k_starts<PRED><<<grid, THREADS, smem, s>>>(a, starts, count, from, last);
-    return cudaGetLastError();
+    if (const cudaError_t e = allow_shared(once, k_level<COMP, PRED, LEAN>, most); e != cudaSuccess) return e;
+    const size_t smem = a.n <= BITS ? base + ((a.n + 31) / 32 * 4 + 15) / 16 * 16 : base;
+    const int grid = a.small == TINY ? 1 : sms;  // TINY: every level is the first block's
+    for (int k = 0; k < count; k++) {
+        const cudaError_t e = chain(k_level<COMP, PRED, LEAN>, grid, THREADS, smem, s, a, in);
+        if (e != cudaSuccess) return e;
+        in ^= 1;
+    }
+    return cudaSuccess;
 }
 
 // `count` launches of level kernels, of which the first reads st[in]; one past
 // the last level does nothing (and costs about 1.4 us)
 template <bool COMP, bool PRED>
 inline cudaError_t launch_levels(const Level& a, int count, int& in, int sms, cudaStream_t s) {
-    // shared memory comes out of L1, which answers a wide level's tests: a graph
-    // whose bits would not fit it takes less
-    constexpr size_t base = sizeof(Run<PRED>) * WARPS + sizeof(Local), most = base + BITS / 8;
-    static_assert(most <= 227 * 1024 - 64, "one block per SM");
-    static OncePerDevice once;
-    if (const cudaError_t e = allow_shared(once, k_level<COMP, PRED>, most); e != cudaSuccess) return e;
-    const size_t smem = a.n <= BITS ? base + ((a.n + 31) / 32 * 4 + 15) / 16 * 16 : base;
-    const int grid = a.small == TINY ? 1 : sms;  // TINY: every level is the first block's
-    for (int k = 0; k < count; k++) {
-        const cudaError_t e = chain(k_level<COMP, PRED>, grid, THREADS, smem, s, a, in);
-        if (e != cudaSuccess) return e;
-        in ^= 1;
-    }
-    return cudaSuccess;
+    return a.off ? launch_levels_as<COMP, PRED, true>(a, count, in, sms, s)
+                 : launch_levels_as<COMP, PRED, false>(a, count, in, sms, s);
 }
 
 }  // namespace hbl

@@ -47,14 +47,17 @@ struct hb_visit {
     bool own_stream = false;
     uint64_t n = 0, m = 0;
     void* block = nullptr;         // holds the arrays below
+    hbl::Form form{false, hbl::UNIT_LG};
+    uint64_t* d_off = nullptr;     // (wide form: only while the handle is made)
     uint32_t* d_succ = nullptr;
+    hbl::Entry* d_info = nullptr;  // (wide form)
     uint32_t* d_visited = nullptr;
     uint32_t* d_queue = nullptr;   // every node visited since the last reset, in visit order,
-    hbl::Entry* d_info = nullptr;
-    hbl::Entry* d_entry = nullptr; // its entry in its level,
+    hbl::Entry* d_entry = nullptr; // its entry in its level (wide form)
+    uint32_t* d_unit = nullptr;    // or the units before it there (lean form),
     uint32_t* d_tile[2] = {nullptr, nullptr};
     uint32_t* d_qpred = nullptr;   // its predecessor
-    uint32_t* d_qdist = nullptr;   // and distance
+    uint32_t* d_qdist = nullptr;   // and distance (wide form; lean: hbl::end_of_level)
     uint32_t* d_dist = nullptr;    // hb_visit_each: distance and predecessor by node (allocated there)
     uint32_t* d_pred = nullptr;
     uint32_t* d_roots = nullptr;   // a piece of the roots of the current visit
@@ -96,40 +99,56 @@ static int visit_cuda(hb_visit* v, cudaError_t e, const char* what) {
 // copy takes ten times the wait between two pieces).
 static uint64_t root_piece(uint64_t n) { return std::max<uint64_t>(std::min<uint64_t>(n, 1u << 22), 1); }
 
-// The arrays of a visit on graph v->n, v->m, all in one allocation: a handle of
-// 3e5 nodes takes 0.40 ms to make and 0.26 to free, with an allocation for each
-// array 0.66 and 0.50 (4e6 nodes: 1.5 and 0.40 instead of 1.8 and 0.79). *off gets the place where the offsets go until k_info has
-// read them; the entries come over them.
-static cudaError_t visit_alloc(hb_visit* v, uint64_t** off) {
-    const uint64_t n = v->n, m = v->m;
+// The arrays of a visit, all in one allocation: a handle of 3e5 nodes takes 0.40
+// ms to make and 0.26 to free, with an allocation for each array 0.66 and 0.50
+// (4e6 nodes: 1.5 and 0.40 instead of 1.8 and 0.79). Places them from `base` on
+// (null: nowhere yet) and returns their bytes. In the wide form the offsets stand
+// where the entries come once k_info has read them.
+static size_t visit_layout(hb_visit* v, const hbl::Form& f, char* base) {
+    const uint64_t n = v->n, m = v->m, rows = (n + 1) * 8;
     size_t total = 0;
-    auto need = [&](uint64_t bytes) {
-        const size_t at = total;
+    auto place = [&](auto** p, uint64_t bytes) {
+        if (base) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(base + total);
         total += (std::max<uint64_t>(bytes, 1) + 255) / 256 * 256;
-        return at;
     };
-    const size_t succ = need(m * 4), info = need(n * sizeof(hbl::Entry)),
-                 entry = need(std::max<uint64_t>(n * sizeof(hbl::Entry), (n + 1) * 8)), visited = need((n + 31) / 32 * 4),
-                 queue = need(n * 4), qpred = need(n * 4), qdist = need(n * 4), roots = need(root_piece(n) * 4),
-                 tile0 = need(hbl::tiles(n, m) * 4), tile1 = need(hbl::tiles(n, m) * 4), ctl = need(sizeof(hbl::Control)),
-                 bad = need(sizeof(int));
-    const cudaError_t e = cudaMalloc(&v->block, total);
-    if (e != cudaSuccess) return e;
-    auto place = [&](auto** p, size_t at) { *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>((char*)v->block + at); };
-    place(&v->d_succ, succ);
-    place(&v->d_info, info);
-    place(&v->d_entry, entry);
-    place(off, entry);
-    place(&v->d_visited, visited);
-    place(&v->d_queue, queue);
-    place(&v->d_qpred, qpred);
-    place(&v->d_qdist, qdist);
-    place(&v->d_roots, roots);
-    place(&v->d_tile[0], tile0);
-    place(&v->d_tile[1], tile1);
-    place(&v->d_ctl, ctl);
-    place(&v->d_bad, bad);
-    return cudaSuccess;
+    place(&v->d_succ, m * 4);
+    place(&v->d_off, f.lean ? rows : std::max<uint64_t>(n * sizeof(hbl::Entry), rows));
+    if (f.lean) {
+        place(&v->d_unit, n * 4);
+    } else {
+        v->d_entry = reinterpret_cast<hbl::Entry*>(v->d_off);
+        place(&v->d_info, n * sizeof(hbl::Entry));
+        place(&v->d_qdist, n * 4);
+    }
+    place(&v->d_visited, (n + 31) / 32 * 4);
+    place(&v->d_queue, n * 4);
+    place(&v->d_qpred, n * 4);
+    place(&v->d_roots, root_piece(n) * 4);
+    place(&v->d_tile[0], hbl::tiles(n, m, f.lg) * 4);
+    place(&v->d_tile[1], hbl::tiles(n, m, f.lg) * 4);
+    place(&v->d_ctl, sizeof(hbl::Control));
+    place(&v->d_bad, sizeof(int));
+    return total;
+}
+
+static cudaError_t visit_alloc(hb_visit* v, const uint64_t* off) {
+    const uint64_t n = v->n, m = v->m;
+    const hbl::Form lean = hbl::choose_form(n, m, UINT64_MAX, 0, 0);
+    const size_t wide = visit_layout(v, hbl::Form{false, hbl::UNIT_LG}, nullptr);
+    const size_t more = wide - visit_layout(v, lean, nullptr);
+    size_t free_bytes = 0, all = 0;
+    if (more > hbl::WIDE_BYTES)
+        if (const cudaError_t e = cudaMemGetInfo(&free_bytes, &all); e != cudaSuccess) return e;
+    v->form = hbl::choose_form(n, m, hbl::longest_row(off, n, m), more, free_bytes);
+    cudaError_t e = hbk::fail_allocation() ? cudaErrorMemoryAllocation
+                                           : cudaMalloc(&v->block, visit_layout(v, v->form, nullptr));
+    if (e == cudaErrorMemoryAllocation && !v->form.lean) {
+        cudaGetLastError();
+        v->form = lean;
+        e = hbk::fail_allocation() ? cudaErrorMemoryAllocation : cudaMalloc(&v->block, visit_layout(v, lean, nullptr));
+    }
+    if (e == cudaSuccess) visit_layout(v, v->form, (char*)v->block);
+    return e;
 }
 
 // One visit from the given roots; dist and pred (by node, device) get its
@@ -141,12 +160,15 @@ static int visit_levels(hb_visit* v, const uint64_t* roots, size_t nroots, uint6
     const uint64_t q0 = v->tail;
     hbl::Level a{};
     a.info = v->d_info;
+    a.off = v->form.lean ? v->d_off : nullptr;
+    a.lg = v->form.lg;
     a.succ = v->d_succ;
     a.visited = v->d_visited;
     a.dist = dist;
     a.pred = pred;
     a.queue = v->d_queue;
     a.entry = v->d_entry;
+    a.unit = v->d_unit;
     a.qpred = v->d_qpred;
     a.qdist = v->d_qdist;
     a.ctl = v->d_ctl;
@@ -154,7 +176,7 @@ static int visit_levels(hb_visit* v, const uint64_t* roots, size_t nroots, uint6
     a.tile[0] = v->d_tile[0];
     a.tile[1] = v->d_tile[1];
     a.n = v->n;
-    a.small = hbl::small_units(v->n, v->m);
+    a.small = hbl::small_units(v->n, v->m, v->form.lg);
     std::vector<uint32_t> r32(nroots);
     for (size_t i = 0; i < nroots; i++) r32[i] = (uint32_t)roots[i];
     *v->h_ctl = hbl::Control{};
@@ -188,6 +210,32 @@ static int visit_levels(hb_visit* v, const uint64_t* roots, size_t nroots, uint6
     float ms = 0.f;
     cudaEventElapsedTime(&ms, v->ev0, v->ev1);
     st.device_ms = ms;
+    return HB_OK;
+}
+
+// The first k events of the visit that began at queue slot q0 and reached `count`
+// nodes, into the caller's arrays (null: not wanted). On return the stream is idle.
+static int visit_events(hb_visit* v, uint64_t q0, uint64_t count, uint64_t k, uint32_t* nodes, uint32_t* preds,
+                        uint32_t* dists) {
+    if (k == 0 || !(nodes || preds || dists)) return HB_OK;
+    cudaStream_t s = v->stream;
+    if (nodes)
+        VC(v, cudaMemcpyAsync(nodes, v->d_queue + q0, k * 4, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
+    if (preds)
+        VC(v, cudaMemcpyAsync(preds, v->d_qpred + q0, k * 4, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
+    if (dists)
+        VC(v, cudaMemcpyAsync(dists, (v->form.lean ? v->d_unit : v->d_qdist) + q0, k * 4, cudaMemcpyDeviceToHost, s),
+           "cudaMemcpyAsync");
+    VC(v, cudaStreamSynchronize(s), "cudaStreamSynchronize");
+    if (dists && v->form.lean) {
+        // each expanded level's first entry is its end (hbl::end_of_level)
+        uint32_t d = 0;
+        for (uint64_t b = 0; b < k; d++) {
+            const uint64_t e = std::min<uint64_t>(k, dists[b] ? dists[b] - q0 : count);
+            std::fill(dists + b, dists + e, d);
+            b = e;
+        }
+    }
     return HB_OK;
 }
 
@@ -242,11 +290,10 @@ int hb_visit_create(const hb_graph_view* g, int device, void* stream, hb_visit**
         v->own_stream = true;
     }
     cudaDeviceGetAttribute(&v->sms, cudaDevAttrMultiProcessorCount, device);
-    uint64_t* d_off = nullptr;
-    if ((r = visit_cuda(v, visit_alloc(v, &d_off), "cudaMalloc")) ||
+    if ((r = visit_cuda(v, visit_alloc(v, g->offsets), "cudaMalloc")) ||
         (r = visit_cuda(v, cudaMallocHost((void**)&v->h_ctl, sizeof(hbl::Control)), "cudaMallocHost")))
         return fail(r);
-    if ((r = visit_cuda(v, cudaMemcpyAsync(d_off, g->offsets, (n + 1) * 8, cudaMemcpyHostToDevice, v->stream),
+    if ((r = visit_cuda(v, cudaMemcpyAsync(v->d_off, g->offsets, (n + 1) * 8, cudaMemcpyHostToDevice, v->stream),
                         "cudaMemcpyAsync")))
         return fail(r);
     if (m && (r = visit_cuda(v, cudaMemcpyAsync(v->d_succ, g->successors, m * 4, cudaMemcpyHostToDevice,
@@ -258,15 +305,17 @@ int hb_visit_create(const hb_graph_view* g, int device, void* stream, hb_visit**
     int bad = 0;
     if ((r = visit_cuda(v, cudaMemsetAsync(d_bad, 0, sizeof(int), v->stream), "cudaMemsetAsync"))) return fail(r);
     const int grid = (int)std::min<uint64_t>((std::max(n, m) + 255) / 256 + 1, 8192);
-    hbv::k_visit_validate<<<grid, 256, 0, v->stream>>>(d_off, v->d_succ, n, m, d_bad);
+    hbv::k_visit_validate<<<grid, 256, 0, v->stream>>>(v->d_off, v->d_succ, n, m, d_bad);
     if ((r = visit_cuda(v, cudaGetLastError(), "k_visit_validate")) ||
         (r = visit_cuda(v, cudaMemcpyAsync(&bad, d_bad, sizeof(int), cudaMemcpyDeviceToHost, v->stream),
                         "cudaMemcpyAsync")) ||
         (r = visit_cuda(v, cudaStreamSynchronize(v->stream), "cudaStreamSynchronize")))
         return fail(r);
     if (bad) return fail(visit_err(v, HB_ERR_INVALID, "graph has decreasing offsets or successors >= num_nodes"));
-    hbl::k_info<<<(int)std::min<uint64_t>(n / 256 + 1, 8192), 256, 0, v->stream>>>(d_off, n, v->d_info);
-    if ((r = visit_cuda(v, cudaGetLastError(), "k_info"))) return fail(r);
+    if (!v->form.lean) {
+        hbl::k_info<<<(int)std::min<uint64_t>(n / 256 + 1, 8192), 256, 0, v->stream>>>(v->d_off, n, v->d_info);
+        if ((r = visit_cuda(v, cudaGetLastError(), "k_info"))) return fail(r);
+    }
     v->host_visited.assign(std::max<uint64_t>(words, 1), 0);
     if ((r = visit_cuda(v, cudaEventCreate(&v->ev0), "cudaEventCreate")) ||
         (r = visit_cuda(v, cudaEventCreate(&v->ev1), "cudaEventCreate")))
@@ -304,16 +353,7 @@ int hb_visit_run(hb_visit* v, const uint64_t* roots, size_t nroots, uint64_t max
     if (int r = visit_levels(v, roots, nroots, max_distance, nullptr, nullptr, st)) return r;
     const uint64_t count = st.visited;
     // the events into the caller's buffers
-    if (count && (nodes || preds || dists)) {
-        const size_t k = std::min<uint64_t>(capacity, count);
-        if (nodes)
-            VC(v, cudaMemcpyAsync(nodes, v->d_queue + q0, k * 4, cudaMemcpyDeviceToHost, v->stream), "cudaMemcpyAsync");
-        if (preds)
-            VC(v, cudaMemcpyAsync(preds, v->d_qpred + q0, k * 4, cudaMemcpyDeviceToHost, v->stream), "cudaMemcpyAsync");
-        if (dists)
-            VC(v, cudaMemcpyAsync(dists, v->d_qdist + q0, k * 4, cudaMemcpyDeviceToHost, v->stream), "cudaMemcpyAsync");
-        VC(v, cudaStreamSynchronize(v->stream), "cudaStreamSynchronize");
-    }
+    if (int r = visit_events(v, q0, count, std::min<uint64_t>(capacity, count), nodes, preds, dists)) return r;
     if (stats) *stats = st;
     if (capacity < count)
         return visit_err(v, HB_ERR_INVALID, "capacity holds fewer than the " + std::to_string(count) +
@@ -334,19 +374,29 @@ int hb_visit_each(hb_visit* v, const uint64_t* roots, size_t nroots, uint32_t* d
     VC(v, cudaMemcpyAsync(v->host_visited.data(), v->d_visited, words * 4, cudaMemcpyDeviceToHost, s),
        "cudaMemcpyAsync");
     // the caller's entries, which the visits write over by node on the device
-    // (in place of a pass of scattered host writes over the events)
-    if (dist) {
-        if (!v->d_dist) VC(v, cudaMalloc((void**)&v->d_dist, v->n * 4), "cudaMalloc");
+    // (in place of a pass of scattered host writes over the events, which is left
+    // for a device without room for them)
+    bool by_node = true;
+    auto room = [&](uint32_t** p) {
+        if (!by_node || *p) return HB_OK;
+        const cudaError_t e = hbk::fail_allocation() ? cudaErrorMemoryAllocation : cudaMalloc((void**)p, v->n * 4);
+        if (e != cudaErrorMemoryAllocation) return visit_cuda(v, e, "cudaMalloc");
+        cudaGetLastError();
+        by_node = false;
+        return HB_OK;
+    };
+    if (dist)
+        if (int r = room(&v->d_dist)) return r;
+    if (pred)
+        if (int r = room(&v->d_pred)) return r;
+    if (by_node && dist)
         VC(v, cudaMemcpyAsync(v->d_dist, dist, v->n * 4, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
-    }
-    if (pred) {
-        if (!v->d_pred) VC(v, cudaMalloc((void**)&v->d_pred, v->n * 4), "cudaMalloc");
+    if (by_node && pred)
         VC(v, cudaMemcpyAsync(v->d_pred, pred, v->n * 4, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
-    }
     VC(v, cudaStreamSynchronize(s), "cudaStreamSynchronize");
     int rc = HB_OK;
     bool wrote = false;
-    std::vector<uint32_t> nodes;
+    std::vector<uint32_t> nodes, ps, ds;
     for (size_t i = 0; i < nroots && rc == HB_OK; i++) {
         const uint64_t r = roots[i];
         if (r >= v->n) {
@@ -356,8 +406,20 @@ int hb_visit_each(hb_visit* v, const uint64_t* roots, size_t nroots, uint32_t* d
         if ((v->host_visited[r >> 5] >> (r & 31)) & 1) continue;  // seq.rs:130: already visited
         hb_visit_stats st{};
         const uint64_t q0 = v->tail;
-        rc = visit_levels(v, &r, 1, UINT64_MAX, dist ? v->d_dist : nullptr, pred ? v->d_pred : nullptr, st);
-        wrote = true;
+        rc = visit_levels(v, &r, 1, UINT64_MAX, by_node && dist ? v->d_dist : nullptr,
+                          by_node && pred ? v->d_pred : nullptr, st);
+        if (!by_node && rc == HB_OK) {
+            nodes.resize(st.visited);
+            ps.resize(pred ? st.visited : 0);
+            ds.resize(dist ? st.visited : 0);
+            rc = visit_events(v, q0, st.visited, st.visited, nodes.data(), pred ? ps.data() : nullptr,
+                              dist ? ds.data() : nullptr);
+            for (uint64_t k = 0; k < st.visited && rc == HB_OK; k++) {
+                if (dist) dist[nodes[k]] = ds[k];
+                if (pred) pred[nodes[k]] = ps[k];
+            }
+        }
+        wrote = by_node;
         if (rc != HB_OK || i + 1 == nroots) break;
         // what is visited by now, for the next roots: the bitmap, or the few nodes of a small visit
         if (st.visited > words) {

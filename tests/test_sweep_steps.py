@@ -51,3 +51,47 @@ def test_sizes(hb, n, level):
     """One node and a few, both sides of a block's threads, of the graphs whose
     levels one block takes, and more nodes than have their bits in shared memory."""
     _check(hb, hb.Graph.weblike(n, cap=min(n, 3000), window=min(64, n), seed=n), level)
+
+
+def _acyclic(hb, n, degree, seed):
+    """Every arc leads to a larger node, so that every arc is between components."""
+    rng = np.random.RandomState(seed)
+    rows = [np.unique(rng.randint(v + 1, n, degree)) if v + 1 < n else np.zeros(0, int) for v in range(n)]
+    off = np.concatenate([[0], np.cumsum([len(r) for r in rows])])
+    return hb.Graph.from_csr(off.astype(np.uint64), np.concatenate(rows).astype(np.uint32))
+
+
+def _check_failing(hb, g, fail, fails):
+    """The sweep where allocation `fail` fails (0 would be the rows and entries of the
+    visits); `fails`: the sweep makes that many."""
+    if fail is None:
+        return _check(hb, g, "radius_diameter")
+    hb.debug_fail_allocations(fail)
+    try:
+        _check(hb, g, "radius_diameter")
+        # what is left of the count fails a handle's creation
+        small = hb.Graph.erdos_renyi(100, 3, 1)
+        build = hb.HyperBallBuilder.new(small, hb.HyperLogLogBuilder(100).log_2_num_reg(4).build()).build
+        if fails:
+            build().close()
+        else:
+            with pytest.raises(hb.HyperBallError):
+                build()
+    finally:
+        hb.debug_fail_allocations(-1)
+
+
+@pytest.mark.parametrize("n,degree", [(2_000, 1), (2_000, 2), (2_000, 6), (300, 60)])
+@pytest.mark.parametrize("fail", [None, 1, 2])
+def test_list_of_arcs_between_components(hb, n, degree, fail):
+    """Up to two such arcs a node stand in the bounds' arrays; where the list of more
+    (1: its sources, 2: its targets) cannot be allocated the host passes over all arcs."""
+    _check_failing(hb, _acyclic(hb, n, degree, degree), fail, degree > 2)
+
+
+@pytest.mark.parametrize("fail", [None, 1, 2, 3, 4, 5])
+def test_more_tiles_than_nodes(hb, fail):
+    """Arcs between two components, often repeated: the tiles' counts do not fit the bounds' arrays."""
+    m = 2048 * 5 + 7
+    g = hb.Graph.from_csr(np.array([0, m, m, m], dtype=np.uint64), np.resize([1, 2], m).astype(np.uint32))
+    _check_failing(hb, g, fail, True)

@@ -57,6 +57,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "hb_internal.h"
@@ -813,27 +814,44 @@ struct Sweeper {
 
     // The arcs between components (comp, and d_comp on the device), in arc order.
     // A host pass over every arc took 5.9 ms on a web-like graph of 2.6 M arcs.
-    void cross_arcs(std::vector<uint32_t>& src, std::vector<uint32_t>& dst) {
+    // The list and its counts stand in the bounds' arrays, which are set later;
+    // what does not fit there is allocated, up to LISTED arcs (an acyclic graph
+    // lists all of its arcs, 8 bytes each here and 16 on the host). False: more,
+    // or no room, and nothing is listed.
+    static constexpr u64 LISTED = 1ull << 27;
+    bool cross_arcs(std::vector<uint32_t>& src, std::vector<uint32_t>& dst) {
         const u64 nt = hbk::arc_tiles(m);
-        if (nt == 0) return;
+        if (nt == 0) return true;
         struct Temp {
             std::vector<void*> ps;
             ~Temp() {
                 for (void* p : ps) cudaFree(p);
             }
         } temp;
-        auto get = [&](auto** p, u64 count) {
-            alloc(p, count);
-            temp.ps.push_back(*p);
+        // `count` words in `place` (n of 64 bits), or else in an allocation
+        auto get = [&](auto** p, u64 count, u64* place) {
+            using T = std::remove_reference_t<decltype(**p)>;
+            if (count * sizeof(T) <= n * 8) {
+                *p = reinterpret_cast<T*>(place);
+                return true;
+            }
+            void* q = nullptr;
+            const cudaError_t e = hbk::fail_allocation() ? cudaErrorMemoryAllocation : cudaMalloc(&q, count * sizeof(T));
+            if (e == cudaErrorMemoryAllocation) {
+                cudaGetLastError();
+                return false;
+            }
+            ck(e, "cudaMalloc");
+            temp.ps.push_back(q);
+            *p = static_cast<T*>(q);
+            return true;
         };
         uint32_t *tile = nullptr, *d_src = nullptr, *d_dst = nullptr;
         unsigned long long *count = nullptr, *scratch = nullptr;
         u64* at = nullptr;
         const u64 sl = hbk::scan_scratch_len(nt + 1);
-        get(&tile, nt);
-        get(&count, nt + 1);
-        get(&at, nt + 1);
-        get(&scratch, sl);
+        if (!get(&tile, nt, d_fl) || !get(&count, nt + 1, d_fh) || !get(&at, nt + 1, d_bl) || !get(&scratch, sl, d_bh))
+            return false;
         auto launch = [&](int e, const char* what) { ck((cudaError_t)e, what); };
         ck(cudaMemsetAsync(count + nt, 0, 8, s), "cudaMemsetAsync");
         launch(hbk::launch_tile_start(d_off, n, tile, s), "k_tile_start");
@@ -842,15 +860,15 @@ struct Sweeper {
         u64 total = 0;
         ck(cudaMemcpyAsync(&total, at + nt, 8, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
         sync();
-        if (total == 0) return;
-        get(&d_src, total);
-        get(&d_dst, total);
+        if (total == 0) return true;
+        if (total > LISTED || !get(&d_src, total, d_ft) || !get(&d_dst, total, d_bt)) return false;
         launch(hbk::launch_cross_arcs(d_off, n, m, tile, d_succ, d_comp, count, at, d_src, d_dst, s), "k_cross_arcs");
         src.resize(total);
         dst.resize(total);
         ck(cudaMemcpyAsync(src.data(), d_src, total * 4, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
         ck(cudaMemcpyAsync(dst.data(), d_dst, total * 4, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
         sync();
+        return true;
     }
 
     // computer.rs:487-542
@@ -1174,35 +1192,24 @@ int run(const hb_graph_view* g, const hb_graph_view* t, int level, const uint8_t
     ck(cudaMemcpyAsync(w.d_comp, w.comp.data(), n * 4, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
     mark("components");
     if (!w.undirected) {
-        // scc_graph.rs:118-227, over the arcs between components alone (found
-        // on the device, in arc order), grouped by their component: the order
-        // in which the reference meets them
-        std::vector<uint32_t> src, dst;
-        w.cross_arcs(src, dst);
-        std::vector<u64> first(w.ncomp + 1, 0);
-        for (uint32_t v : src) first[w.comp[v] + 1]++;
-        for (u64 c = 0; c < w.ncomp; c++) first[c + 1] += first[c];
-        std::vector<u64> order(src.size());
-        {
-            std::vector<u64> at(first.begin(), first.end() - 1);
-            for (u64 k = 0; k < src.size(); k++) order[at[w.comp[src[k]]]++] = k;
-        }
+        // scc_graph.rs:118-227: of the arcs between two components the one with the
+        // largest value; a component's arcs in arc order, as the reference meets them
         std::vector<uint32_t> bs(w.ncomp, 0xffffffffu), be(w.ncomp, 0);
         std::vector<uint32_t> children;
         auto value = [&](u64 a, u64 b) { return ht.deg(a) + hg.deg(b); };
-        for (u64 c = 0; c < w.ncomp; c++) {
-            for (u64 k = first[c]; k < first[c + 1]; k++) {
-                const uint32_t v = src[order[k]], x = dst[order[k]], xc = w.comp[x];
-                if (bs[xc] == 0xffffffffu) {
-                    bs[xc] = v;
-                    be[xc] = x;
-                    children.push_back(xc);
-                }
-                if (value(v, x) > value(bs[xc], be[xc])) {
-                    bs[xc] = v;
-                    be[xc] = x;
-                }
+        auto meet = [&](uint32_t v, uint32_t x) {
+            const uint32_t xc = w.comp[x];
+            if (bs[xc] == 0xffffffffu) {
+                bs[xc] = v;
+                be[xc] = x;
+                children.push_back(xc);
             }
+            if (value(v, x) > value(bs[xc], be[xc])) {
+                bs[xc] = v;
+                be[xc] = x;
+            }
+        };
+        auto close = [&](u64 c) {
             w.seg[c] = w.ctarget.size();
             for (uint32_t ch : children) {
                 w.ctarget.push_back(ch);
@@ -1211,6 +1218,37 @@ int run(const hb_graph_view* g, const hb_graph_view* t, int level, const uint8_t
                 bs[ch] = 0xffffffffu;
             }
             children.clear();
+        };
+        // keys grouped by component, each group in order
+        auto grouped = [&](u64 count, auto&& comp_of, auto& order) {
+            std::vector<u64> first(w.ncomp + 1, 0);
+            for (u64 k = 0; k < count; k++) first[comp_of(k) + 1]++;
+            for (u64 c = 0; c < w.ncomp; c++) first[c + 1] += first[c];
+            std::vector<u64> at(first.begin(), first.end() - 1);
+            order.resize(count);
+            for (u64 k = 0; k < count; k++) order[at[comp_of(k)]++] = k;
+            return first;
+        };
+        std::vector<uint32_t> src, dst;
+        if (w.cross_arcs(src, dst)) {
+            std::vector<u64> order;
+            const auto first = grouped(src.size(), [&](u64 k) { return w.comp[src[k]]; }, order);
+            for (u64 c = 0; c < w.ncomp; c++) {
+                for (u64 k = first[c]; k < first[c + 1]; k++) meet(src[order[k]], dst[order[k]]);
+                close(c);
+            }
+        } else {
+            // node by node, with nothing kept for an arc
+            std::vector<uint32_t> members;
+            const auto first = grouped(n, [&](u64 v) { return w.comp[v]; }, members);
+            for (u64 c = 0; c < w.ncomp; c++) {
+                for (u64 k = first[c]; k < first[c + 1]; k++) {
+                    const uint32_t v = members[k];
+                    for (u64 e = hg.off[v]; e < hg.off[v + 1]; e++)
+                        if (w.comp[hg.succ[e]] != c) meet(v, hg.succ[e]);
+                }
+                close(c);
+            }
         }
     }
     mark("component arcs");

@@ -1281,9 +1281,16 @@ int iter_finish(hb_handle* h, IterPlan& p, bool from_graph, double union_ms, hb_
 // Waits until the iteration's last kernel has written the totals. They are its
 // last store, marked by their moment: seeing them takes the host about 2 us less
 // than waiting for the stream, which is asked every so often all the same (it
-// tells of errors). Work that follows is ordered by the stream.
+// tells of errors). Work that follows is ordered by the stream. Looking takes a
+// whole core, as waiting does by default: a program that asked the device to
+// block or to yield (cudaSetDeviceFlags) gets the stream's wait, which does.
 cudaError_t await_totals(hb_handle* h, cudaStream_t s) {
     if (h->events) return cudaStreamSynchronize(s);
+    unsigned flags = 0;
+    const cudaError_t e = cudaGetDeviceFlags(&flags);
+    if (e != cudaSuccess) return e;
+    flags &= cudaDeviceScheduleMask;
+    if (flags == cudaDeviceScheduleBlockingSync || flags == cudaDeviceScheduleYield) return cudaStreamSynchronize(s);
     const unsigned long long* end = &h->h_tot->end;
     for (unsigned k = 1;; k++) {
         if (__atomic_load_n(end, __ATOMIC_ACQUIRE) != 0) return cudaSuccess;

@@ -514,9 +514,9 @@ int hb_device_transpose_noalloc(const uint64_t* d_offsets, const uint32_t* d_suc
  * restore the defaults. No reference counterpart. */
 int hb_debug_far_wait(hb_handle* h, uint32_t polls, uint32_t extra_tx_bytes);
 /* Test hook (process-wide): the device allocation (a handle's creation, its
- * discount arrays, a visit's arrays, a sweep's rows) that is the (after + 1)-th
+ * discount arrays, a visit's arrays, a sweep's rows, a stage for results) that is the (after + 1)-th
  * from now fails once, as a cudaMalloc failure would: with HB_ERR_OOM, or, where
- * a visit or a sweep has a smaller form of its arrays, by taking that; after < 0
+ * a call has a way without that memory, by taking it; after < 0
  * turns it off. A failing call releases what it had allocated. No reference
  * counterpart. */
 int hb_debug_fail_allocations(int64_t after);
@@ -534,7 +534,8 @@ uint64_t hb_kernel_launches(const hb_handle* h);
  * for the next one, so creating and destroying handles in a loop maps no new
  * memory. This returns the reserved, unused memory of `device` to the device
  * (memory in use is untouched), and frees the small page-locked host blocks
- * that destroyed handles left for reuse. No reference counterpart. */
+ * that destroyed handles left for reuse and those that staged results (eight of
+ * 1 MiB at most). No reference counterpart. */
 int hb_release_cached_memory(int device);
 
 #ifdef __cplusplus

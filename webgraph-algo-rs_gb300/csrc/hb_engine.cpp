@@ -110,8 +110,6 @@ cudaError_t pool_alloc(int device, void** p, size_t bytes, cudaStream_t s) {
 // handle. Freed blocks are kept for the next handle instead of going back
 // through cudaFreeHost, which may synchronise the device under the other
 // handles' work (the job server destroys handles while others run).
-// Of the large ones, which stage results, kStagesKept at most are kept.
-constexpr size_t kStageBytes = 1u << 20, kStagesKept = 8;
 std::mutex g_pinned_mu;
 std::multimap<size_t, void*> g_pinned_free;
 
@@ -137,15 +135,41 @@ cudaError_t pinned_alloc(void** p, size_t bytes) {
 
 void pinned_free(void* p, size_t bytes) {
     if (!p) return;
-    const size_t c = pinned_class(bytes);
+    std::lock_guard<std::mutex> lk(g_pinned_mu);
+    g_pinned_free.emplace(pinned_class(bytes), p);
+}
+
+// Page-locked blocks that stage small results: at most kStages are ever made (a
+// getter that finds them all in use goes without one), and they are kept, so no
+// call pays for one twice and none is freed under other handles' work.
+constexpr size_t kStageBytes = 1u << 20, kStages = 8;
+size_t g_stages = 0;              // made and not released (g_pinned_mu)
+std::vector<void*> g_stages_free;
+
+// null: none to be had
+void* stage_take() {
     {
         std::lock_guard<std::mutex> lk(g_pinned_mu);
-        if (c < kStageBytes || g_pinned_free.count(c) < kStagesKept) {
-            g_pinned_free.emplace(c, p);
-            return;
+        if (!g_stages_free.empty()) {
+            void* p = g_stages_free.back();
+            g_stages_free.pop_back();
+            return p;
         }
+        if (g_stages == kStages) return nullptr;
+        g_stages_free.reserve(kStages);
+        g_stages++;
     }
-    cudaFreeHost(p);
+    void* p = nullptr;
+    if (!hbk::fail_allocation() && cudaMallocHost(&p, kStageBytes) == cudaSuccess) return p;
+    cudaGetLastError();
+    std::lock_guard<std::mutex> lk(g_pinned_mu);
+    g_stages--;
+    return nullptr;
+}
+
+void stage_give(void* p) {
+    std::lock_guard<std::mutex> lk(g_pinned_mu);
+    g_stages_free.push_back(p);
 }
 
 }  // namespace
@@ -1677,16 +1701,13 @@ int copy_nodes_range(const hb_handle* h, const double* src, double* dst, uint64_
     hb_handle* hh = const_cast<hb_handle*>(h);
     if (count == 0) return HB_OK;
     HB_CUDA(hh, cudaSetDevice(h->device));
-    if (count * 8 <= kStageBytes) {
+    if (void* stage = count * 8 <= kStageBytes ? stage_take() : nullptr) {
         // up to here the kernel writes page-locked memory and the host copies on:
         // an allocation, a copy to pageable memory and a second wait less
-        void* stage = nullptr;
-        cudaError_t e = pinned_alloc(&stage, kStageBytes);
-        if (e != cudaSuccess) return cuda_err(hh, e, "cudaMallocHost");
-        e = (cudaError_t)hbk::launch_gather_f64(src, h->d_inv + start, static_cast<double*>(stage), count, h->stream);
+        cudaError_t e = (cudaError_t)hbk::launch_gather_f64(src, h->d_inv + start, static_cast<double*>(stage), count, h->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
         if (e == cudaSuccess) std::memcpy(dst, stage, count * 8);
-        pinned_free(stage, kStageBytes);
+        stage_give(stage);
         return e == cudaSuccess ? HB_OK : cuda_err(hh, e, "launch_gather_f64");
     }
     double* tmp = nullptr;
@@ -2246,11 +2267,15 @@ int hb_release_cached_memory(int device) {
     }
     // the page-locked blocks no handle holds
     std::multimap<size_t, void*> blocks;
+    std::vector<void*> stages;
     {
         std::lock_guard<std::mutex> lk(g_pinned_mu);
         blocks.swap(g_pinned_free);
+        stages.swap(g_stages_free);
+        g_stages -= stages.size();
     }
     for (auto& b : blocks) cudaFreeHost(b.second);
+    for (void* p : stages) cudaFreeHost(p);
     cudaGetLastError();
     return HB_OK;
 }

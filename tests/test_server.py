@@ -101,3 +101,18 @@ def test_server_reports_failures_loudly_without_a_device(product_lib):
     with pytest.raises(hb.NotRunError):
         s.neighborhood_function(j)
     s.close()
+
+
+@pytest.mark.gpu
+def test_single_job_leaves_the_reserved_sms():
+    """A job that runs alone keeps to the SMs that the reserve leaves: one of them
+    takes many times as long as all."""
+    g = hb.Graph.erdos_renyi(300_000, 8, 3)
+    times = {}
+    for reserve in (0, 10_000):  # of more than there are: all but one
+        s = hb.HyperBallServer(max_active=1, union_sm_reserve=reserve)
+        j = s.submit(g, 8, sum_of_distances=True)
+        s.wait(j, timeout=600)
+        times[reserve] = s.stats()["union_ms"]
+        s.close()
+    assert times[10_000] > 8 * times[0], times

@@ -1037,8 +1037,10 @@ int enqueue_pre(hb_handle* h, hbk::UnionArgs& a, bool first_systolic, cudaStream
     return HB_OK;
 }
 
-// The heavy-node kernel (side stream) and the window kernel of this handle.
-int enqueue_union(hb_handle* h, const hbk::UnionArgs& a, cudaStream_t s, bool window, bool chained) {
+// The heavy-node kernel (side stream) and the window kernel of this handle, the
+// latter on `sms` SMs (0: all).
+int enqueue_union(hb_handle* h, const hbk::UnionArgs& a, cudaStream_t s, bool window, bool chained, int sms = 0) {
+    auto on = [&](int grid) { return sms > 0 ? std::min(grid, (grid + h->sms - 1) / h->sms * sms) : grid; };
     if (h->events || h->n_heavy) chained = false;
     if (h->n_heavy) {
         // The heavy nodes (one CTA each) start first on the side stream; the
@@ -1058,11 +1060,11 @@ int enqueue_union(hb_handle* h, const hbk::UnionArgs& a, cudaStream_t s, bool wi
         HB_CUDA(h, cudaEventRecord(h->join, h->side));
     }
     if (window && h->n_tiles && a.staged)
-        HB_LAUNCH(h, hbk::launch_union_staged(h->log2m, a, a.occ ? h->grid_staged_occ : h->grid_staged, s,
+        HB_LAUNCH(h, hbk::launch_union_staged(h->log2m, a, on(a.occ ? h->grid_staged_occ : h->grid_staged), s,
                                               chained));
     else if (window && h->n_tiles)
         HB_LAUNCH(h, hbk::launch_union_tile(h->log2m, a,
-                                            a.occ == 2 ? h->grid_tile_two : a.occ ? h->grid_tile_occ : h->grid_tile,
+                                            on(a.occ == 2 ? h->grid_tile_two : a.occ ? h->grid_tile_occ : h->grid_tile),
                                             s, chained));
     return HB_OK;
 }
@@ -1113,9 +1115,9 @@ int enqueue_post(hb_handle* h, const hbk::UnionArgs& a, cudaStream_t s, bool ext
 // reads the totals from h->h_tot (and, for batches, h->h_inst_*) once s is
 // synchronised; the per-iteration constants come from h->h_ic.
 int enqueue_iteration(hb_handle* h, hbk::UnionArgs a, bool first_systolic, cudaStream_t s,
-                      bool external) {
+                      bool external, int sms = 0) {
     int r = enqueue_pre(h, a, first_systolic, s, external, !external);
-    if (!r) r = enqueue_union(h, a, s, true, !external);
+    if (!r) r = enqueue_union(h, a, s, true, !external, sms);
     if (!r) r = enqueue_join(h, s);
     if (!r) r = enqueue_post(h, a, s, external, !external);
     return r;
@@ -1361,6 +1363,7 @@ struct MultiCtx {
     // the shared launch's job table (its kernel parameters)
     std::unique_ptr<hbk::JobsArgs> jobs;
     int grid = 1;
+    int sms = 0;                      // that a union launch may hold (0: all)
     cudaEvent_t u0 = nullptr, u1 = nullptr;  // around the union part (shared launch, heavy kernels)
     cudaEvent_t b0 = nullptr, b1 = nullptr;  // around the whole step
     // a handle with a stream of its own runs its pre and post parts there, so
@@ -1465,7 +1468,7 @@ static int multi_init(MultiCtx& mc, int device, cudaStream_t s) {
 // nodes in all, 2.69 instead of 4.30 ms with 64 of 1e4, 12.2 instead of 15.5 ms
 // with 128 of 4e4 (one after the other with their own kernels: 2.02, 4.47, 14.5).
 // Many running jobs of a server keep the shared kernel: their launches would
-// cost more.
+// cost more. A single one's kernel leaves the SMs free that the shared one does.
 static bool branched(const std::vector<hb_handle*>& hs, const MultiCtx& mc) { return mc.branches || hs.size() == 1; }
 
 // The launches of one step on stream x (the handles' plans are final).
@@ -1477,7 +1480,7 @@ static int multi_enqueue(std::vector<hb_handle*>& hs, std::vector<IterPlan>& pla
     int r;
     if (branched(hs, mc)) {
         *njobs = 0;
-        if (hs.size() == 1) return enqueue_iteration(hs[0], plans[0].a, plans[0].first_systolic, x, external);
+        if (hs.size() == 1) return enqueue_iteration(hs[0], plans[0].a, plans[0].first_systolic, x, external, mc.sms);
         cudaError_t e = cudaEventRecord(mc.fork_ev[0], x);
         for (size_t j = 0; j < hs.size() && e == cudaSuccess; j++) {
             const cudaStream_t y = hs[j]->cap;  // capturing: part of the capture by its wait
@@ -1797,6 +1800,7 @@ void hb_multi_reserve_sms(hb_multi* m, uint32_t sms) {
     const int per_sm = std::max(1, hbk::jobs_grid(m->mc.device) / std::max(all, 1));
     const int used = std::max(1, all - (int)std::min<uint32_t>(sms, (uint32_t)all - 1));
     m->mc.grid = per_sm * used;
+    m->mc.sms = used;
 }
 
 int hb_multi_set_stream(hb_handle* h, void* stream) {

@@ -86,7 +86,8 @@ typedef struct hb_options {
     uint64_t weight_seed;     /* seeds the values added for weights (the reference uses a non-reproducible RNG, HB:1167-1174) */
     void* stream;             /* cudaStream_t to launch on; NULL = legacy default stream */
     uint32_t small_max_degree;  /* tuning: nodes up to this out-degree run one lane-group each; HB_AUTO = 64 (see hb_tune_degree_buckets) */
-    uint32_t medium_max_degree; /* tuning: nodes up to this out-degree run one 8-lane team each, above: one CTA; HB_AUTO = 512, or 1024 when the counters take 128 MiB or more */
+    uint32_t medium_max_degree; /* tuning: nodes up to this out-degree run one 8-lane team each, above: one CTA; HB_AUTO = 512, or 1024 when the counters take 128 MiB or more;
+                                   so does 4096 beside small_max_degree 64, the pair that hb_tune_degree_buckets falls back to */
     uint32_t union_variant;     /* tuning: HB_AUTO = the autotuner picks the union-kernel variant per graph
                                    (see hb_union_variant_count); else the index of a fixed variant.
                                    Every variant gives bit-identical results. */
@@ -154,7 +155,8 @@ int hb_run_until_done(hb_handle* h);
  * CTA each (above). Builds a handle per candidate pair (small_max in
  * {32, 64, 128, 256, 512, 1024}, medium_max in {4096, 16384, 65536}) from `opts`, times
  * the union kernels over `iterations` standard iterations (at least 2; the
- * first is not counted) and returns the fastest pair and its union time.
+ * first is not counted) and returns the fastest pair and its union time; (64,
+ * 4096) is the default of HB_AUTO and is returned where no pair is clearly faster.
  * Pass the pair as hb_options.small_max_degree / medium_max_degree; every
  * pair gives identical results. No reference counterpart: the reference
  * splits work by arc granularity only (HB:280-283, HB:1012). */

@@ -86,7 +86,7 @@ typedef struct hb_options {
     uint64_t weight_seed;     /* seeds the values added for weights (the reference uses a non-reproducible RNG, HB:1167-1174) */
     void* stream;             /* cudaStream_t to launch on; NULL = legacy default stream */
     uint32_t small_max_degree;  /* tuning: nodes up to this out-degree run one lane-group each; HB_AUTO = 64 (see hb_tune_degree_buckets) */
-    uint32_t medium_max_degree; /* tuning: nodes up to this out-degree run one 8-lane team each, above: one CTA; HB_AUTO = 512, or 1024 when the counters take 128 MiB or more;
+    uint32_t medium_max_degree; /* tuning: nodes up to this out-degree run one 8-lane team each, above: one CTA; HB_AUTO = 512, 1024 when the counters take 128 MiB or more, 2048 from 1.5 GiB on;
                                    so does 4096 beside small_max_degree 64, the pair that hb_tune_degree_buckets falls back to */
     uint32_t union_variant;     /* tuning: HB_AUTO = the autotuner picks the union-kernel variant per graph
                                    (see hb_union_variant_count); else the index of a fixed variant.

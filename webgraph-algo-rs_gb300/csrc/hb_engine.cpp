@@ -1404,13 +1404,20 @@ static constexpr uint32_t kDefaultSmallMax = 64, kDefaultMediumMax = 4096;
 // time, so a node of 4096 arcs is 512 dependent gathers, about 0.28 ms: the
 // whole iteration of a graph whose counters are small, and hidden only where
 // an iteration takes milliseconds. Above the bound a node is a block's.
-// Union time of a standard iteration with bounds 4096 / 1024 / 512 / 256:
-// web-like 2e5, log2m 5 (6 MB of counters) 94 / 49 / 41 / 45 us; web-like 1e6,
-// log2m 6 (64 MB) 278 / 170 / 161 / 174 us; R-MAT 2^20, log2m 8 (268 MB) 563 /
-// 546 / 575 / 573 us; web-like 3.3e7, log2m 6 (2.1 GB) 4.66 / 4.65 / 4.94 /
-// 5.64 ms.
+// Whole runs with a transpose, ms, with bounds 512 / 1024 / 2048 / 4096:
+//   web-like, log2m 6: 5e5 nodes (30 MiB of counters) 1.73 / 1.88 / 2.35 / 3.13,
+//     1e6 (61) 2.80 / 2.95 / 3.45 / 4.59, 2e6 (122) 4.95 / 5.01 / 5.62 / 7.01,
+//     4e6 (244) 9.16 / 8.93 / 9.46 / 11.1, 8e6 (488) 18.7 / 17.8 / 18.2 / 20.2,
+//     1.6e7 (976) 37.3 / 35.1 / 35.3 / 37.3, 3.3e7 (2014) 76.9 / 71.7 / 70.9 / 73.0,
+//     2^26 (4096) 159.6 / 148.3 / 145.5 / 147.7;
+//   log2m 8: 3e5 (73) 2.46 / 2.66 / 3.38 / 4.68, 1e6 (244) 6.38 / 6.55 / 7.28 / 9.04;
+//   R-MAT, 16 arcs a node, log2m 8: 2^18 (64) 1.01 / 1.09 / 1.09 / 1.44, 2^19 (128)
+//     1.91 / 1.90 / 2.11 / 2.88, 2^20 (256) 3.75 / 3.59 / 4.00 / 3.98, 2^21 (512)
+//     6.44 / 6.49 / 6.36 / 6.95, 2^24 (4096) 60.9 / 60.9 / 59.2 / 59.5.
+// What grows with the counters is the time that hides a team's walk.
 static uint32_t auto_medium_max(uint64_t n, uint64_t counter_bytes) {
-    return n * counter_bytes >= (128ull << 20) ? 1024 : 512;
+    const uint64_t mib = (n * counter_bytes) >> 20;
+    return mib >= 1536 ? 2048 : mib >= 128 ? 1024 : 512;
 }
 
 static void multi_free(MultiCtx& mc) {

@@ -634,8 +634,8 @@ class HyperBallBuilder:
     def degree_buckets(self, small_max, medium_max):
         """Nodes of out-degree up to small_max run one lane group each, up to
         medium_max one 8-lane team each, above one CTA each (defaults 64 and
-        512, or 1024 when the counters take 128 MiB or more, which (64, 4096)
-        stands for; tune_degree_buckets picks them per graph). The results do not
+        512, 1024 when the counters take 128 MiB or more and 2048 from 1.5 GiB
+        on, which (64, 4096) stands for; tune_degree_buckets picks them per graph). The results do not
         depend on them."""
         self._small, self._medium = int(small_max), int(medium_max)
         return self

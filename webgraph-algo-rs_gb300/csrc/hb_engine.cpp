@@ -1199,18 +1199,26 @@ void iter_plan(hb_handle* h, IterPlan& p) {
     p.launches0 = hbk::launch_count();
     hbk::UnionArgs& a = p.a;
     a = union_args(h);
-    // Where at least a quarter of the counters changed in the previous
-    // iteration, merge all successors without waiting for their modified bits
-    // (init marks every counter modified, HB:1208, so the first iteration
-    // merges them all). A skipped merge saves a 2^log2m-byte row, the test
-    // costs a dependent load per arc: web-like 3.3e7, log2m 6, iterations 11
-    // and 12 (modified below 7/8) take 5.37 and 4.98 ms testing, 4.55 and
-    // 4.51 ms merging all; R-MAT 2^20, log2m 8 (half of the nodes have no
-    // successor and never change) 0.77 against 0.68 ms. A quarter is where a
-    // handle with a transpose turns systolic (HB:795-810); without one, the
-    // iterations below it test.
+    // Where at least a share of the counters changed in the previous iteration,
+    // merge all successors without waiting for their modified bits (init marks
+    // every counter modified, HB:1208, so the first iteration merges them all). A
+    // skipped merge saves a 2^log2m-byte row, the test costs a dependent load per
+    // arc, so the share grows with the row. Union of the iteration, us, merging all
+    // / testing, by the share that changed before:
+    //   log2m 6: web-like 2e6 0.49: 277 / 289, 0.24: 263 / 263; R-MAT 2^20 0.52:
+    //     222 / 254, 0.23: 164 / 166
+    //   log2m 7: web-like 2e6 0.52: 462 / 515, 0.25: 453 / 468; R-MAT 2^20 0.23: 217 / 219
+    //   log2m 8: web-like 2e6 0.56: 804 / 856, 0.28: 782 / 757; R-MAT 2^20 0.52:
+    //     537 / 629, 0.28: 497 / 349; R-MAT 2^18 0.46: 116 / 119
+    //   log2m 9: web-like 2e6 0.57: 1518 / 1535, 0.29: 1473 / 1266; R-MAT 2^18 0.46: 221 / 215
+    //   log2m 10: web-like 2e6 0.59: 2971 / 2770, 0.30: 2896 / 2121; R-MAT 2^20 0.52:
+    //     1940 / 2230, 0.43: 1831 / 1225; out-regular 1e6 0.34: 1529 / 994
+    // (with a quarter for every size, runs at log2m 10 took 1 to 3% longer than
+    // with 7/8). A quarter is where a handle with a transpose turns systolic
+    // (HB:795-810).
+    const uint64_t eighths = h->log2m <= 7 ? 2 : h->log2m == 8 ? 3 : 4;
     const uint64_t changed_before = h->iteration == 0 ? n : prev_mod;
-    a.gather_all = !h->systolic && changed_before >= n / 4;
+    a.gather_all = !h->systolic && changed_before >= n * eighths / 8;
     // the union-kernel variant (identical results; see Tuner)
     p.merged = a.gather_all ? m - h->self_loops : h->pending_visited;
     const int cls = h->systolic ? -1 : a.gather_all ? 0 : 1;

@@ -302,9 +302,8 @@ __device__ __forceinline__ double warp_sum_f64(double x) {
 // length; each lane keeps PIPE counter gathers in flight while the ids and
 // modified bits of the next PIPE successors load.
 //
-// In iterations where at least a quarter of the counters changed before
-// (`gather_all`), a
-// successor's counter is merged without its modified bit: an unmodified
+// In iterations where enough of the counters changed before (`gather_all`, see
+// iter_plan), a successor's counter is merged without its modified bit: an unmodified
 // successor's counter is already contained in the node's own
 // (c_{t-1}(u) = c_{t-2}(u) <= c_{t-1}(v)), and so is the node's own counter,
 // so merging them changes nothing and no dependent bitmap load stands before

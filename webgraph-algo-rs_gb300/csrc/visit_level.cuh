@@ -47,11 +47,21 @@ constexpr int MAX_SMALL = 1024;  // small levels of one launch
 // a warp queues its claimed nodes GROUP at a time, and when it holds as many; it
 // takes those of half a tile at once
 constexpr int GROUP = 64, RUN = GROUP + 128;
-// units of a level that one block takes: where the visited bits stand in shared
+// Units of a level that one block takes: where the visited bits stand in shared
 // memory and where they don't (a test of 32 scattered bits takes the block's one
-// load unit about 4 cycles there, 32 in global memory)
+// load unit about 4 cycles there, 32 in global memory). Device time of whole
+// visits, us, with 0 / 512 / 1024 / 2048 / 4096 units: bits in shared memory,
+// web-like 2.6e5 143 / 130 / 122 / 123 / 130, out-regular 2.6e5 140 / 121 / 121 /
+// 118 / 150, out-regular 6e4 119 / 98 / 97 / 94 / 115; in global memory, out-regular
+// 6e5 173 / 159 / 160 / 160 / 216, web-like 4e6 471 / 453 / 458 / 453 / 452,
+// out-regular 4e6 471 / 449 / 452 / 451 / 515.
 constexpr uint32_t SMALL = 2048, SMALL_GLOBAL = 512;
-constexpr uint32_t TINY = 16384;       // any level of a graph of at most this many units
+// Any level of a graph of at most this many units, whose launches are then one
+// block each. Visits in one block / cut by level, us: web-like, 3,000 units 39 / 40,
+// 6,700 53 / 58, 10,100 68 / 73, 13,600 74 / 67, 20,400 94 / 81; out-regular, 8,000
+// units 46 / 50, 12,000 55 / 54, 16,000 62 / 54. Sweeps of symmetric graphs, ms:
+// 6,000 units 144 / 155, 8,000 232 / 262, 10,000 313 / 319, 13,000 365 / 337.
+constexpr uint32_t TINY = 10240;
 constexpr uint32_t CAP = 512;          // entries of a level in shared memory
 constexpr uint32_t BITS = 512 * 1024;  // nodes whose visited bits fit shared memory
 

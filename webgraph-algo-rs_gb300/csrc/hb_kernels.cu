@@ -63,43 +63,6 @@ __device__ __forceinline__ void stamp_after(TilePartial* t) {
 }
 
 // ---------------------------------------------------------------------------
-// block-level publish of per-thread statistics into one partial slot
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void publish(double nf, unsigned long long vis, unsigned long long modc,
-                                        unsigned long long scanned, TilePartial* slot) {
-    __shared__ double s_nf[32];
-    __shared__ unsigned long long s_v[32], s_m[32], s_s[32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        nf = __dadd_rn(nf, __shfl_xor_sync(0xffffffffu, nf, off));
-        vis += __shfl_xor_sync(0xffffffffu, vis, off);
-        modc += __shfl_xor_sync(0xffffffffu, modc, off);
-        scanned += __shfl_xor_sync(0xffffffffu, scanned, off);
-    }
-    if (lane == 0) {
-        s_nf[warp] = nf;
-        s_v[warp] = vis;
-        s_m[warp] = modc;
-        s_s[warp] = scanned;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        unsigned long long tv = 0, tm = 0, ts = 0;
-        const int nwarps = (blockDim.x + 31) >> 5;
-        for (int w = 0; w < nwarps; w++) {
-            t = __dadd_rn(t, s_nf[w]);
-            tv += s_v[w];
-            tm += s_m[w];
-            ts += s_s[w];
-        }
-        *slot = TilePartial{t, tv, tm, ts};
-    }
-    __syncthreads();
-}
-
-// ---------------------------------------------------------------------------
 // End of a node's union, for the nodes whose counter changed: the per-node
 // arithmetic of HB:1052-1093, by the lanes that hold the new counter (one of
 // them does the f64 part), while it is still in registers:
@@ -870,10 +833,9 @@ __global__ void __launch_bounds__(256, MINB) k_union_window(const __grid_constan
 
 // ---------------------------------------------------------------------------
 // Several HyperBall instances in one launch: the window work of up to
-// MAX_JOBS handles (the log2m groups of a batch, the running jobs of a
-// server), each with its own arguments and log2m in {4, 6, 8}, drained from
-// one cursor. A block first turns the jobs' work-item counts into a prefix
-// in shared memory; a warp maps each item it takes to its job and runs it
+// MAX_JOBS handles (the running jobs of a server), each with its own arguments
+// and log2m in {4, 6, 8}, drained from one cursor. A block first turns the
+// jobs' work-item counts into a prefix in shared memory; a warp maps each item it takes to its job and runs it
 // exactly as k_union_window would (same items, lanes and order, so every
 // counter and per-item neighbourhood-function part is that job's alone).
 // Integer totals go to each job's partial slot when the warp moves to
@@ -2760,7 +2722,7 @@ int staged_grid(int log2m, int device, int occ) {
 }
 
 // 3 blocks per SM (80 registers, a few spilled) measured faster than 2
-// (128 registers, none spilled) on the batched workload: 266.6 against
+// (128 registers, none spilled) on 4,096 graphs in three groups: 266.6 against
 // 313.6 ms of union time per run
 int launch_union_jobs(const JobsArgs& p, int grid, void* stream) {
     if (p.njobs > (uint32_t)MAX_JOBS) return (int)cudaErrorInvalidValue;

@@ -1,6 +1,7 @@
 """The two forms of a visit's arrays: the choice between them on the host, and on
 the GPU the lean one, which stands in where the wide one's allocation fails,
 against the oracle at the sizes where its paths change."""
+import ctypes
 import os
 import subprocess
 
@@ -145,6 +146,52 @@ def test_distances_by_node_without_room(hb, oracle, lean):
     assert np.all(dist[~seen] == 77) and seen.sum() > 1000
     up = seen & (dist > 0)
     assert np.all(dist[pred[up]] + 1 == dist[up])
+    v.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("which", ["dist", "pred", "both"])
+@pytest.mark.parametrize("lean", [False, True])
+@pytest.mark.parametrize("room", [True, False])
+def test_arrays_by_node(hb, oracle, which, lean, room):
+    """Distances and predecessors by node stand where the events' do; only the lean
+    form needs an allocation, for both, and does without it too. Events after that
+    are whole again."""
+    n = 30_000
+    g = hb.Graph.weblike(n, cap=3000, window=64, seed=9)
+    roots = list(range(100, 200)) + [5, 29_000, 5]
+    want = oracle.OracleVisit(g.offsets, g.successors).visit_each(roots)
+    v = (_Lean(hb) if lean else hb).ParFair(g)
+    dist = np.full(n, 50_000, np.uint32) if which != "pred" else None
+    pred = np.full(n, 50_000, np.uint32) if which != "dist" else None  # no node
+    lib, r = hb.load_library(), np.asarray(roots, dtype=np.uint64)
+    if not room:
+        hb.debug_fail_allocations(0)
+    try:
+        rc = lib.hb_visit_each(v._h, r.ctypes.data_as(ctypes.POINTER(ctypes.c_uint64)), len(r),
+                               dist.ctypes.data if dist is not None else None,
+                               pred.ctypes.data if pred is not None else None, n)
+        assert rc == hb.HB_OK
+        if not room and not (lean and which == "both"):
+            with pytest.raises(hb.HyperBallError):  # nothing was allocated: the failure is still to come
+                hb.HyperBallBuilder.new(g, hb.HyperLogLogBuilder(n).log_2_num_reg(4).build()).build()
+    finally:
+        hb.debug_fail_allocations(-1)
+    seen = (dist if dist is not None else pred) != 50_000
+    assert seen.sum() > 1000 and not seen.all()
+    if dist is not None:
+        np.testing.assert_array_equal(dist[seen], want[seen])
+    if pred is not None:
+        assert np.array_equal(pred != 50_000, seen)
+        up = seen & (want > 0)
+        assert np.all(want[pred[up]] + 1 == want[up])
+    v.reset()
+    nodes, preds, dists, _ = v.par_visit([5], max_distance=3)
+    on, _, od = oracle.OracleVisit(g.offsets, g.successors).visit([5], 3)
+    d = np.full(n, -1, np.int64)
+    d[on.astype(np.int64)] = od
+    np.testing.assert_array_equal(d[nodes], dists)
+    assert len(nodes) == len(on) and np.all(d[preds[dists > 0]] + 1 == dists[dists > 0])
     v.close()
 
 

@@ -94,7 +94,7 @@ struct Level {
     uint32_t* unit;        // the units before them in their level (see end_of_level),
     uint32_t* tile[2];     // a level's slots by units / 32, and the next level's (tiles() words each)
     uint32_t* qpred;       // their predecessors and
-    uint32_t* qdist;       // their distances (PRED; not in the lean form)
+    uint32_t* qdist;       // their distances (PRED; not in the lean form), or null
     Control* ctl;
     uint64_t n;
     uint32_t lg;           // a unit's arcs (lean; else UNIT_LG)
@@ -199,8 +199,9 @@ __device__ __forceinline__ void put_group(const Level& a, unsigned long long* ta
             }
             if (a.dist) a.dist[v[i]] = d;
             if constexpr (PRED) {
-                a.qpred[slot] = run.pred[k];
-                if constexpr (!LEAN) a.qdist[slot] = d;
+                if (a.qpred) a.qpred[slot] = run.pred[k];
+                if constexpr (!LEAN)
+                    if (a.qdist) a.qdist[slot] = d;
                 if (a.pred) a.pred[v[i]] = run.pred[k];
             }
             if (t1 == t0 + 1) {

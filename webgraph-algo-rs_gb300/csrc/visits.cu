@@ -58,8 +58,7 @@ struct hb_visit {
     uint32_t* d_tile[2] = {nullptr, nullptr};
     uint32_t* d_qpred = nullptr;   // its predecessor
     uint32_t* d_qdist = nullptr;   // and distance (wide form; lean: hbl::end_of_level)
-    uint32_t* d_dist = nullptr;    // hb_visit_each: distance and predecessor by node (allocated there)
-    uint32_t* d_pred = nullptr;
+    uint32_t* d_dist = nullptr;    // hb_visit_each: distances by node where d_qpred is the predecessors (lean form)
     uint32_t* d_roots = nullptr;   // a piece of the roots of the current visit
     hbl::Control* d_ctl = nullptr;
     hbl::Control* h_ctl = nullptr; // page-locked copy
@@ -152,7 +151,8 @@ static cudaError_t visit_alloc(hb_visit* v, const uint64_t* off) {
 }
 
 // One visit from the given roots; dist and pred (by node, device) get its
-// nodes' entries, or are null. On return the stream is idle.
+// nodes' entries, or are null. They may stand where the queue's predecessors and
+// distances do, which are then not written. On return the stream is idle.
 static int visit_levels(hb_visit* v, const uint64_t* roots, size_t nroots, uint64_t max_distance, uint32_t* dist,
                         uint32_t* pred, hb_visit_stats& st) {
     if (nroots == 0) return HB_OK;
@@ -169,8 +169,9 @@ static int visit_levels(hb_visit* v, const uint64_t* roots, size_t nroots, uint6
     a.queue = v->d_queue;
     a.entry = v->d_entry;
     a.unit = v->d_unit;
-    a.qpred = v->d_qpred;
-    a.qdist = v->d_qdist;
+    auto unless_by_node = [&](uint32_t* p) { return p == dist || p == pred ? nullptr : p; };
+    a.qpred = unless_by_node(v->d_qpred);
+    a.qdist = unless_by_node(v->d_qdist);
     a.ctl = v->d_ctl;
     a.max_d = (uint32_t)std::min<uint64_t>(max_distance, 0xffffffffull);
     a.tile[0] = v->d_tile[0];
@@ -245,7 +246,6 @@ static void visit_free(hb_visit* v) {
     if (v->stream) cudaStreamSynchronize(v->stream);
     cudaFree(v->block);
     cudaFree(v->d_dist);
-    cudaFree(v->d_pred);
     if (v->h_ctl) cudaFreeHost(v->h_ctl);
     if (v->ev0) cudaEventDestroy(v->ev0);
     if (v->ev1) cudaEventDestroy(v->ev1);
@@ -373,26 +373,28 @@ int hb_visit_each(hb_visit* v, const uint64_t* roots, size_t nroots, uint32_t* d
     cudaStream_t s = v->stream;
     VC(v, cudaMemcpyAsync(v->host_visited.data(), v->d_visited, words * 4, cudaMemcpyDeviceToHost, s),
        "cudaMemcpyAsync");
-    // the caller's entries, which the visits write over by node on the device
-    // (in place of a pass of scattered host writes over the events, which is left
-    // for a device without room for them)
+    // The caller's entries, which the visits write over by node on the device (in
+    // place of a pass of scattered host writes over the events, which is left for
+    // a device without room for them). They stand where the events' would.
+    uint32_t *by_dist = nullptr, *by_pred = pred ? v->d_qpred : nullptr;
     bool by_node = true;
-    auto room = [&](uint32_t** p) {
-        if (!by_node || *p) return HB_OK;
-        const cudaError_t e = hbk::fail_allocation() ? cudaErrorMemoryAllocation : cudaMalloc((void**)p, v->n * 4);
-        if (e != cudaErrorMemoryAllocation) return visit_cuda(v, e, "cudaMalloc");
-        cudaGetLastError();
-        by_node = false;
-        return HB_OK;
-    };
-    if (dist)
-        if (int r = room(&v->d_dist)) return r;
-    if (pred)
-        if (int r = room(&v->d_pred)) return r;
-    if (by_node && dist)
-        VC(v, cudaMemcpyAsync(v->d_dist, dist, v->n * 4, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
-    if (by_node && pred)
-        VC(v, cudaMemcpyAsync(v->d_pred, pred, v->n * 4, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
+    if (dist) {
+        by_dist = !v->form.lean ? v->d_qdist : !pred ? v->d_qpred : v->d_dist;
+        if (!by_dist) {
+            const cudaError_t e = hbk::fail_allocation() ? cudaErrorMemoryAllocation
+                                                         : cudaMalloc((void**)&v->d_dist, v->n * 4);
+            if (e == cudaErrorMemoryAllocation) {
+                cudaGetLastError();
+                v->d_dist = by_pred = nullptr;
+                by_node = false;
+            } else {
+                VC(v, e, "cudaMalloc");
+            }
+            by_dist = v->d_dist;
+        }
+    }
+    if (by_dist) VC(v, cudaMemcpyAsync(by_dist, dist, v->n * 4, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
+    if (by_pred) VC(v, cudaMemcpyAsync(by_pred, pred, v->n * 4, cudaMemcpyHostToDevice, s), "cudaMemcpyAsync");
     VC(v, cudaStreamSynchronize(s), "cudaStreamSynchronize");
     int rc = HB_OK;
     bool wrote = false;
@@ -406,8 +408,7 @@ int hb_visit_each(hb_visit* v, const uint64_t* roots, size_t nroots, uint32_t* d
         if ((v->host_visited[r >> 5] >> (r & 31)) & 1) continue;  // seq.rs:130: already visited
         hb_visit_stats st{};
         const uint64_t q0 = v->tail;
-        rc = visit_levels(v, &r, 1, UINT64_MAX, by_node && dist ? v->d_dist : nullptr,
-                          by_node && pred ? v->d_pred : nullptr, st);
+        rc = visit_levels(v, &r, 1, UINT64_MAX, by_dist, by_pred, st);
         if (!by_node && rc == HB_OK) {
             nodes.resize(st.visited);
             ps.resize(pred ? st.visited : 0);
@@ -437,9 +438,9 @@ int hb_visit_each(hb_visit* v, const uint64_t* roots, size_t nroots, uint32_t* d
     if (wrote) {
         int e = HB_OK;
         if (dist)
-            e = visit_cuda(v, cudaMemcpyAsync(dist, v->d_dist, v->n * 4, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
+            e = visit_cuda(v, cudaMemcpyAsync(dist, by_dist, v->n * 4, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
         if (pred && e == HB_OK)
-            e = visit_cuda(v, cudaMemcpyAsync(pred, v->d_pred, v->n * 4, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
+            e = visit_cuda(v, cudaMemcpyAsync(pred, by_pred, v->n * 4, cudaMemcpyDeviceToHost, s), "cudaMemcpyAsync");
         if (e == HB_OK) e = visit_cuda(v, cudaStreamSynchronize(s), "cudaStreamSynchronize");
         if (rc == HB_OK) rc = e;
     }

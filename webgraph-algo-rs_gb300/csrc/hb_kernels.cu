@@ -11,7 +11,7 @@
 //                          successors' counters, modified test, next-state
 //                          store, and for changed counters the exact count,
 //                          neighbourhood-function part and per-node f64 sums
-//                          (finish_node) while the counter is in registers;
+//                          (finish_scalars) while the counter is in registers;
 //   3. k_union_heavy     — the same for the heavy nodes, one CTA per node or
 //                          segment of one, beside the window kernel;
 //   4. k_mark_preds      — systolic iterations: predecessors of modified nodes
@@ -75,7 +75,7 @@ __device__ __forceinline__ void stamp_after(TilePartial* t) {
 // and the in-degree of a changed node is added to the arcs the next
 // iteration visits.
 // ---------------------------------------------------------------------------
-// The per-node values finish_node reads (measured: loading them before the
+// The per-node values finish_scalars reads (measured: loading them before the
 // gather instead gains nothing and costs registers).
 struct NodeSums {
     double pre, sod, harm;
@@ -273,7 +273,7 @@ __device__ __forceinline__ double warp_sum_f64(double x) {
 // the gather. Visited arcs are not counted per arc at all: every predecessor
 // of a node modified in t-1 is scanned in t, in every mode, so
 // visited_t = sum over u modified in t-1 of (in-degree of u without
-// self-loops), which finish_node accumulates for the next iteration.
+// self-loops), which finish_scalars accumulates for the next iteration.
 // ---------------------------------------------------------------------------
 constexpr int WINDOW = 1024;
 // lanes of the team that runs one medium node: 8 arc lanes of G chunk lanes

@@ -33,7 +33,7 @@
 // accesses. Web-like 2.6e5 (2.6 M arcs), 621 visits: 0.15 ms a visit, where three
 // launches a level, eight levels at a time, and four synchronisations took
 // 0.69; every eccentricity of a symmetric graph of 3000 nodes, whose visits one
-// block runs: 58 us a step where it took 130.
+// block runs: 54 us a step where it took 130.
 // The strongly connected component of the largest out-degree node comes from
 // two device visits (one for a symmetric graph); the host runs Tarjan's
 // algorithm (sccs/tarjan.rs) or the symmetric labelling (sccs/symm_seq.rs) on

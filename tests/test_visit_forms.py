@@ -220,3 +220,27 @@ def test_lean_sweep_symmetric(hb):
     for f in test_sweep_steps.FIELDS:
         assert got[f] == want[f], f
     np.testing.assert_array_equal(got["forward_eccentricities"], want["forward_eccentricities"])
+
+
+@pytest.mark.gpu
+def test_sweep_on_a_nearly_full_device(hb):
+    """4e6 components where 0.6 GiB are free: 85 bytes a node and 60 a
+    component fit, 40 more a node do not."""
+    torch = pytest.importorskip("torch")
+    n = 4_000_000
+    g = hb.Graph.from_csr(np.minimum(np.arange(n + 1), 20).astype(np.uint64), np.arange(1, 21).astype(np.uint32))
+    t = g.transpose()
+    hb.exact_sum_sweep(g, t, level="diameter")  # what the first sweep of a process brings along
+    torch.cuda.empty_cache()
+    hb.release_cached_memory(0)
+    want = hb.exact_sum_sweep(g, t, level="diameter")
+    free = torch.cuda.mem_get_info()[0]
+    left = n * (85 + 60) + (48 << 20)
+    held = [torch.empty(free - left, dtype=torch.uint8, device="cuda")]
+    try:
+        got = hb.exact_sum_sweep(g, t, level="diameter")
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    for f in ("diameter", "diametral_vertex", "diameter_iterations", "sweeps"):
+        assert got[f] == want[f]

@@ -653,16 +653,17 @@ struct Sweeper {
 
     // The wide form's arrays, in one allocation: the entries, and every node's row
     // forward and backward. The transpose's offsets stand where the entries come
-    // once its rows are known. Without room for them beside the program's other
-    // data the visits take the lean form (hbl::choose_form).
+    // once its rows are known. Where they take more than their share of the free
+    // memory the visits take the lean form (hbl::choose_form): up to 60 bytes a
+    // component are still to come.
     void alloc_rows(const u64* off, const u64* toff) {
         const u64 entries = std::max<u64>(n * sizeof(hbl::Entry), (n + 1) * 8), rows = n * sizeof(hbl::Entry);
         const u64 bytes = entries + (undirected ? 1 : 2) * rows;
         const u64 more = bytes - (undirected ? 0 : (n + 1) * 8);
         size_t free_bytes = 0, all = 0;
-        if (more > hbl::WIDE_BYTES) ck(cudaMemGetInfo(&free_bytes, &all), "cudaMemGetInfo");
+        ck(cudaMemGetInfo(&free_bytes, &all), "cudaMemGetInfo");
         const u64 longest = std::max(hbl::longest_row(off, n, m), undirected ? 0 : hbl::longest_row(toff, n, m));
-        form = hbl::choose_form(n, m, longest, more, free_bytes);
+        form = hbl::choose_form(n, m, longest, more <= free_bytes / hbl::WIDE_SHARE ? more : UINT64_MAX, free_bytes);
         if (!form.lean) {
             const cudaError_t e = hbk::fail_allocation() ? cudaErrorMemoryAllocation : cudaMalloc(&wide, bytes);
             if (e == cudaErrorMemoryAllocation) {
